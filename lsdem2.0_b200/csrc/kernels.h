@@ -64,10 +64,10 @@ struct ShapeView {
   // support tables (cube map of SUP_M x SUP_M cells per face, per shape, template units,
   // rounded up): per cell the values at its four corner directions (p, q), (p + 1, q),
   // (p, q + 1), (p + 1, q + 1) of the largest projection of the nodes (sup_n) and of the
-  // points bounding the solid (sup_s, where the trilinear phi can be <= 0)
+  // solid (sup_s, every point where the trilinear phi is <= 0); shapes of particles only
   const float4* sup_n;
   const float4* sup_s;
-  const float* sup_r;           // per shape: largest |p| over the sup_s points, rounded up
+  const float* sup_r;           // per shape: largest |p| of the solid's grid cells, rounded up
 };
 
 // Arithmetic form of the narrowphase and contact forces.
@@ -78,7 +78,7 @@ constexpr int SUP_M = 24;
 constexpr int SUP_CELLS = 6 * SUP_M * SUP_M;
 constexpr int SUP_VERTS = 6 * (SUP_M + 1) * (SUP_M + 1);
 void launch_support_tables(int nshapes, const double3* node_pos, const int* node_off, const int* node_cnt,
-                           const double3* pts, const long long* pts_off, float* vtx, float4* sup_n, float4* sup_s,
+                           const double4* pts, const long long* pts_off, float* vtx, float4* sup_n, float4* sup_s,
                            float* sup_r, cudaStream_t s);
 
 // A set of rigid bodies (particles or walls).

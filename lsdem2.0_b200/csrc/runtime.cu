@@ -406,7 +406,7 @@ struct lsdem_solver {
   DArr<int4> pk_meta;
   DArr<float4> pk_q;
   // support tables of the shapes (pair separation test of the candidate search)
-  DArr<double3> sup_pts;
+  DArr<double4> sup_pts;
   DArr<long long> sup_off;
   DArr<float4> sup_n, sup_s;
   DArr<float> sup_r, sup_vtx;
@@ -838,74 +838,43 @@ void initialize(lsdem_solver* s) {
     CK(s->s_clf.upload(clf.data(), clf.size(), st));
   }
   {
-    // support tables: per shape, points whose convex hull holds every point where the
-    // trilinear phi is <= 0, template units. The grid is refined by two (points at half
-    // spacings): phi restricted to one of the eight sub-cells of a cell is trilinear
-    // with the sub-cell's corner values, and a multilinear function takes its minimum
-    // over a box at a corner, so a point with phi <= 0 lies in a sub-cell with a corner
-    // phi <= 0. Those corners are marked (each with a tolerance above the rounding of
-    // its interpolation), the marks dilated by one refined point in every direction
-    // (the corners of every such sub-cell), and only the points with a 6-neighbour
-    // outside the set kept (the largest projection of a lattice set is reached there).
-    std::vector<double3> pts;
+    // support tables: per shape, the corners (template units, phi in w) of every grid cell
+    // that holds a point where the solid phi <= 0 can end: phi has both signs on it, or it
+    // is a boundary cell of the grid with phi <= 0 somewhere (k_support_vertices; the
+    // tolerance is above the rounding of the interpolation). Only particles' shapes are
+    // ever looked up.
+    std::vector<double4> pts;
     std::vector<long long> poff{0};
-    for (const ShapeHost& sh : s->shapes) {
+    std::vector<uint8_t> used(s->shapes.size(), 0);
+    for (int sh : s->P.shape) used[sh] = 1;
+    for (size_t q = 0; q < s->shapes.size(); ++q) {
+      const ShapeHost& sh = s->shapes[q];
       const int gx = sh.size[0], gy = sh.size[1], gz = sh.size[2];
-      const int nx = 2 * gx - 1, ny = 2 * gy - 1, nz = 2 * gz - 1;
-      const size_t N = (size_t)nx * ny * nz;
-      auto id = [&](int x, int y, int z) { return (size_t)x + (size_t)nx * (y + (size_t)ny * z); };
-      auto gv = [&](int x, int y, int z) { return sh.sdf[(size_t)x + (size_t)gx * (y + (size_t)gy * z)]; };
-      std::vector<uint8_t> m(N, 0), t(N);
-      for (int z = 0; z + 1 < gz; ++z)
+      const size_t sy = (size_t)gx, sz = (size_t)gx * gy;
+      std::vector<uint8_t> m(used[q] ? sz * gz : 0, 0);
+      for (int z = 0; z + 1 < gz && used[q]; ++z)
         for (int y = 0; y + 1 < gy; ++y)
           for (int x = 0; x + 1 < gx; ++x) {
-            double c[8], lo = 1e300, hi = -1e300, mag = 0.;
-            for (int k = 0; k < 8; ++k) {
-              c[k] = gv(x + (k & 1), y + ((k >> 1) & 1), z + (k >> 2));
-              lo = std::min(lo, c[k]);
-              hi = std::max(hi, c[k]);
-              mag = std::max(mag, std::fabs(c[k]));
+            const size_t i0 = (size_t)x + sy * y + sz * z;
+            const double* c = &sh.sdf[i0];
+            const double v[8] = {c[0], c[1], c[sy], c[sy + 1], c[sz], c[sz + 1], c[sz + sy], c[sz + sy + 1]};
+            double lo = v[0], hi = v[0];
+            for (int k = 1; k < 8; ++k) {
+              lo = std::min(lo, v[k]);
+              hi = std::max(hi, v[k]);
             }
-            const double tol = 1e-12 * mag;
-            if (lo > tol) continue;  // phi > 0 on the whole cell
-            for (int k = 0; k < 27; ++k) {
-              const int i = k % 3, j = (k / 3) % 3, l = k / 9;
-              double v;
-              if (hi <= tol) {
-                v = lo;  // phi <= 0 on the whole cell
-              } else {
-                const double fx = 0.5 * i, fy = 0.5 * j, fz = 0.5 * l;
-                const double c00 = c[0] * (1 - fx) + c[1] * fx, c10 = c[2] * (1 - fx) + c[3] * fx;
-                const double c01 = c[4] * (1 - fx) + c[5] * fx, c11 = c[6] * (1 - fx) + c[7] * fx;
-                v = (c00 * (1 - fy) + c10 * fy) * (1 - fz) + (c01 * (1 - fy) + c11 * fy) * fz;
-              }
-              if (v <= tol) m[id(2 * x + i, 2 * y + j, 2 * z + l)] = 1;
-            }
+            const double tol = 1e-12 * std::max(std::fabs(lo), std::fabs(hi));
+            const bool edge = x == 0 || y == 0 || z == 0 || x + 2 == gx || y + 2 == gy || z + 2 == gz;
+            if (lo > tol || (hi < -tol && !edge)) continue;
+            for (int k = 0; k < 8; ++k) m[i0 + (k & 1) + sy * ((k >> 1) & 1) + sz * (k >> 2)] = 1;
           }
-      // separable dilation by one point along x, y, z (the 27-neighbourhood)
-      for (int ax = 0; ax < 3; ++ax) {
-        for (int z = 0; z < nz; ++z)
-          for (int y = 0; y < ny; ++y)
-            for (int x = 0; x < nx; ++x) {
-              const int c[3] = {x, y, z}, lim[3] = {nx, ny, nz};
-              uint8_t v = m[id(x, y, z)];
-              if (c[ax] > 0) v |= m[id(x - (ax == 0), y - (ax == 1), z - (ax == 2))];
-              if (c[ax] + 1 < lim[ax]) v |= m[id(x + (ax == 0), y + (ax == 1), z + (ax == 2))];
-              t[id(x, y, z)] = v;
-            }
-        m.swap(t);
-      }
-      for (int z = 0; z < nz; ++z)
-        for (int y = 0; y < ny; ++y)
-          for (int x = 0; x < nx; ++x) {
-            if (!m[id(x, y, z)]) continue;
-            const bool edge = x == 0 || y == 0 || z == 0 || x == nx - 1 || y == ny - 1 || z == nz - 1;
-            if (!edge && m[id(x - 1, y, z)] && m[id(x + 1, y, z)] && m[id(x, y - 1, z)] && m[id(x, y + 1, z)] &&
-                m[id(x, y, z - 1)] && m[id(x, y, z + 1)])
-              continue;
-            pts.push_back(make_double3(sh.origin[0] + 0.5 * sh.h * x, sh.origin[1] + 0.5 * sh.h * y,
-                                       sh.origin[2] + 0.5 * sh.h * z));
-          }
+      size_t i = 0;
+      for (int z = 0; z < gz && used[q]; ++z)
+        for (int y = 0; y < gy; ++y)
+          for (int x = 0; x < gx; ++x, ++i)
+            if (m[i])
+              pts.push_back(make_double4(sh.origin[0] + sh.h * x, sh.origin[1] + sh.h * y, sh.origin[2] + sh.h * z,
+                                         sh.sdf[i]));
       poff.push_back((long long)pts.size());
     }
     const int ns = (int)s->shapes.size();
