@@ -238,19 +238,25 @@ struct StepArgs {
   const float* mlp_band;     // per shape: trust band + error bound, in template spacings
   NetView net[2];            // learned form, per narrowphase launch
   int nshapes;
-  // Neighbour lists (exact, optional): *reuse is set non-zero when a particle moved
-  // more than sqrt(move2) from its position at the last list build; the cell sort and
+  // Neighbour lists (exact, optional): *reuse is set non-zero when a point of a particle
+  // may have moved more than `move` since the last list build; the cell sort and
   // the list rebuild run only then. The step's kick clears it.
   int* reuse;
-  double move2;
+  float move;             // 0.4 skin
   float skin;             // neighbour-list margin beyond the candidate reach (length)
   double3* xb;            // particle order: position at the last list build
-  int* nbr;               // sorted order of the last sort: entry j of position t at j * n + t
-  int* nbr_cnt;           // sorted order: entries, -1 when the list overflowed
+  float4* qb;             // particle order: orientation at the last list build
+  int* nbr;               // particle order: entry j of particle A at j * n + A
+  int* nbr_cnt;           // particle order: entries, -1 when the list overflowed
   int nbr_cap;
   int4* pk_meta;          // sorted order, written with cell_pk: cell key, body index, shape, FP32 scale bits
   float4* pk_q;           // sorted order, written with cell_pk: FP32 orientation
 };
+
+// Neighbour lists: when *a.reuse is set, the cell sort of the keys into sorted_idx and the
+// lists (neighbours.cu); sums: REBUILD_SUMS entries.
+constexpr int REBUILD_SUMS = 4096;
+void launch_rebuild(const StepArgs& a, const BucketScratch& w, int* sorted_idx, int* sums, cudaStream_t s);
 
 // Template data for the learned-SDF kernels (mlp.cu).
 struct MlpShapeData {

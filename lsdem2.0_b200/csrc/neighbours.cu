@@ -1,0 +1,174 @@
+// Rebuild of the neighbour lists: cell sort, packed records and lists in one cooperative launch.
+//
+// A step launches it after its drift; between rebuilds every block returns at once. As separate
+// launches the sort alone was ten that returned at once, 1.9 us each of the 58 us that a step of
+// 2,000 particles took; a rebuild's phases, one grid barrier apart, take no longer than those
+// launches did.
+//
+// A list holds, per particle A, the bodies B > A that some step may find before the next
+// rebuild: bounding spheres within reach + skin, and no direction found along which the two are
+// 0.8 skin apart. Until the next rebuild no point of a body moves by more than 0.4 skin
+// (k_integrate_first, the turn of the body included), so bodies that were 0.8 skin apart have no
+// contact. Listing only what is that near, a twelfth of the bodies within reach + skin in the
+// settling configuration, is what makes the steps between rebuilds cheap.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "cell_sort.cuh"
+#include "separation.cuh"
+
+namespace lsdem {
+
+namespace cg = cooperative_groups;
+
+static constexpr unsigned FULL = 0xffffffffu;
+static constexpr int RB_THREADS = 256;
+
+// The stable cell sort of bucket_sort (sort_scan.cu), phase by phase.
+LD void grid_cell_sort(cg::grid_group& grid, const int* key, int n, int ncells, const BucketScratch& w, int* sorted_idx,
+                       int* sums, int* sw) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+  const int nb = ncells + 2, m = nb + 1;
+  for (int i = tid; i < m; i += T) w.counts[i] = w.fill[i] = 0;
+  if (tid == 0) w.big_count[0] = w.big_count[1] = 0;
+  grid.sync();
+  for (int i = tid; i < n; i += T) atomicAdd(&w.counts[bucket_of(key[i], ncells)], 1);
+  grid.sync();
+  // exclusive scan over nb + 1 entries: each block a chunk
+  const int chunk = (m + gridDim.x - 1) / gridDim.x, c0 = min(m, (int)blockIdx.x * chunk), c1 = min(m, c0 + chunk);
+  int sum = 0, tot;
+  for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) sum += __ldcg(w.counts + i);
+  block_exclusive_scan<int>(sum, sw, &tot);
+  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+  grid.sync();
+  sum = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += blockDim.x) sum += __ldcg(sums + i);
+  int base;
+  block_exclusive_scan<int>(sum, sw, &base);
+  for (int i0 = c0; i0 < c1; i0 += blockDim.x) {
+    const int i = i0 + threadIdx.x;
+    const int v = i < c1 ? __ldcg(w.counts + i) : 0;
+    const int ex = block_exclusive_scan<int>(v, sw, &tot);
+    if (i < c1) w.offs[i] = base + ex;
+    base += tot;
+  }
+  grid.sync();
+  // scatter; a special bucket longer than a warp can rank is placed in index order instead
+  const int n0 = __ldcg(w.offs + 1), nL = n - __ldcg(w.offs + ncells + 1);
+  for (int i = tid; i < n; i += T) {
+    const int b = bucket_of(key[i], ncells);
+    if ((b == 0 && n0 > 64) || (b == ncells + 1 && nL > 64)) continue;
+    sorted_idx[__ldcg(w.offs + b) + atomicAdd(&w.fill[b], 1)] = i;
+  }
+  if (blockIdx.x == 0) special_buckets(key, n, ncells, w.offs, sorted_idx, sw);
+  grid.sync();
+  for (int b = tid; b < nb; b += T) {
+    const int s = w.offs[b], L = w.offs[b + 1] - s;
+    if (L <= 1 || (b == 0 && L > 64)) continue;
+    if (L > 64) w.big_list[atomicAdd(&w.big_count[0], 1)] = b;
+    else if (L > 8) w.tmp[atomicAdd(&w.big_count[1], 1)] = b;
+    else small_bucket(key, b == ncells + 1, s, L, sorted_idx);
+  }
+  grid.sync();
+  const int nbig = __ldcg(w.big_count), nmid = __ldcg(w.big_count + 1);
+  for (int q = tid >> 5; q < nmid; q += T >> 5) {
+    const int b = __ldcg(w.tmp + q), s = w.offs[b];
+    mid_bucket(key, b == ncells + 1, s, w.offs[b + 1] - s, sorted_idx);
+  }
+  if (nbig > 0) {
+    grid.sync();  // tmp held the list of the buckets above
+    for (int q = blockIdx.x; q < nbig; q += gridDim.x) {
+      const int b = __ldcg(w.big_list + q), s = w.offs[b];
+      big_bucket(key, b == ncells + 1, s, w.offs[b + 1] - s, sorted_idx, w.tmp);
+      __syncthreads();
+    }
+  }
+  grid.sync();
+}
+
+__global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScratch w, int* __restrict__ sorted_idx,
+                                                           int* __restrict__ sums) {
+  if (*a.reuse == 0) return;
+  __shared__ int sw[32];
+  cg::grid_group grid = cg::this_grid();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+  const int n = a.P.n;
+  grid_cell_sort(grid, a.P.key, n, a.pg.ncells, w, sorted_idx, sums, sw);
+  if (tid == 0) atomicAdd(&a.status->builds, 1);
+  for (int k = tid; k < n; k += T) pack_cell(a, k, __ldcg(sorted_idx + k));
+  grid.sync();
+  // lists, threads in cell-sorted order (the lanes of a warp walk the same cells in step)
+  const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
+  const bool sep = a.S.sup_n != nullptr;
+  const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
+  int need = 0;
+  for (int t = tid; t < n; t += T) {
+    const float4 pa = a.cell_pk[t], qA = a.pk_q[t];
+    const int4 mA = a.pk_meta[t];
+    const int A = mA.y;
+    const double3 xA = a.P.pos[A];
+    const float n1a = n1_f(pa);
+    // A's ball of reach + skin can reach past the 27 cells (cells are only 2 rmax wide;
+    // reach + skin is up to 2.1 rmax): every cell it overlaps is walked (at most two more per
+    // side), with a rounding margin far beyond the FP32 test's
+    const double R = a.P.radius[A] + a.rmax + (double)a.skin;
+    const double ext = 1.001 * R + 1e-4 * (fabs(xA.x) + fabs(xA.y) + fabs(xA.z) + 4.0 * R);
+    const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
+    int3 lo = ball_cell(xA - d3(ext, ext, ext), a.pg), hi = ball_cell(xA + d3(ext, ext, ext), a.pg);
+    lo = make_int3(min(lo.x, max(c.x - 1, 0)), min(lo.y, max(c.y - 1, 0)), min(lo.z, max(c.z - 1, 0)));
+    hi = make_int3(max(hi.x, min(c.x + 1, a.pg.size.x - 1)), max(hi.y, min(c.y + 1, a.pg.size.y - 1)),
+                   max(hi.z, min(c.z + 1, a.pg.size.z - 1)));
+    int nl = 0;
+    for (int z = lo.z; z <= hi.z; ++z) {
+      for (int y = lo.y; y <= hi.y; ++y) {
+        // the cells of a row are contiguous in the sorted order
+        const int h0 = lin3(make_int3(lo.x, y, z), a.pg.size);
+        const int st = __ldcg(w.offs + h0 + 1), en = __ldcg(w.offs + h0 + (hi.x - lo.x) + 2);
+#pragma unroll 2
+        for (int k = st; k < en; ++k) {
+          const float4 pb = a.cell_pk[k];
+          const float Rs = __fmul_rn(__fmaf_rn(1e-5f, __fadd_rn(n1a, n1_f(pb)), __fadd_rn(reach_f(pa, n1a, pb), a.skin)),
+                                     1.0f + 1e-4f);
+          if (dist2_f(pa, pb) > __fmul_rn(Rs, Rs)) continue;
+          const int4 mB = a.pk_meta[k];
+          if (mB.y <= A) continue;
+          if (sep && pair_separated<2>(sup, pa, n1a, qA, __int_as_float(mA.w), mA.z, pb, a.pk_q[k],
+                                       __int_as_float(mB.w), mB.z, gap))
+            continue;
+          if (nl < a.nbr_cap) a.nbr[(size_t)nl * n + A] = mB.y;
+          ++nl;
+        }
+      }
+    }
+    // an overflowed list: the batch re-runs with longer lists
+    a.nbr_cnt[A] = nl <= a.nbr_cap ? nl : -1;
+    if (nl > a.nbr_cap) atomicOr(&a.status->flags, OVF_NBR);
+    need = max(need, nl);
+    a.xb[A] = xA;
+    const Quat q = a.P.quat[A];
+    a.qb[A] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
+  }
+  need = __reduce_max_sync(FULL, need);
+  if ((threadIdx.x & 31) == 0 && need > 0) atomicMax(&a.status->need_nbr, need);
+}
+
+void launch_rebuild(const StepArgs& a, const BucketScratch& w, int* sorted_idx, int* sums, cudaStream_t s) {
+  static int blocks = 0;  // resident at once, the same on every B200
+  if (blocks == 0) {
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rebuild, RB_THREADS, 0);
+    blocks = std::min(std::max(1, sms * per), REBUILD_SUMS);
+  }
+  if (a.P.n <= 0) return;
+  // one thread per body or two buckets; fewer blocks make the barriers of a small system cheaper
+  const int want = std::max((a.P.n + RB_THREADS - 1) / RB_THREADS, (a.pg.ncells / 2 + RB_THREADS) / RB_THREADS);
+  StepArgs aa = a;
+  BucketScratch ww = w;
+  void* args[] = {&aa, &ww, &sorted_idx, &sums};
+  cudaLaunchCooperativeKernel((const void*)k_rebuild, dim3(std::min(want, blocks)), dim3(RB_THREADS), args, 0, s);
+}
+
+}  // namespace lsdem

@@ -402,7 +402,8 @@ struct lsdem_solver {
   bool grow_nbr = false;
   DArr<int> reuse;
   DArr<double3> xb;
-  DArr<int> nbr, nbr_cnt;
+  DArr<float4> qb;
+  DArr<int> nbr, nbr_cnt, rb_sums;
   DArr<int4> pk_meta;
   DArr<float4> pk_q;
   // support tables of the shapes (pair separation test of the candidate search)
@@ -412,7 +413,6 @@ struct lsdem_solver {
   DArr<float> sup_r, sup_vtx;
   int nbr_cap = 24;
   float skin = 0.f;
-  double move2 = 0.;
   long long builds = 0;      // steps that sorted and rebuilt the lists (lists on)
   SlotsDev slots[2][3];      // [history parity][kind]
   ContactsDev con[2];
@@ -1004,9 +1004,10 @@ void initialize(lsdem_solver* s) {
     // particle moved 0.4 of it (pairs approach by at most twice that)
     const double sr = 0.1 * s->rmax_p;
     s->skin = (float)sr;
-    s->move2 = (0.4 * sr) * (0.4 * sr);
     CK(s->reuse.alloc(1));
     CK(s->xb.alloc(std::max(n, 1)));
+    CK(s->qb.alloc(std::max(n, 1)));
+    CK(s->rb_sums.alloc(REBUILD_SUMS));
     CK(s->nbr_cnt.alloc(std::max(n, 1)));
     CK(s->pk_meta.alloc(std::max(n, 1)));
     CK(s->pk_q.alloc(std::max(n, 1)));
@@ -1162,9 +1163,10 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.rmax = s->rmax_p;
   const bool reuse = s->reuse_on && s->reuse.p;
   a.reuse = reuse ? s->reuse.p : nullptr;
-  a.move2 = s->move2;
+  a.move = 0.4f * s->skin;
   a.skin = s->skin;
   a.xb = s->xb.p;
+  a.qb = s->qb.p;
   a.nbr = reuse ? s->nbr.p : nullptr;
   a.nbr_cnt = s->nbr_cnt.p;
   a.nbr_cap = s->nbr_cap;
@@ -1251,8 +1253,8 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
   BucketScratch w{s->bk_counts.p, s->bk_fill.p, s->bk_offs.p, s->bk_scan.p, s->bk_big.p, s->bk_bigc.p, s->bk_tmp.p};
   {
     PhaseTimer pt(s, 1);
-    bucket_sort(a.P.key, a.P.n, s->pg.ncells, w, s->cell_idx.p, s->sorted_key.p, s->cell_start.p, s->cell_end.p, st,
-                a.reuse);
+    if (a.nbr) launch_rebuild(a, w, s->cell_idx.p, s->rb_sums.p, st);
+    else bucket_sort(a.P.key, a.P.n, s->pg.ncells, w, s->cell_idx.p, s->sorted_key.p, s->cell_start.p, s->cell_end.p, st);
   }
   BucketScratch w2{s->bk2_counts.p, s->bk2_fill.p, s->bk2_offs.p, s->bk2_scan.p, s->bk2_big.p, s->bk2_bigc.p,
                    s->bk2_tmp.p};
@@ -1318,8 +1320,8 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
                s->b_state.p};
     launch_bonds(a, b, st);
   }
-  // kernels launched up to here: kick/drift/keys, cell sort (10; with neighbour lists
-  // they return at once between rebuilds), packing + candidates, narrowphase; periodic:
+  // kernels launched up to here: kick/drift/keys, cell sort and packing (11; one with
+  // neighbour lists), candidates, narrowphase; periodic:
   // wrap/images, clamped keys, cell sort (9), image compaction + packing + candidates,
   // ghost narrowphase; bonds. The precision forms add one contact pass per narrowphase
   // and a separate wall screen; the learned form the network pass and the compaction
@@ -1328,7 +1330,7 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
   const int lrn = a.mlp_inf ? 2 : 0;
   const int nf = fp32 ? 1 + (s->W.n() > 0 ? 1 : 0) + lrn : 0;
   const int ng = fp32 ? 1 + lrn : 0;
-  if (a.P.n > 0) s->launches += 14 + nf + (s->nsets > 0 ? 15 + ng : 0) + (s->bonds.bonded.empty() ? 0 : 1);
+  if (a.P.n > 0) s->launches += (a.nbr ? 4 : 14) + nf + (s->nsets > 0 ? 15 + ng : 0) + (s->bonds.bonded.empty() ? 0 : 1);
   CK(cudaGetLastError());
 }
 

@@ -9,7 +9,7 @@
 // key read three times, index written twice, plus 8 B per cell.
 #include <algorithm>
 
-#include "kernels.h"
+#include "cell_sort.cuh"
 
 namespace lsdem {
 
@@ -20,33 +20,6 @@ static constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 // Launches given a gate flag return at once when it is zero (the step keeps the
 // last sort's results, which are still in place).
 __device__ __forceinline__ bool idle(const int* gate) { return gate && *gate == 0; }
-
-template <typename T>
-__device__ T block_exclusive_scan(T v, T* smem_warp, T* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  T x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    T y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) smem_warp[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    T w = (lane < (int)(blockDim.x >> 5)) ? smem_warp[lane] : T(0);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      T y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    smem_warp[lane] = w;
-  }
-  __syncthreads();
-  T warp_off = warp > 0 ? smem_warp[warp - 1] : T(0);
-  if (total) *total = smem_warp[(blockDim.x >> 5) - 1];
-  __syncthreads();
-  return warp_off + x - v;
-}
 
 template <typename T>
 __global__ void k_scan_tile_sums(const T* __restrict__ in, long long n, T* __restrict__ sums, const int* gate) {
@@ -134,11 +107,6 @@ void scan_i64(const long long* in, long long* out, long long n, long long* tmp, 
 
 // ---------------------------------------------------------------------------
 // Bucket sort by cell key.
-// Bucket of a key: 0 for -1 (outside the domain), 1 + key for a cell, and a
-// last bucket for keys >= ncells (a centre rounding onto the upper domain face),
-// which, as in the reference, sort after every cell, by key, and belong to none.
-__device__ __forceinline__ int bucket_of(int k, int ncells) { return k < 0 ? 0 : (k >= ncells ? ncells + 1 : k + 1); }
-
 __global__ void k_bucket_clear(int* __restrict__ counts, int* __restrict__ fill, int m, int* __restrict__ big_count,
                                const int* gate) {
   if (idle(gate)) return;
@@ -176,35 +144,7 @@ __global__ void k_special_buckets(const int* __restrict__ key, int n, int ncells
                                   int* __restrict__ sorted_idx, const int* gate) {
   if (idle(gate)) return;
   __shared__ int sw[32];
-  const int L = ncells + 1;
-  const int n0 = offs[1] - offs[0], nL = offs[L + 1] - offs[L];
-  if (n0 <= 64 && nL <= 64) return;
-  int base0 = offs[0], baseL = offs[L];
-  for (int t0 = 0; t0 < n; t0 += blockDim.x) {
-    const int i = t0 + threadIdx.x;
-    const int b = i < n ? bucket_of(key[i], ncells) : -1;
-    const int f0 = b == 0 && n0 > 64, fL = b == L && nL > 64;
-    int tot0, totL;
-    const int r0 = block_exclusive_scan<int>(f0, sw, &tot0);
-    const int rL = block_exclusive_scan<int>(fL, sw, &totL);
-    if (f0) sorted_idx[base0 + r0] = i;
-    if (fL) sorted_idx[baseL + rL] = i;
-    base0 += tot0;
-    baseL += totL;
-  }
-}
-
-// (key, index) order: a stable sort by key puts the keys past the last cell, which
-// share the last bucket, in ascending key and then index order.
-__device__ __forceinline__ bool key_idx_less(int ka, int a, int kb, int b) { return ka < kb || (ka == kb && a < b); }
-
-// Compare-exchange of two (key, index) entries.
-__device__ __forceinline__ void cx(int& ka, int& a, int& kb, int& b) {
-  if (key_idx_less(kb, b, ka, a)) {
-    const int t = a, tk = ka;
-    a = b; ka = kb;
-    b = t; kb = tk;
-  }
+  special_buckets(key, n, ncells, offs, sorted_idx, sw);
 }
 
 // Cell ranges [start, end) of every cell (-1 when empty; findStartAndEnd,
@@ -239,21 +179,7 @@ __global__ void k_bucket_fix(const int* __restrict__ key, const int* __restrict_
     mid_list[atomicAdd(&big_count[1], 1)] = b;
     return;
   }
-  const bool bykey = b == ncells + 1;
-  int v[8], k[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    v[j] = j < L ? sorted_idx[s + j] : 0x7fffffff;
-    k[j] = (j < L && bykey) ? key[v[j]] : (j < L ? 0 : 0x7fffffff);
-  }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-#pragma unroll
-    for (int j = r & 1; j + 1 < 8; j += 2) cx(k[j], v[j], k[j + 1], v[j + 1]);
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    if (j < L) sorted_idx[s + j] = v[j];
+  small_bucket(key, b == ncells + 1, s, L, sorted_idx);
 }
 
 // One warp per listed bucket of 9 to 64 members: ranked by particle index in registers
@@ -267,27 +193,7 @@ __global__ void k_bucket_mid(const int* __restrict__ key, const int* __restrict_
   for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < nmid; q += (gridDim.x * blockDim.x) >> 5) {
     const int b = mid_list[q];
     const int s = offs[b], L = offs[b + 1] - s;
-    const int v0 = lane < L ? sorted_idx[s + lane] : 0x7fffffff;
-    const int v1 = lane + 32 < L ? sorted_idx[s + 32 + lane] : 0x7fffffff;
-    int r0 = 0, r1 = 0;
-    if (b == ncells + 1) {
-      const int k0 = lane < L ? key[v0] : 0x7fffffff, k1 = lane + 32 < L ? key[v1] : 0x7fffffff;
-      for (int j = 0; j < 32; ++j) {
-        const int u0 = __shfl_sync(0xffffffffu, v0, j), u1 = __shfl_sync(0xffffffffu, v1, j);
-        const int w0 = __shfl_sync(0xffffffffu, k0, j), w1 = __shfl_sync(0xffffffffu, k1, j);
-        r0 += key_idx_less(w0, u0, k0, v0) + key_idx_less(w1, u1, k0, v0);
-        r1 += key_idx_less(w0, u0, k1, v1) + key_idx_less(w1, u1, k1, v1);
-      }
-    } else {
-      for (int j = 0; j < 32; ++j) {
-        const int u0 = __shfl_sync(0xffffffffu, v0, j), u1 = __shfl_sync(0xffffffffu, v1, j);
-        r0 += (u0 < v0) + (u1 < v0);
-        r1 += (u0 < v1) + (u1 < v1);
-      }
-    }
-    __syncwarp();
-    if (lane < L) sorted_idx[s + r0] = v0;
-    if (lane + 32 < L) sorted_idx[s + r1] = v1;
+    mid_bucket(key, b == ncells + 1, s, L, sorted_idx);
   }
 }
 // One block per bucket longer than 64: rank of each member by index (by key, then
@@ -298,26 +204,7 @@ __global__ void k_bucket_big(const int* __restrict__ key, const int* __restrict_
   if (idle(gate) || (int)blockIdx.x >= *big_count) return;
   const int b = big_list[blockIdx.x];
   const int s = offs[b], e = offs[b + 1], L = e - s;
-  for (int k = threadIdx.x; k < L; k += blockDim.x) tmp[s + k] = sorted_idx[s + k];
-  __syncthreads();
-  if (b == ncells + 1) {
-    for (int k = threadIdx.x; k < L; k += blockDim.x) {
-      const int v = tmp[s + k], kv = key[v];
-      int r = 0;
-      for (int m = 0; m < L; ++m) {
-        const int u = tmp[s + m];
-        r += key_idx_less(key[u], u, kv, v);
-      }
-      sorted_idx[s + r] = v;
-    }
-    return;
-  }
-  for (int k = threadIdx.x; k < L; k += blockDim.x) {
-    const int v = tmp[s + k];
-    int r = 0;
-    for (int m = 0; m < L; ++m) r += tmp[s + m] < v;
-    sorted_idx[s + r] = v;
-  }
+  big_bucket(key, b == ncells + 1, s, L, sorted_idx, tmp);
 }
 
 __global__ void k_sorted_keys(const int* __restrict__ key, const int* __restrict__ sorted_idx, int n,

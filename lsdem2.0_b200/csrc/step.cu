@@ -16,6 +16,7 @@
 #include <cuda_fp16.h>
 
 #include "kernels.h"
+#include "separation.cuh"
 
 namespace lsdem {
 
@@ -103,11 +104,19 @@ __global__ void k_integrate_first(StepArgs a) {
     P.torque[i] = d3(0., 0., 0.);
     const int key = hash_key(x, a.pg);
     if (a.reuse) {
-      // a move beyond the neighbour-list margin (a periodic wrap included) needs a new
-      // sort and new lists; so does a body entering or leaving the domain, since the
+      // a move or turn beyond the neighbour-list margin (a periodic wrap included) needs a
+      // new sort and new lists; so does a body entering or leaving the domain, since the
       // lists hold only bodies that were in a cell at the build
       const double3 m = x - a.xb[i];
-      if (dot(m, m) > a.move2 || (key < 0) != (P.key[i] < 0)) atomicOr(a.reuse, 2);
+      const float4 b = a.qb[i];
+      const double dq = (q.q0 - b.x) * (q.q0 - b.x) + (q.q1 - b.y) * (q.q1 - b.y) + (q.q2 - b.z) * (q.q2 - b.z) +
+                        (q.q3 - b.w) * (q.q3 - b.w);
+      // a point of the body at distance p from its centre has moved by at most |m| + 2 |dq| p
+      // (|dq| is 2 sin(angle / 4), its chord 2 sin(angle / 2) p); FP32 roundings, that of qb
+      // among them, are within the 1e-6
+      const float r = (float)P.radius[i];
+      const float move = sqrtf((float)dot(m, m)) + (2.0f * sqrtf((float)dq) + 1e-6f) * r;
+      if (!(move * (1.0f + 1e-6f) <= a.move) || (key < 0) != (P.key[i] < 0)) atomicOr(a.reuse, 2);
     }
     P.key[i] = key;
     if (a.pgh.cnt) a.pgh.cnt[i] = 0;
@@ -217,15 +226,7 @@ LD void append_pairs(int* list, int* ctr, int A, int cap, int cnt) {
 // walks (the particle grid's, then the image search's).
 __global__ void k_pack_cells(StepArgs a, const int* __restrict__ idx) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.P.n) return;
-  const int B = idx[k];
-  const double3 x = a.P.pos[B];
-  a.cell_pk[k] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)a.P.radius[B]);
-  if (a.pk_meta) {
-    a.pk_meta[k] = make_int4(a.P.key[B], B, a.P.shape[B], __float_as_int((float)a.P.scale[B]));
-    const Quat q = a.P.quat[B];
-    a.pk_q[k] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
-  }
+  if (k < a.P.n) pack_cell(a, k, idx[k]);
 }
 
 // ---------------------------------------------------------------------------
@@ -329,167 +330,158 @@ void launch_support_tables(int nshapes, const double3* node_pos, const int* node
   k_support_pack<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(nshapes, vtx, sup_n, sup_s);
 }
 
-// The separation test runs in FP32 on the packed records of the candidate search, with
-// explicitly rounded operations, so that every place it is inlined at decides a pair alike.
-LD float3 rot_f(float3 v, float w, float a, float b, float c) {
-  const float tx = __fmul_rn(2.0f, __fmaf_rn(b, v.z, -__fmul_rn(c, v.y)));
-  const float ty = __fmul_rn(2.0f, __fmaf_rn(c, v.x, -__fmul_rn(a, v.z)));
-  const float tz = __fmul_rn(2.0f, __fmaf_rn(a, v.y, -__fmul_rn(b, v.x)));
-  return make_float3(__fadd_rn(__fmaf_rn(w, tx, v.x), __fmaf_rn(b, tz, -__fmul_rn(c, ty))),
-                     __fadd_rn(__fmaf_rn(w, ty, v.y), __fmaf_rn(c, tx, -__fmul_rn(a, tz))),
-                     __fadd_rn(__fmaf_rn(w, tz, v.z), __fmaf_rn(a, ty, -__fmul_rn(b, tx))));
-}
-LD float dot_f(float3 a, float3 b) { return __fmaf_rn(a.x, b.x, __fmaf_rn(a.y, b.y, __fmul_rn(a.z, b.z))); }
-
-// Upper bound of the support h(u) from the table of one shape, and the bound's gradient g:
-// on the cone of a cell's triangle the bound is linear in u, so g is the point it is reached
-// at (a point near the shape's support point along u). 0 when u = 0.
-LD float sup_bound_f(const float4* __restrict__ tab, float3 u, float3& g) {
-  const float ax = fabsf(u.x), ay = fabsf(u.y), az = fabsf(u.z);
-  int f;
-  float p, q, m;
-  if (ax >= ay && ax >= az) { f = u.x >= 0.f ? 0 : 1; m = ax; p = u.y; q = u.z; }
-  else if (ay >= az) { f = u.y >= 0.f ? 2 : 3; m = ay; p = u.z; q = u.x; }
-  else { f = u.z >= 0.f ? 4 : 5; m = az; p = u.x; q = u.y; }
-  g = make_float3(0.f, 0.f, 0.f);
-  if (!(m > 0.f)) return 0.f;
-  const float r = __frcp_rn(m);
-  p = __fmul_rn(p, r);
-  q = __fmul_rn(q, r);
-  const float x = __fmul_rn(__fadd_rn(p, 1.0f), 0.5f * SUP_M);
-  const float y = __fmul_rn(__fadd_rn(q, 1.0f), 0.5f * SUP_M);
-  const int i = min(max((int)floorf(x), 0), SUP_M - 1), j = min(max((int)floorf(y), 0), SUP_M - 1);
-  const float s = fminf(fmaxf(__fsub_rn(x, (float)i), 0.f), 1.f), t = fminf(fmaxf(__fsub_rn(y, (float)j), 0.f), 1.f);
-  const float4 c = __ldg(tab + (f * SUP_M + j) * SUP_M + i);
-  const bool low = __fadd_rn(s, t) <= 1.0f;
-  const float ds = low ? __fsub_rn(c.y, c.x) : __fsub_rn(c.w, c.z), dt = low ? __fsub_rn(c.z, c.x) : __fsub_rn(c.w, c.y);
-  const float v = low ? __fmaf_rn(s, ds, __fmaf_rn(t, dt, c.x))
-                      : __fmaf_rn(__fsub_rn(s, 1.0f), ds, __fmaf_rn(__fsub_rn(t, 1.0f), dt, c.w));
-  const float gp = __fmul_rn(ds, 0.5f * SUP_M), gq = __fmul_rn(dt, 0.5f * SUP_M);
-  const float g0 = __fmaf_rn(-gp, p, __fmaf_rn(-gq, q, v)), gm = (f & 1) ? -g0 : g0;
-  g = f < 2 ? make_float3(gm, gp, gq) : (f < 4 ? make_float3(gq, gm, gp) : make_float3(gp, gq, gm));
-  return __fmul_rn(m, v);
-}
-
-struct SupTabs {
-  const float4* n;  // nodes
-  const float4* s;  // solid
-  const float* r;   // largest |p| of the solid's points
-};
-
-// Separating-axis test of the pair (A, B). For a direction s, every node of A projects onto s
-// at most scale_A h_n(A, R_A^T s) beyond x_A, and every point where B's interpolated phi is
-// <= 0 at least scale_B h_s(B, -R_B^T s) before x_B; if the two reaches sum to less than
-// s . (x_B - x_A) for any s, no node of A can be inside B and the pair has no contact.
-// The first direction is the line of centres. While a direction does not separate, the two
-// support points it gives, delta = (B's) - (A's), give the next: s + 1.75 (e / |delta|^2) delta,
-// e what s . delta lacks of the margin, over-relaxed towards the half space that s must lie in
-// (the separating vector step of K. Chung and W. Wang, "Quick collision detection of polytopes in
-// virtual environments", 1996, with 1.75 in place of its reflection's 2). Of the pairs of a
-// random packing of superquadrics that some direction separates, the line of centres finds
-// four fifths, one more direction 97 %, SEP_DIRS directions 99.7 %. The bodies of a pair that
-// is kept are within a few per cent of their size of touching, so this test sets the work of
-// everything after it: settling configuration of 2M particles, candidate pairs per step
-// 490k -> 225k; bonded lattice of 12,000, 43.8k -> 6.8k
-// (25k and none with the tables of k_support_vertices).
-// Margins: the FP32 centres differ from the FP64 ones by at most 2^-24 of each
-// coordinate, so the distance by 1.2e-7 (n1 + D); 2e-6 for the FP32 orientation and
-// rotation, and 2e-6 for the rounding of the face
-// coordinates and of the interpolation (the interpolated plane point moves by a few
-// 1e-7, and the values, at most sqrt(3) times the set's largest |p|, round by a few
-// ulps); a direction error e moves a support by at most e times the set's largest |p|
-// (the bounding radius for A's nodes, scale_B sup_r for B's solid). |s| = 1 and the rotation
-// keeps it within 1e-6, and s . (x_B - x_A) rounds by less than 1e-6 D, covered by the relative
-// 1e-5. Each margin is taken several times over, and they are the same for every direction: a
-// direction is exact by itself, whichever way it was found.
-static constexpr int SEP_DIRS = 5;
-LD bool pair_separated(const SupTabs& S, float4 pa, float n1a, float4 qA, float scA, int shA, float4 pb, float4 qb,
-                       float scB, int shB) {
-  const float3 d = make_float3(__fsub_rn(pb.x, pa.x), __fsub_rn(pb.y, pa.y), __fsub_rn(pb.z, pa.z));
-  const float D2 = dot_f(d, d);
-  if (!(D2 > 0.f)) return false;
-  const float D = __fsqrt_rn(D2), Di = __frcp_rn(D);
-  const float n1 = __fadd_rn(n1a, __fadd_rn(__fadd_rn(fabsf(pb.x), fabsf(pb.y)), fabsf(pb.z)));
-  const float eps = __fadd_rn(__fmul_rn(__fmul_rn(4e-7f, __fadd_rn(n1, D)), Di), 8e-6f);
-  const float rho = __fadd_rn(pa.w, __fmul_rn(scB, __ldg(S.r + shB)));
-  const float slack = __fmaf_rn(eps, rho, __fmaf_rn(1e-6f, n1, __fmul_rn(1e-5f, D)));
-  const float4* tA = S.n + (size_t)shA * SUP_CELLS;
-  const float4* tB = S.s + (size_t)shB * SUP_CELLS;
-  float3 s = make_float3(__fmul_rn(d.x, Di), __fmul_rn(d.y, Di), __fmul_rn(d.z, Di));
-#pragma unroll 1
-  for (int k = 0;; ++k) {
-    float3 gA, gB;
-    const float hA = __fmul_rn(scA, sup_bound_f(tA, rot_f(s, qA.x, -qA.y, -qA.z, -qA.w), gA));
-    const float hB = __fmul_rn(scB, sup_bound_f(tB, rot_f(make_float3(-s.x, -s.y, -s.z), qb.x, -qb.y, -qb.z, -qb.w), gB));
-    const float sd = dot_f(s, d), need = __fmul_rn(__fadd_rn(__fadd_rn(hA, hB), slack), 1.0f + 1e-5f);
-    if (need < sd) return true;
-    if (k == SEP_DIRS - 1) return false;
-    const float3 wA = rot_f(gA, qA.x, qA.y, qA.z, qA.w), wB = rot_f(gB, qb.x, qb.y, qb.z, qb.w);
-    const float3 dl = make_float3(__fmaf_rn(scB, wB.x, __fmaf_rn(-scA, wA.x, d.x)),
-                                  __fmaf_rn(scB, wB.y, __fmaf_rn(-scA, wA.y, d.y)),
-                                  __fmaf_rn(scB, wB.z, __fmaf_rn(-scA, wA.z, d.z)));
-    const float dd = dot_f(dl, dl);
-    if (!(dd > __fmul_rn(1e-10f, D2))) return false;
-    const float c = __fdiv_rn(__fmul_rn(1.75f, __fsub_rn(need, sd)), dd);
-    s = make_float3(__fmaf_rn(c, dl.x, s.x), __fmaf_rn(c, dl.y, s.y), __fmaf_rn(c, dl.z, s.z));
-    const float i = __frsqrt_rn(dot_f(s, s));
-    s = make_float3(__fmul_rn(s.x, i), __fmul_rn(s.y, i), __fmul_rn(s.z, i));
-  }
-}
-
-// Bounding-sphere test of the candidate search on the FP32 copies (centre and
-// bounding radius): the reach carries a margin that covers their rounding
-// (relative 1e-5 plus 1e-6 of the coordinates). Written with explicitly rounded
-// operations so that every caller evaluates it to the same bits.
-LD float reach_f(float4 pa, float n1a, float4 pb) {
-  const float n1 = __fadd_rn(n1a, __fadd_rn(__fadd_rn(fabsf(pb.x), fabsf(pb.y)), fabsf(pb.z)));
-  return __fmaf_rn(1e-6f, n1, __fmul_rn(__fadd_rn(pa.w, pb.w), 1.0f + 1e-5f));
-}
-LD float dist2_f(float4 pa, float4 pb) {
-  const float dx = __fsub_rn(pb.x, pa.x), dy = __fsub_rn(pb.y, pa.y), dz = __fsub_rn(pb.z, pa.z);
-  return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-}
-
-// Cell index along one axis of the point v, by floor and clamped to [0, n - 1]:
-// monotone in v and equal to the key's int() cell for points inside the grid.
-LD int ball_axis(double v, double mn, double inv, int n) {
-  const double f = floor((v - mn) * inv);
-  return f <= 0.0 ? 0 : (f >= (double)(n - 1) ? n - 1 : (int)f);
-}
-LD int3 ball_cell(double3 p, const GridP& g) {
-  return make_int3(ball_axis(p.x, g.mn.x, g.inv.x, g.size.x), ball_axis(p.y, g.mn.y, g.inv.y, g.size.y),
-                   ball_axis(p.z, g.mn.z, g.inv.z, g.size.z));
-}
-
 // Candidate partners of each particle A.
 // Particle partners: B > A, visible (in a cell), bounding spheres within
 // reach (|xA - xB| <= rA + rB is necessary for any node of A to pass the
 // reference's |node - xB| <= rB test, which in turn implies B lies in the
 // node's 27-cell window since cells are at least 2 max radius wide). The test
 // runs on the FP32 copies (reach_f), so the candidates are a superset of the
-// exact ones; the narrowphase decides every node exactly. A pair whose reaches along
-// the line of centres fall short of the distance (pair_separated) has no node of A
-// inside B and is dropped.
+// exact ones; the narrowphase decides every node exactly. A pair that some direction
+// separates (pair_separated) has no node of A inside B and is dropped.
 // Wall partners: visible walls whose SDF grid box the bounding sphere reaches and
 // whose interpolated phi is not provably positive over it (wall_far).
-// One thread per particle, threads in cell-sorted order: the lanes of a warp
-// mostly share a cell, so they walk the same 27 cells (z, y, x order) in step
-// and their occupant loads are broadcasts. Slots are filled in cell-walk then
-// sorted-occupant order.
-// The walk visits the cells of the window in ascending key order and the occupants
-// of a cell in ascending index (stable sort), so its partners come in ascending
+
+// Wall partners of particle A (few), in wall order; returns how many there are.
+LD int wall_candidates(const StepArgs& a, int A, double3 xA, double rA) {
+  const int capw = a.pw.cap;
+  int nw = 0;
+  for (int w = 0; w < a.W.n; ++w) {
+    if (a.W.key[w] < 0) continue;
+    const double3 l = rotate_inv(xA - a.W.pos[w], a.W.quat[w]);
+    double3 lo, hi;
+    grid_box(a.W.origin[w], a.W.invh[w], a.S.gsize[a.W.shape[w]], lo, hi);
+    const double reach = rA * (1.0 + 1e-9) + coord_slack(xA, a.W.pos[w]) + 1e-12 * len(hi - lo);
+    if (box_dist(l, lo, hi) > reach) continue;
+    if (wall_far(a, w, l, reach)) continue;
+    if (nw < capw) a.pw.id[(size_t)A * capw + nw] = w;
+    ++nw;
+  }
+  if (capw > 0) a.pw.cnt[A] = nw < capw ? nw : capw;
+  if (nw > capw) atomicOr(&a.status->flags, OVF_WALL);
+  return nw;
+}
+
+// End of a candidate kernel (all lanes of the warp): the flat pair lists of the precision
+// forms, the largest demands, one atomic per warp.
+LD void candidates_done(const StepArgs& a, int A, bool on, int n, int nw) {
+  if (a.pl.ctr) {
+    append_pairs(a.pl.list[0], &a.pl.ctr[0], A, a.pp.cap, on ? min(n, a.pp.cap) : 0);
+    if (a.pw.cap > 0) append_pairs(a.pl.list[1], &a.pl.ctr[1], A, a.pw.cap, on ? min(nw, a.pw.cap) : 0);
+  }
+  n = __reduce_max_sync(FULL, n);
+  nw = __reduce_max_sync(FULL, nw);
+  if ((threadIdx.x & 31) == 0) {
+    if (n > 0) atomicMax(&a.status->need_pp, n);
+    if (nw > 0) atomicMax(&a.status->need_wall, nw);
+  }
+}
+
+// Slots of A in ascending (cell key, index) order, the walk's.
+LD void order_slots(const StepArgs& a, int* out, int n) {
+  for (int u = 1; u < n; ++u) {
+    const int B = out[u], kb = a.P.key[B];
+    int v = u - 1;
+    for (; v >= 0; --v) {
+      const int C = out[v], kc = a.P.key[C];
+      if (kc < kb || (kc == kb && C < B)) break;
+      out[v + 1] = C;
+    }
+    out[v + 1] = B;
+  }
+}
+
+// Candidates from the neighbour lists (k_rebuild, neighbours.cu): per particle A the bodies
+// B > A that the step's tests may find, in (cell key, index) order at the build. A pair of a
+// step is a listed one whose cell is in the window of A's cell, whose spheres reach and that no
+// direction separates; the slots are in the order of the present (key, index), the walk's.
+//
+// The warp's list entries are tested one lane per entry, whoever owns it: a particle has 0 to 4
+// of them, so a lane testing its own would leave most lanes idle. Everything is in particle
+// order, so that only the partners' records are gathered. A warp takes PER particles: 32, or 8
+// while all the warps are resident at once, when the chain of dependent loads of an entry is
+// what counts and not the lanes.
+template <int PER>
+__global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
+  __shared__ int s_cnt[4][32];
+  const int lane = threadIdx.x & 31;
+  int* cnt = s_cnt[threadIdx.x >> 5];
+  const int t0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER;
+  const int A = t0 + lane;
+  const bool on = lane < PER && A < a.P.n;
+  const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
+  const int cap = a.pp.cap;
+  const int listed = on ? max(a.nbr_cnt[A], 0) : 0;
+  cnt[lane] = 0;
+  int incl = listed;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(FULL, incl, o);
+    if (lane >= o) incl += v;
+  }
+  const int total = __shfl_sync(FULL, incl, 31);
+  unsigned moved = 0;  // owners one of whose partners changed its place in the order
+  __syncwarp();
+  for (int i0 = 0; i0 < total; i0 += 32) {
+    const int i = i0 + lane;
+    int ow = 0;  // the first lane whose inclusive count exceeds i
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const int v = __shfl_sync(FULL, incl, ow + o - 1);
+      if (v <= i) ow += o;
+    }
+    const int first = __shfl_sync(FULL, incl - listed, ow);
+    const int j = i - first, oA = t0 + ow;
+    bool keep = false, after = true;
+    int B = -1, kB = -1;
+    if (i < total) {
+      B = __ldg(a.nbr + (size_t)j * a.P.n + oA);
+      kB = a.P.key[B];
+    }
+    const int pB = __shfl_up_sync(FULL, B, 1), pk = __shfl_up_sync(FULL, kB, 1);
+    if (i < total) {
+      const double3 xA = a.P.pos[oA], xB = a.P.pos[B];
+      const CandRec ra = cand_rec(a.P, oA, xA), rb = cand_rec(a.P, B, xB);
+      if (j > 0) {
+        const int C = lane > 0 ? pB : __ldg(a.nbr + (size_t)(j - 1) * a.P.n + oA);
+        const int kC = lane > 0 ? pk : a.P.key[C];
+        after = kC < kB || (kC == kB && C < B);
+      }
+      const float n1a = n1_f(ra.p), R = reach_f(ra.p, n1a, rb.p);
+      if (kB >= 0 && kB < a.pg.ncells && !(dist2_f(ra.p, rb.p) > __fmul_rn(R, R))) {
+        const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
+        const int sx = a.pg.size.x, sxy = a.pg.size.x * a.pg.size.y;
+        const int bx = kB % sx, by = (kB / sx) % a.pg.size.y, bz = kB / sxy;
+        keep = abs(bx - c.x) <= 1 && abs(by - c.y) <= 1 && abs(bz - c.z) <= 1 &&
+               !pair_separated(sup, ra.p, n1a, ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh);
+      }
+    }
+    const unsigned m = __ballot_sync(FULL, keep);
+    const int base = cnt[ow];
+    const int rank = __popc(m & lanemask_lt() & (~0u << max(first - i0, 0)));
+    if (keep && base + rank < cap) a.pp.id[(size_t)oA * cap + base + rank] = B;
+    const int nx = __shfl_down_sync(FULL, ow, 1);
+    __syncwarp();
+    if (i < total && (lane == 31 || nx != ow || i + 1 == total)) cnt[ow] = base + rank + keep;
+    moved |= __reduce_or_sync(FULL, after ? 0u : 1u << ow);
+    __syncwarp();
+  }
+  int n = 0, nw = 0;
+  if (on) {
+    n = cnt[lane];
+    if (((moved >> lane) & 1u) && n <= cap) order_slots(a, a.pp.id + (size_t)A * cap, n);
+    a.pp.cnt[A] = n < cap ? n : cap;
+    if (n > cap) atomicOr(&a.status->flags, OVF_PP);
+    if (a.W.n > 0) nw = wall_candidates(a, A, a.P.pos[A], a.P.radius[A]);
+  }
+  candidates_done(a, A, on, n, nw);
+}
+
+// Candidates without neighbour lists: every step sorts the cells and walks the 27 of each
+// particle. One thread per particle, threads in cell-sorted order: the lanes of a warp
+// mostly share a cell, so they walk the same cells (z, y, x order) in step and their occupant
+// loads are broadcasts. The walk visits the cells of the window in ascending key order and
+// the occupants of a cell in ascending index (stable sort), so its partners come in ascending
 // (cell key, index) order.
-//
-// Neighbour lists: a step that sorts and rebuilds them (*reuse != 0) also keeps, per
-// sorted position, the sorted positions k of the walk's partners within reach + skin
-// (plus 1e-5 of the coordinates, beyond the FP32 rounding of either test). Until the
-// next rebuild the sort is not run (thread t and position k keep their bodies) and
-// every particle stays within sqrt(move2) = 0.4 skin of its position at the build, so
-// a pair that passes the test now was within reach + skin then. A listed partner is a
-// walk partner when its current cell is in the window of A's current clamped cell and
-// it passes the same FP32 test; sorted by (current key, index) the listed partners
-// are exactly the walk's, in the walk's order.
-//
 // The bounding-sphere test fills the slots with sorted positions (the first SLOT_SH of a
 // particle in shared memory, the rest in their place in global memory); the separation test
 // then runs over the warp's filled slots with one lane per pair, whoever owns it (a particle
@@ -508,27 +500,20 @@ __device__ __noinline__ bool pair_separated_call(SupTabs sup, const float4* pk, 
   return pair_separated_at(sup, pk, meta, q, t, k);
 }
 
-//
-// A warp takes PER particles: 32, or 8 while all the warps are resident at once. A small
-// system has too few warps to hide the chain of dependent loads of a direction, and with 8
-// particles the pairs of a warp fit one round of its lanes.
-template <int PER>
-__global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
+__global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
   const int lane = threadIdx.x & 31;
-  const int t0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER;
-  const int t = lane < PER ? t0 + lane : a.P.n;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, t0 = t - lane;
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const bool sep = a.S.sup_n != nullptr;
   const int cap = a.pp.cap;
-  __shared__ int s_slot[4][PER][SLOT_SH + 1];
+  __shared__ int s_slot[4][32][SLOT_SH + 1];
   const int warp = threadIdx.x >> 5;
   auto slot = [&](int owner, int A, int j) -> int& {
     return j < SLOT_SH ? s_slot[warp][owner][j] : a.pp.id[(size_t)A * cap + j];
   };
-  int n = 0, nw = 0, nl = 0, A = 0;
+  int n = 0, nw = 0, A = 0;
   int fixed = 0;  // leading slots whose pairs have been tested already
   int extra = 0;  // pairs that found no slot
-  bool ordered = true;
   double3 xA = d3(0., 0., 0.);
   double rA = 0.;
   int* out = a.pp.id;
@@ -559,103 +544,21 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
         ++extra;
       }
     };
-    const bool rebuild = a.nbr && *a.reuse != 0;
-    if (t == 0 && rebuild) atomicAdd(&a.status->builds, 1);
-    const int listed = a.nbr && !rebuild ? a.nbr_cnt[t] : -1;
     const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
-    if (listed >= 0) {
-      const int sx = a.pg.size.x, sxy = a.pg.size.x * a.pg.size.y;
-      int lk = -1, lb = -1;
-      // four entries at a time: their list reads, then their key and centre
-      // gathers, are issued together rather than one dependent chain per entry
-      for (int j0 = 0; j0 < listed; j0 += 4) {
-        int kk[4];
-        int2 mb[4];  // key, index
-        float4 pb[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) kk[u] = j0 + u < listed ? __ldg(a.nbr + (size_t)(j0 + u) * a.P.n + t) : -1;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (kk[u] >= 0) {
-            mb[u] = __ldg(reinterpret_cast<const int2*>(a.pk_meta + kk[u]));
-            pb[u] = __ldg(a.cell_pk + kk[u]);
-          }
-        }
-        unsigned hit = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float R = reach_f(pa, n1a, pb[u]);
-          if (kk[u] >= 0 && !(dist2_f(pa, pb[u]) > __fmul_rn(R, R))) hit |= 1u << u;
-        }
-#pragma unroll 1
-        for (; hit; hit &= hit - 1) {
-          const int u = __ffs(hit) - 1;
-          const bool odd = u & 1, high = u >> 1;
-          const int k = high ? (odd ? mb[3].x : mb[2].x) : (odd ? mb[1].x : mb[0].x);
-          const int B = high ? (odd ? mb[3].y : mb[2].y) : (odd ? mb[1].y : mb[0].y);
-          const int kB = high ? (odd ? kk[3] : kk[2]) : (odd ? kk[1] : kk[0]);
-          if (k < 0 || k >= a.pg.ncells) continue;
-          const int bx = k % sx, by = (k / sx) % a.pg.size.y, bz = k / sxy;
-          if (abs(bx - c.x) > 1 || abs(by - c.y) > 1 || abs(bz - c.z) > 1) continue;
-          if (k < lk || (k == lk && B < lb)) ordered = false;
-          lk = k;
-          lb = B;
-          push(kB);
-        }
-      }
-    } else {
-      // the (up to) 3 cells of a row along x are contiguous in the sorted order
-      const int x0 = c.x > 0 ? c.x - 1 : 0, x1 = c.x < a.pg.size.x - 1 ? c.x + 1 : a.pg.size.x - 1;
-      // A rebuild lists every body within reach + skin of A, and that ball can reach
-      // past the 27 cells (cells are only 2 rmax wide; reach + skin is up to 2.1 rmax):
-      // it walks the cells the ball overlaps (at most two more per side), with a
-      // rounding margin far beyond the FP32 list test's, and takes candidates only
-      // from the 27-cell window, so the candidates and their order are the walk's.
-      int3 lo = make_int3(x0, max(c.y - 1, 0), max(c.z - 1, 0));
-      int3 hi = make_int3(x1, min(c.y + 1, a.pg.size.y - 1), min(c.z + 1, a.pg.size.z - 1));
-      if (rebuild) {
-        const double R = rA + a.rmax + (double)a.skin;
-        const double ext = 1.001 * R + 1e-4 * (fabs(xA.x) + fabs(xA.y) + fabs(xA.z) + 4.0 * R);
-        const int3 e0 = ball_cell(xA - d3(ext, ext, ext), a.pg), e1 = ball_cell(xA + d3(ext, ext, ext), a.pg);
-        lo = make_int3(min(lo.x, e0.x), min(lo.y, e0.y), min(lo.z, e0.z));
-        hi = make_int3(max(hi.x, e1.x), max(hi.y, e1.y), max(hi.z, e1.z));
-      }
-      for (int z = lo.z; z <= hi.z; ++z) {
-        for (int y = lo.y; y <= hi.y; ++y) {
-          const int h0 = lin3(make_int3(lo.x, y, z), a.pg.size);
-          const int st = __ldg(a.cell_off + h0 + 1), en = __ldg(a.cell_off + h0 + (hi.x - lo.x) + 2);
-          // sorted positions of the row's cells inside the 27-cell window
-          int wst = 0, wen = 0;
-          if (abs(z - c.z) <= 1 && abs(y - c.y) <= 1) {
-            wst = __ldg(a.cell_off + h0 + (x0 - lo.x) + 1);
-            wen = __ldg(a.cell_off + h0 + (x1 - lo.x) + 2);
-          }
+    // the (up to) 3 cells of a row along x are contiguous in the sorted order
+    const int x0 = max(c.x - 1, 0), x1 = min(c.x + 1, a.pg.size.x - 1);
+    for (int z = max(c.z - 1, 0); z <= min(c.z + 1, a.pg.size.z - 1); ++z) {
+      for (int y = max(c.y - 1, 0); y <= min(c.y + 1, a.pg.size.y - 1); ++y) {
+        const int h0 = lin3(make_int3(x0, y, z), a.pg.size);
+        const int st = __ldg(a.cell_off + h0 + 1), en = __ldg(a.cell_off + h0 + (x1 - x0) + 2);
 #pragma unroll 2
-          for (int k = st; k < en; ++k) {
-            const float4 pb = __ldg(a.cell_pk + k);  // read-only: loads may run ahead of the slot stores
-            const float R = reach_f(pa, n1a, pb);
-            const float d2 = dist2_f(pa, pb);
-            if (rebuild) {
-              const float n1 = __fadd_rn(n1a, __fadd_rn(__fadd_rn(fabsf(pb.x), fabsf(pb.y)), fabsf(pb.z)));
-              const float Rs = __fmul_rn(__fmaf_rn(1e-5f, n1, __fadd_rn(R, a.skin)), 1.0f + 1e-4f);
-              if (d2 > __fmul_rn(Rs, Rs)) continue;
-              if (a.pk_meta[k].y <= A) continue;
-              if (nl < a.nbr_cap) a.nbr[(size_t)nl * a.P.n + t] = k;
-              ++nl;
-            }
-            if (k < wst || k >= wen) continue;
-            if (d2 > __fmul_rn(R, R)) continue;
-            if (!rebuild && a.pk_meta[k].y <= A) continue;
-            push(k);
-          }
+        for (int k = st; k < en; ++k) {
+          const float4 pb = __ldg(a.cell_pk + k);  // read-only: loads may run ahead of the slot stores
+          const float R = reach_f(pa, n1a, pb);
+          if (dist2_f(pa, pb) > __fmul_rn(R, R)) continue;
+          if (a.pk_meta[k].y <= A) continue;
+          push(k);
         }
-      }
-      if (rebuild) {
-        // an overflowed list would need a walk on an unsorted step: the batch re-runs
-        // with longer lists
-        a.nbr_cnt[t] = nl <= a.nbr_cap ? nl : -1;
-        if (nl > a.nbr_cap) atomicOr(&a.status->flags, OVF_NBR);
-        a.xb[A] = xA;
       }
     }
   }
@@ -694,57 +597,22 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
       if (B >= 0) out[w++] = B;
     }
     n = w + extra;
-    if (!ordered && n <= cap) {
-      // a partner changed cells since the build: restore the walk's order
-      for (int u = 1; u < n; ++u) {
-        const int B = out[u], kb = a.P.key[B];
-        int v = u - 1;
-        for (; v >= 0; --v) {
-          const int C = out[v], kc = a.P.key[C];
-          if (kc < kb || (kc == kb && C < B)) break;
-          out[v + 1] = C;
-        }
-        out[v + 1] = B;
-      }
-    }
     a.pp.cnt[A] = n < cap ? n : cap;
     if (n > cap) atomicOr(&a.status->flags, OVF_PP);
-    // walls (few), in wall order
-    const int capw = a.pw.cap;
-    for (int w = 0; w < a.W.n; ++w) {
-      if (a.W.key[w] < 0) continue;
-      const double3 l = rotate_inv(xA - a.W.pos[w], a.W.quat[w]);
-      double3 lo, hi;
-      grid_box(a.W.origin[w], a.W.invh[w], a.S.gsize[a.W.shape[w]], lo, hi);
-      const double reach = rA * (1.0 + 1e-9) + coord_slack(xA, a.W.pos[w]) + 1e-12 * len(hi - lo);
-      if (box_dist(l, lo, hi) > reach) continue;
-      if (wall_far(a, w, l, reach)) continue;
-      if (nw < capw) a.pw.id[(size_t)A * capw + nw] = w;
-      ++nw;
-    }
-    if (capw > 0) a.pw.cnt[A] = nw < capw ? nw : capw;
-    if (nw > capw) atomicOr(&a.status->flags, OVF_WALL);
+    nw = wall_candidates(a, A, xA, rA);
   }
-  if (a.pl.ctr) {  // precision form: flat pair lists
-    append_pairs(a.pl.list[0], &a.pl.ctr[0], A, a.pp.cap, t < a.P.n ? min(n, cap) : 0);
-    if (a.pw.cap > 0) append_pairs(a.pl.list[1], &a.pl.ctr[1], A, a.pw.cap, t < a.P.n ? min(nw, a.pw.cap) : 0);
-  }
-  // largest demand of the warp, one atomic per warp
-  n = __reduce_max_sync(FULL, n);
-  nw = __reduce_max_sync(FULL, nw);
-  nl = __reduce_max_sync(FULL, nl);
-  if ((threadIdx.x & 31) == 0) {
-    if (n > 0) atomicMax(&a.status->need_pp, n);
-    if (nw > 0) atomicMax(&a.status->need_wall, nw);
-    if (nl > 0) atomicMax(&a.status->need_nbr, nl);
-  }
+  candidates_done(a, A, t < a.P.n, n, nw);
 }
 
 void launch_candidates(const StepArgs& a, cudaStream_t s) {
   if (a.P.n <= 0) return;
+  if (a.nbr) {
+    if (a.P.n <= num_sms() * 20 * 8) k_candidates<8><<<(a.P.n + 31) / 32, 128, 0, s>>>(a);
+    else k_candidates<32><<<(a.P.n + 127) / 128, 128, 0, s>>>(a);
+    return;
+  }
   k_pack_cells<<<(a.P.n + 255) / 256, 256, 0, s>>>(a, a.cell_idx);
-  if (a.P.n <= num_sms() * 20 * 8) k_candidates<8><<<(a.P.n + 31) / 32, 128, 0, s>>>(a);
-  else k_candidates<32><<<(a.P.n + 127) / 128, 128, 0, s>>>(a);
+  k_candidates_walk<<<(a.P.n + 127) / 128, 128, 0, s>>>(a);
 }
 
 // ---------------------------------------------------------------------------
