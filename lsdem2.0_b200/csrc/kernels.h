@@ -246,6 +246,9 @@ struct StepArgs {
   float skin;             // neighbour-list margin beyond the candidate reach (length)
   double3* xb;            // particle order: position at the last list build
   float4* qb;             // particle order: orientation at the last list build
+  float4* rec;            // particle order, 2 per particle, written with the drift: FP32 centre and
+                          //   cell key; FP32 orientation
+  const float4* rec_s;    // particle order: FP32 bounding radius, FP32 scale, shape, 0
   int* nbr;               // particle order: entry j of particle A at j * n + A
   int* nbr_cnt;           // particle order: entries, -1 when the list overflowed
   int nbr_cap;

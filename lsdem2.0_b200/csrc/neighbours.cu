@@ -24,6 +24,7 @@ namespace cg = cooperative_groups;
 
 static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int RB_THREADS = 256;
+static constexpr int RB_BUF = 12;  // bodies within reach + skin a lane gathers before the warp tests them
 
 // The stable cell sort of bucket_sort (sort_scan.cu), phase by phase.
 LD void grid_cell_sort(cg::grid_group& grid, const int* key, int n, int ncells, const BucketScratch& w, int* sorted_idx,
@@ -91,6 +92,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
                                                            int* __restrict__ sums) {
   if (*a.reuse == 0) return;
   __shared__ int sw[32];
+  __shared__ int s_buf[RB_THREADS / 32][32 * RB_BUF], s_cnt[RB_THREADS / 32][32];
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
   const int n = a.P.n;
@@ -98,59 +100,107 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   if (tid == 0) atomicAdd(&a.status->builds, 1);
   for (int k = tid; k < n; k += T) pack_cell(a, k, __ldcg(sorted_idx + k));
   grid.sync();
-  // lists, threads in cell-sorted order (the lanes of a warp walk the same cells in step)
+  // Lists, threads in cell-sorted order (the lanes of a warp walk the same cells in step). A lane
+  // walks until its shared buffer of bodies within reach + skin is full; the warp's buffers are
+  // then tested one lane per pair, since a lane testing as it walks would leave most of the
+  // warp idle (2M settling particles: a rebuild RB_OLD us that way, RB_NEW us now).
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const bool sep = a.S.sup_n != nullptr;
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
+  const int lane = threadIdx.x & 31;
+  int* buf = s_buf[threadIdx.x >> 5];
+  int* cnt = s_cnt[threadIdx.x >> 5];
   int need = 0;
-  for (int t = tid; t < n; t += T) {
-    const float4 pa = a.cell_pk[t], qA = a.pk_q[t];
-    const int4 mA = a.pk_meta[t];
-    const int A = mA.y;
-    const double3 xA = a.P.pos[A];
-    const float n1a = n1_f(pa);
-    // A's ball of reach + skin can reach past the 27 cells (cells are only 2 rmax wide;
-    // reach + skin is up to 2.1 rmax): every cell it overlaps is walked (at most two more per
-    // side), with a rounding margin far beyond the FP32 test's
-    const double R = a.P.radius[A] + a.rmax + (double)a.skin;
-    const double ext = 1.001 * R + 1e-4 * (fabs(xA.x) + fabs(xA.y) + fabs(xA.z) + 4.0 * R);
-    const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
-    int3 lo = ball_cell(xA - d3(ext, ext, ext), a.pg), hi = ball_cell(xA + d3(ext, ext, ext), a.pg);
-    lo = make_int3(min(lo.x, max(c.x - 1, 0)), min(lo.y, max(c.y - 1, 0)), min(lo.z, max(c.z - 1, 0)));
-    hi = make_int3(max(hi.x, min(c.x + 1, a.pg.size.x - 1)), max(hi.y, min(c.y + 1, a.pg.size.y - 1)),
-                   max(hi.z, min(c.z + 1, a.pg.size.z - 1)));
-    int nl = 0;
-    for (int z = lo.z; z <= hi.z; ++z) {
-      for (int y = lo.y; y <= hi.y; ++y) {
-        // the cells of a row are contiguous in the sorted order
-        const int h0 = lin3(make_int3(lo.x, y, z), a.pg.size);
-        const int st = __ldcg(w.offs + h0 + 1), en = __ldcg(w.offs + h0 + (hi.x - lo.x) + 2);
-#pragma unroll 2
-        for (int k = st; k < en; ++k) {
-          const float4 pb = a.cell_pk[k];
-          const float Rs = __fmul_rn(__fmaf_rn(1e-5f, __fadd_rn(n1a, n1_f(pb)), __fadd_rn(reach_f(pa, n1a, pb), a.skin)),
-                                     1.0f + 1e-4f);
-          if (dist2_f(pa, pb) > __fmul_rn(Rs, Rs)) continue;
-          const int4 mB = a.pk_meta[k];
-          if (mB.y <= A) continue;
-          if (sep && pair_separated<2>(sup, pa, n1a, qA, __int_as_float(mA.w), mA.z, pb, a.pk_q[k],
-                                       __int_as_float(mB.w), mB.z, gap))
-            continue;
-          if (nl < a.nbr_cap) a.nbr[(size_t)nl * n + A] = mB.y;
-          ++nl;
+  for (int t0 = tid - lane; t0 < n; t0 += T) {
+    const int t = t0 + lane;
+    float4 pa = make_float4(0.f, 0.f, 0.f, 0.f);
+    float n1a = 0.f;
+    int A = 0, r = 0, rows = 0, ny = 1, k = 0, en = 0;
+    int3 lo = make_int3(0, 0, 0), hi = lo;
+    double3 xA = d3(0., 0., 0.);
+    if (t < n) {
+      pa = a.cell_pk[t];
+      n1a = n1_f(pa);
+      A = a.pk_meta[t].y;
+      xA = a.P.pos[A];
+      // A's ball of reach + skin can reach past the 27 cells (cells are only 2 rmax wide;
+      // reach + skin is up to 2.1 rmax): every cell it overlaps is walked (at most two more per
+      // side), with a rounding margin far beyond the FP32 test's
+      const double R = a.P.radius[A] + a.rmax + (double)a.skin;
+      const double ext = 1.001 * R + 1e-4 * (fabs(xA.x) + fabs(xA.y) + fabs(xA.z) + 4.0 * R);
+      const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
+      lo = ball_cell(xA - d3(ext, ext, ext), a.pg);
+      hi = ball_cell(xA + d3(ext, ext, ext), a.pg);
+      lo = make_int3(min(lo.x, max(c.x - 1, 0)), min(lo.y, max(c.y - 1, 0)), min(lo.z, max(c.z - 1, 0)));
+      hi = make_int3(max(hi.x, min(c.x + 1, a.pg.size.x - 1)), max(hi.y, min(c.y + 1, a.pg.size.y - 1)),
+                     max(hi.z, min(c.z + 1, a.pg.size.z - 1)));
+      ny = hi.y - lo.y + 1;
+      rows = ny * (hi.z - lo.z + 1);
+    }
+    cnt[lane] = 0;
+    while (__any_sync(FULL, r < rows || k < en)) {
+      int m = 0;
+      while (m < RB_BUF) {
+        if (k >= en) {
+          if (r >= rows) break;
+          // the cells of a row are contiguous in the sorted order
+          const int h0 = lin3(make_int3(lo.x, lo.y + r % ny, lo.z + r / ny), a.pg.size);
+          k = __ldcg(w.offs + h0 + 1);
+          en = __ldcg(w.offs + h0 + (hi.x - lo.x) + 2);
+          ++r;
+          continue;
         }
+        const float4 pb = a.cell_pk[k];
+        const float Rs = __fmul_rn(__fmaf_rn(1e-5f, __fadd_rn(n1a, n1_f(pb)), __fadd_rn(reach_f(pa, n1a, pb), a.skin)),
+                                   1.0f + 1e-4f);
+        if (!(dist2_f(pa, pb) > __fmul_rn(Rs, Rs)) && a.pk_meta[k].y > A) buf[32 * m++ + lane] = k;
+        ++k;
+      }
+      int incl = m;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int total = __shfl_sync(FULL, incl, 31);
+      __syncwarp();
+      for (int i0 = 0; i0 < total; i0 += 32) {
+        const int i = i0 + lane;
+        const int ow = lane_of(incl, i);
+        const int first = __shfl_sync(FULL, incl - m, ow), oA = __shfl_sync(FULL, A, ow);
+        bool keep = false;
+        int B = 0;
+        if (i < total) {
+          const int kB = buf[32 * (i - first) + ow], to = t0 + ow;
+          const int4 mA = a.pk_meta[to], mB = a.pk_meta[kB];
+          const float4 po = a.cell_pk[to];
+          B = mB.y;
+          keep = !(sep && pair_separated<2>(sup, po, n1_f(po), a.pk_q[to], __int_as_float(mA.w), mA.z, a.cell_pk[kB],
+                                            a.pk_q[kB], __int_as_float(mB.w), mB.z, gap));
+        }
+        const unsigned mk = __ballot_sync(FULL, keep);
+        const int at = cnt[ow] + __popc(mk & ((1u << lane) - 1u) & (~0u << max(first - i0, 0)));
+        if (keep && at < a.nbr_cap) a.nbr[(size_t)at * n + oA] = B;
+        const int nx = __shfl_down_sync(FULL, ow, 1);
+        __syncwarp();
+        if (i < total && (lane == 31 || nx != ow || i + 1 == total)) cnt[ow] = at + keep;
+        __syncwarp();
       }
     }
-    // an overflowed list: the batch re-runs with longer lists
-    a.nbr_cnt[A] = nl <= a.nbr_cap ? nl : -1;
-    if (nl > a.nbr_cap) atomicOr(&a.status->flags, OVF_NBR);
-    need = max(need, nl);
-    a.xb[A] = xA;
-    const Quat q = a.P.quat[A];
-    a.qb[A] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
+    if (t < n) {
+      const int nl = cnt[lane];
+      // an overflowed list: the batch re-runs with longer lists
+      a.nbr_cnt[A] = nl <= a.nbr_cap ? nl : -1;
+      if (nl > a.nbr_cap) atomicOr(&a.status->flags, OVF_NBR);
+      need = max(need, nl);
+      a.xb[A] = xA;
+      const Quat q = a.P.quat[A];
+      a.qb[A] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
+    }
+    __syncwarp();
   }
   need = __reduce_max_sync(FULL, need);
-  if ((threadIdx.x & 31) == 0 && need > 0) atomicMax(&a.status->need_nbr, need);
+  if (lane == 0 && need > 0) atomicMax(&a.status->need_nbr, need);
 }
 
 void launch_rebuild(const StepArgs& a, const BucketScratch& w, int* sorted_idx, int* sums, cudaStream_t s) {

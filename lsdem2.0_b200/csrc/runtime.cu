@@ -402,7 +402,7 @@ struct lsdem_solver {
   bool grow_nbr = false;
   DArr<int> reuse;
   DArr<double3> xb;
-  DArr<float4> qb;
+  DArr<float4> qb, rec, rec_s;  // orientation at the last rebuild; FP32 records of the search
   DArr<int> nbr, nbr_cnt, rb_sums;
   DArr<int4> pk_meta;
   DArr<float4> pk_q;
@@ -1007,6 +1007,15 @@ void initialize(lsdem_solver* s) {
     CK(s->reuse.alloc(1));
     CK(s->xb.alloc(std::max(n, 1)));
     CK(s->qb.alloc(std::max(n, 1)));
+    CK(s->rec.alloc(2 * (size_t)std::max(n, 1)));
+    std::vector<float4> rs((size_t)n);
+    for (int i = 0; i < n; ++i) {
+      float shape;
+      std::memcpy(&shape, &s->P.shape[i], 4);
+      rs[i] = make_float4((float)s->P.radius[i], (float)s->P.scale[i], shape, 0.f);
+    }
+    CK(s->rec_s.upload(rs.data(), rs.size(), st));
+    CK(cudaStreamSynchronize(st));  // rs goes out of scope
     CK(s->rb_sums.alloc(REBUILD_SUMS));
     CK(s->nbr_cnt.alloc(std::max(n, 1)));
     CK(s->pk_meta.alloc(std::max(n, 1)));
@@ -1167,6 +1176,8 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.skin = s->skin;
   a.xb = s->xb.p;
   a.qb = s->qb.p;
+  a.rec = s->rec.p;
+  a.rec_s = s->rec_s.p;
   a.nbr = reuse ? s->nbr.p : nullptr;
   a.nbr_cnt = s->nbr_cnt.p;
   a.nbr_cap = s->nbr_cap;

@@ -140,6 +140,18 @@ LD int3 ball_cell(double3 p, const GridP& g) {
 }
 
 
+// The lane that owns entry i of the warp's entries, given every lane's inclusive count of them
+// (all lanes call it; 31 for an i past the last).
+LD int lane_of(int incl, int i) {
+  int ow = 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const int v = __shfl_sync(0xffffffffu, incl, ow + o - 1);
+    if (v <= i) ow += o;
+  }
+  return ow;
+}
+
 // FP32 record of one particle for the two tests.
 struct CandRec {
   float4 p;  // centre, bounding radius
@@ -147,10 +159,10 @@ struct CandRec {
   float sc;
   int sh;
 };
-LD CandRec cand_rec(const BodyView& P, int i, double3 x) {
-  const Quat q = P.quat[i];
-  return CandRec{make_float4((float)x.x, (float)x.y, (float)x.z, (float)P.radius[i]),
-                 make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3), (float)P.scale[i], P.shape[i]};
+LD CandRec cand_rec(const StepArgs& a, int i, int& key) {
+  const float4 x = a.rec[2 * i], q = a.rec[2 * i + 1], s = __ldg(a.rec_s + i);
+  key = __float_as_int(x.w);
+  return CandRec{make_float4(x.x, x.y, x.z, s.x), q, s.y, __float_as_int(s.z)};
 }
 // Record of body B at sorted position k (the sorted order of the walks).
 LD void pack_cell(const StepArgs& a, int k, int B) {

@@ -119,6 +119,10 @@ __global__ void k_integrate_first(StepArgs a) {
       if (!(move * (1.0f + 1e-6f) <= a.move) || (key < 0) != (P.key[i] < 0)) atomicOr(a.reuse, 2);
     }
     P.key[i] = key;
+    if (a.reuse) {  // the candidate search's records
+      a.rec[2 * i] = make_float4((float)x.x, (float)x.y, (float)x.z, __int_as_float(key));
+      a.rec[2 * i + 1] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
+    }
     if (a.pgh.cnt) a.pgh.cnt[i] = 0;
   } else if (i < a.P.n + a.W.n) {
     const int k = i - a.P.n;
@@ -341,11 +345,52 @@ void launch_support_tables(int nshapes, const double3* node_pos, const int* node
 // Wall partners: visible walls whose SDF grid box the bounding sphere reaches and
 // whose interpolated phi is not provably positive over it (wall_far).
 
+// FP32 copy of a wall's grid box for a first cull: axes (rows of the inverse rotation), centre
+// and half extents in the world and wall frames, and the error bound that goes with them. Every
+// particle is tested against every wall, nearly always far off; in FP64 that test was a third
+// of the search of 2M settling particles.
+struct WallBox {
+  float m[9];
+  float c[3], h[3];
+  float e;
+};
+static constexpr int WALLS_SH = 16;  // walls with a copy in shared memory
+LD void load_wall_box(const StepArgs& a, int w, WallBox& b) {
+  double3 lo, hi;
+  grid_box(a.W.origin[w], a.W.invh[w], a.S.gsize[a.W.shape[w]], lo, hi);
+  const Quat q = a.W.quat[w];
+  const double3 u[3] = {rotate(q, d3(1., 0., 0.)), rotate(q, d3(0., 1., 0.)), rotate(q, d3(0., 0., 1.))};
+  const double3 mid = 0.5 * (lo + hi), half = 0.5 * (hi - lo), c = a.W.pos[w] + rotate(q, mid);
+  for (int k = 0; k < 3; ++k) {
+    b.m[3 * k] = (float)u[k].x; b.m[3 * k + 1] = (float)u[k].y; b.m[3 * k + 2] = (float)u[k].z;
+  }
+  b.c[0] = (float)c.x; b.c[1] = (float)c.y; b.c[2] = (float)c.z;
+  b.h[0] = (float)half.x; b.h[1] = (float)half.y; b.h[2] = (float)half.z;
+  // roundings of c and h (2^-24 each) and of the rotation, taken tenfold; the box's own size
+  // covers a quaternion that is off unit length by less than 1e-6
+  b.e = 4e-6f * (fabsf(b.c[0]) + fabsf(b.c[1]) + fabsf(b.c[2]) + b.h[0] + b.h[1] + b.h[2]);
+}
+// True when the ball (x, r) cannot reach the box.
+LD bool wall_box_far(const WallBox& b, float3 x, float r) {
+  const float dx = x.x - b.c[0], dy = x.y - b.c[1], dz = x.z - b.c[2];
+  const float n1 = fabsf(x.x) + fabsf(x.y) + fabsf(x.z);
+  float d2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float l = fabsf(fmaf(b.m[3 * k], dx, fmaf(b.m[3 * k + 1], dy, b.m[3 * k + 2] * dz)));
+    const float o = fmaxf(l - b.h[k], 0.f);
+    d2 = fmaf(o, o, d2);
+  }
+  const float R = r * (1.0f + 1e-5f) + b.e + 4e-6f * n1;
+  return d2 > R * R * (1.0f + 1e-5f);
+}
+
 // Wall partners of particle A (few), in wall order; returns how many there are.
-LD int wall_candidates(const StepArgs& a, int A, double3 xA, double rA) {
+LD int wall_candidates(const StepArgs& a, const WallBox* box, int A, double3 xA, double rA) {
   const int capw = a.pw.cap;
   int nw = 0;
   for (int w = 0; w < a.W.n; ++w) {
+    if (w < WALLS_SH && wall_box_far(box[w], make_float3((float)xA.x, (float)xA.y, (float)xA.z), (float)rA)) continue;
     if (a.W.key[w] < 0) continue;
     const double3 l = rotate_inv(xA - a.W.pos[w], a.W.quat[w]);
     double3 lo, hi;
@@ -397,50 +442,67 @@ LD void order_slots(const StepArgs& a, int* out, int n) {
 //
 // The warp's list entries are tested one lane per entry, whoever owns it: a particle has 0 to 4
 // of them, so a lane testing its own would leave most lanes idle. Everything is in particle
-// order, so that only the partners' records are gathered. A warp takes PER particles: 32, or 8
-// while all the warps are resident at once, when the chain of dependent loads of an entry is
-// what counts and not the lanes.
+// order, so that only the partners' records are gathered. A warp takes PER particles: as many
+// as leave half the resident warps busy, since with lists this short (0.3 entries a particle
+// in the settling configuration) a round of the warp's lanes is filled by a hundred of them
+// (300k settling particles: 43 us with 32, CAND_NEW us with 128).
 template <int PER>
 __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
-  __shared__ int s_cnt[4][32];
+  constexpr int Q = PER < 32 ? 1 : PER / 32;  // particles per lane: t0 + lane + 32 q
+  __shared__ int s_pre[4][PER + 1];           // exclusive counts of the warp's entries
+  __shared__ int s_cnt[4][PER];               // candidates found
+  __shared__ WallBox s_wall[WALLS_SH];
   const int lane = threadIdx.x & 31;
+  int* pre = s_pre[threadIdx.x >> 5];
   int* cnt = s_cnt[threadIdx.x >> 5];
   const int t0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER;
-  const int A = t0 + lane;
-  const bool on = lane < PER && A < a.P.n;
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const int cap = a.pp.cap;
-  const int listed = on ? max(a.nbr_cnt[A], 0) : 0;
-  cnt[lane] = 0;
-  int incl = listed;
+  int total = 0;
+  {
+    int listed[Q];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += v;
+    for (int q = 0; q < Q; ++q) {
+      const int A = t0 + lane + 32 * q;
+      listed[q] = lane < PER && A < a.P.n ? max(a.nbr_cnt[A], 0) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      int incl = listed[q];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane < PER) {
+        pre[lane + 32 * q] = total + incl - listed[q];
+        cnt[lane + 32 * q] = 0;
+      }
+      total += __shfl_sync(FULL, incl, 31);
+    }
+    if (lane == 0) pre[PER] = total;
   }
-  const int total = __shfl_sync(FULL, incl, 31);
-  unsigned moved = 0;  // owners one of whose partners changed its place in the order
+  unsigned moved[Q];  // this lane's owners one of whose partners changed its place in the order
+#pragma unroll
+  for (int q = 0; q < Q; ++q) moved[q] = 0;
   __syncwarp();
   for (int i0 = 0; i0 < total; i0 += 32) {
     const int i = i0 + lane;
-    int ow = 0;  // the first lane whose inclusive count exceeds i
+    int ow = 0;  // the owner of entry i: the last whose exclusive count does not exceed it
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int v = __shfl_sync(FULL, incl, ow + o - 1);
-      if (v <= i) ow += o;
-    }
-    const int first = __shfl_sync(FULL, incl - listed, ow);
-    const int j = i - first, oA = t0 + ow;
+    for (int o = PER / 2; o > 0; o >>= 1)
+      if (pre[ow + o] <= i) ow += o;
+    const int first = pre[ow], j = i - first, oA = t0 + ow;
     bool keep = false, after = true;
-    int B = -1, kB = -1;
+    int B = -1, kA = -1, kB = -1;
+    CandRec ra, rb;
     if (i < total) {
       B = __ldg(a.nbr + (size_t)j * a.P.n + oA);
-      kB = a.P.key[B];
+      ra = cand_rec(a, oA, kA);
+      rb = cand_rec(a, B, kB);
     }
     const int pB = __shfl_up_sync(FULL, B, 1), pk = __shfl_up_sync(FULL, kB, 1);
     if (i < total) {
-      const double3 xA = a.P.pos[oA], xB = a.P.pos[B];
-      const CandRec ra = cand_rec(a.P, oA, xA), rb = cand_rec(a.P, B, xB);
       if (j > 0) {
         const int C = lane > 0 ? pB : __ldg(a.nbr + (size_t)(j - 1) * a.P.n + oA);
         const int kC = lane > 0 ? pk : a.P.key[C];
@@ -448,32 +510,44 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
       }
       const float n1a = n1_f(ra.p), R = reach_f(ra.p, n1a, rb.p);
       if (kB >= 0 && kB < a.pg.ncells && !(dist2_f(ra.p, rb.p) > __fmul_rn(R, R))) {
-        const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
-        const int sx = a.pg.size.x, sxy = a.pg.size.x * a.pg.size.y;
-        const int bx = kB % sx, by = (kB / sx) % a.pg.size.y, bz = kB / sxy;
+        const int sx = a.pg.size.x, sy = a.pg.size.y;
+        const int3 c = kA >= 0 && kA < a.pg.ncells ? make_int3(kA % sx, (kA / sx) % sy, kA / (sx * sy))
+                                                   : clamp_cell(cell_of(a.P.pos[oA], a.pg), a.pg.size);
+        const int bx = kB % sx, by = (kB / sx) % sy, bz = kB / (sx * sy);
         keep = abs(bx - c.x) <= 1 && abs(by - c.y) <= 1 && abs(bz - c.z) <= 1 &&
                !pair_separated(sup, ra.p, n1a, ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh);
       }
     }
     const unsigned m = __ballot_sync(FULL, keep);
-    const int base = cnt[ow];
-    const int rank = __popc(m & lanemask_lt() & (~0u << max(first - i0, 0)));
-    if (keep && base + rank < cap) a.pp.id[(size_t)oA * cap + base + rank] = B;
+    const int at = cnt[ow] + __popc(m & lanemask_lt() & (~0u << max(min(first - i0, 31), 0)));
+    if (keep && at < cap) a.pp.id[(size_t)oA * cap + at] = B;
     const int nx = __shfl_down_sync(FULL, ow, 1);
     __syncwarp();
-    if (i < total && (lane == 31 || nx != ow || i + 1 == total)) cnt[ow] = base + rank + keep;
-    moved |= __reduce_or_sync(FULL, after ? 0u : 1u << ow);
+    if (i < total && (lane == 31 || nx != ow || i + 1 == total)) cnt[ow] = at + keep;
+    if (__any_sync(FULL, !after)) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) moved[q] |= __reduce_or_sync(FULL, !after && (ow >> 5) == q ? 1u << (ow & 31) : 0u);
+    }
     __syncwarp();
   }
-  int n = 0, nw = 0;
-  if (on) {
-    n = cnt[lane];
-    if (((moved >> lane) & 1u) && n <= cap) order_slots(a, a.pp.id + (size_t)A * cap, n);
-    a.pp.cnt[A] = n < cap ? n : cap;
-    if (n > cap) atomicOr(&a.status->flags, OVF_PP);
-    if (a.W.n > 0) nw = wall_candidates(a, A, a.P.pos[A], a.P.radius[A]);
+  if (a.W.n > 0) {
+    if ((int)threadIdx.x < min(a.W.n, WALLS_SH)) load_wall_box(a, threadIdx.x, s_wall[threadIdx.x]);
+    __syncthreads();
   }
-  candidates_done(a, A, on, n, nw);
+#pragma unroll 1
+  for (int q = 0; q < Q; ++q) {
+    const int A = t0 + lane + 32 * q;
+    const bool on = lane < PER && A < a.P.n;
+    int n = 0, nw = 0;
+    if (on) {
+      n = cnt[lane + 32 * q];
+      if (((moved[q] >> lane) & 1u) && n <= cap) order_slots(a, a.pp.id + (size_t)A * cap, n);
+      a.pp.cnt[A] = n < cap ? n : cap;
+      if (n > cap) atomicOr(&a.status->flags, OVF_PP);
+      if (a.W.n > 0) nw = wall_candidates(a, s_wall, A, a.P.pos[A], a.P.radius[A]);
+    }
+    candidates_done(a, A, on, n, nw);
+  }
 }
 
 // Candidates without neighbour lists: every step sorts the cells and walks the 27 of each
@@ -507,6 +581,9 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
   const bool sep = a.S.sup_n != nullptr;
   const int cap = a.pp.cap;
   __shared__ int s_slot[4][32][SLOT_SH + 1];
+  __shared__ WallBox s_wall[WALLS_SH];
+  if ((int)threadIdx.x < min(a.W.n, WALLS_SH)) load_wall_box(a, threadIdx.x, s_wall[threadIdx.x]);
+  __syncthreads();
   const int warp = threadIdx.x >> 5;
   auto slot = [&](int owner, int A, int j) -> int& {
     return j < SLOT_SH ? s_slot[warp][owner][j] : a.pp.id[(size_t)A * cap + j];
@@ -572,13 +649,7 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
   __syncwarp();
   for (int i0 = 0; i0 < total; i0 += 32) {
     const int i = i0 + lane;
-    int ow = 0;  // the first lane whose inclusive count exceeds i
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int v = __shfl_sync(FULL, incl, ow + o - 1);
-      if (v <= i) ow += o;
-    }
-    ow = min(ow, 31);
+    const int ow = lane_of(incl, i);
     const int j = i - (__shfl_sync(FULL, incl, ow) - __shfl_sync(FULL, n, ow));
     const int oA = __shfl_sync(FULL, A, ow), ofix = __shfl_sync(FULL, fixed, ow);
     if (i < total) {
@@ -599,7 +670,7 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
     n = w + extra;
     a.pp.cnt[A] = n < cap ? n : cap;
     if (n > cap) atomicOr(&a.status->flags, OVF_PP);
-    nw = wall_candidates(a, A, xA, rA);
+    nw = wall_candidates(a, s_wall, A, xA, rA);
   }
   candidates_done(a, A, t < a.P.n, n, nw);
 }
@@ -607,8 +678,10 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
 void launch_candidates(const StepArgs& a, cudaStream_t s) {
   if (a.P.n <= 0) return;
   if (a.nbr) {
-    if (a.P.n <= num_sms() * 20 * 8) k_candidates<8><<<(a.P.n + 31) / 32, 128, 0, s>>>(a);
-    else k_candidates<32><<<(a.P.n + 127) / 128, 128, 0, s>>>(a);
+    const int half = num_sms() * 10;  // warps
+    if (a.P.n >= half * 128) k_candidates<128><<<(a.P.n + 511) / 512, 128, 0, s>>>(a);
+    else if (a.P.n >= half * 32) k_candidates<32><<<(a.P.n + 127) / 128, 128, 0, s>>>(a);
+    else k_candidates<8><<<(a.P.n + 31) / 32, 128, 0, s>>>(a);
     return;
   }
   k_pack_cells<<<(a.P.n + 255) / 256, 256, 0, s>>>(a, a.cell_idx);
