@@ -18,7 +18,7 @@ namespace lsdem {
 enum { FIX_GRADIENT = 1, FIX_SQRTF = 2 };
 
 // Overflow bits of the device status word.
-enum { OVF_PP = 1, OVF_WALL = 2, OVF_GHOST = 4, OVF_CONTACT = 8, OVF_NBR = 16, OVF_NET = 32 };
+enum { OVF_PP = 1, OVF_WALL = 2, OVF_GHOST = 4, OVF_CONTACT = 8, OVF_NBR = 16, OVF_NET = 32, OVF_IMG = 64 };
 
 // Largest demands seen during a batch (whether or not they overflowed), used
 // to grow capacities ahead of an overflow.
@@ -32,8 +32,8 @@ struct Status {
   int builds;        // steps that sorted and rebuilt the neighbour lists
   int need_netq;     // learned form: largest rows of one shape's network queue
   int need_pend;     // learned form: largest count of nodes awaiting the network
+  int need_img;      // largest length of the image list
   int errors;        // a bounded wait in a kernel gave up (results of the batch not valid)
-  int pad;
 };
 
 // Shape templates: SDF grid + surface nodes in cluster order.
@@ -139,7 +139,8 @@ struct GhostView {
   double3* gvel;       // sector: nsets * n image velocities
   double3* gpos;       // nsets * n
   int* gkey;           // nsets * n, clamped cell or -1
-  int* list;           // nsets * n: visible images (set * n + particle), compacted
+  int* list;           // images (set * n + particle) that are visible, or (rebuild) that a step before
+                       //   the next rebuild may find visible, 2 (set * n + particle) + moved; 2 nsets * n
   int* count;          // number of entries in list
 };
 
@@ -204,6 +205,14 @@ struct NetView {
   int* ctr;               // [0] pending cursor, [1] pair records
 };
 
+// Image list of the neighbour lists' rebuild: {A | moved << 31, particle << 3 | set} (moved: the
+// image stands a domain away from the particle, not at it).
+struct ImageList {
+  int2* list;   // nullptr: images searched every step
+  int* count;
+  int cap;
+};
+
 struct StepArgs {
   BodyView P;       // particles
   BodyView W;       // walls
@@ -248,6 +257,8 @@ struct StepArgs {
   float4* qb;             // particle order: orientation at the last list build
   float4* rec;            // particle order, 2 per particle, written with the drift: FP32 centre and
                           //   cell key; FP32 orientation
+  ImageList gl;
+  int wrap_axes;          // periodic axes whose wrap the step does at its end (0: images searched every step)
   const float4* rec_s;    // particle order: FP32 bounding radius, FP32 scale, shape, 0
   int* nbr;               // particle order: entry j of particle A at j * n + A
   int* nbr_cnt;           // particle order: entries, -1 when the list overflowed
@@ -258,8 +269,18 @@ struct StepArgs {
 
 // Neighbour lists: when *a.reuse is set, the cell sort of the keys into sorted_idx and the
 // lists (neighbours.cu); sums: REBUILD_SUMS entries.
+// With a.gl.list the image list, too, from a second sort of the wrapped positions.
 constexpr int REBUILD_SUMS = 4096;
-void launch_rebuild(const StepArgs& a, const BucketScratch& w, int* sorted_idx, int* sums, cudaStream_t s);
+struct ImageSort {
+  BucketScratch w;
+  int* key;      // clamped cell of the wrapped position
+  int* idx;
+  float4* pk;    // sorted order: FP32 wrapped centre, bounding radius
+};
+void launch_rebuild(const StepArgs& a, const BucketScratch& w, const ImageSort& img, int* sorted_idx, int* sums,
+                    cudaStream_t s);
+void launch_image_candidates(const StepArgs& a, cudaStream_t s);
+void launch_wrap(const StepArgs& a, cudaStream_t s);
 
 // Template data for the learned-SDF kernels (mlp.cu).
 struct MlpShapeData {

@@ -404,6 +404,10 @@ struct lsdem_solver {
   DArr<double3> xb;
   DArr<float4> qb, rec, rec_s;  // orientation at the last rebuild; FP32 records of the search
   DArr<int> nbr, nbr_cnt, rb_sums;
+  DArr<int2> img_list;       // image list (k_rebuild)
+  DArr<int> img_count;
+  long long cap_img = 1 << 14;
+  bool grow_img = false;
   DArr<int4> pk_meta;
   DArr<float4> pk_q;
   // support tables of the shapes (pair separation test of the candidate search)
@@ -632,7 +636,7 @@ void alloc_net(lsdem_solver* s) {
   s->cap_netq = std::min<long long>(s->cap_netq, 0x7fffffffLL / ns);
   for (int l = 0; l < 2; ++l) {
     auto& N = s->net[l];
-    const long long pairs = l == 0 ? (long long)n * (s->slots[0][0].cap + s->slots[0][1].cap)
+    const long long pairs = l == 0 ? (long long)n * (s->slots[0][0].cap + s->slots[0][1].cap + s->slots[0][2].cap)
                                    : (long long)n * s->slots[0][2].cap;
     if (l == 1 && s->nsets == 0) {
       N.qcap = N.pcap = N.paircap = 0;
@@ -1042,7 +1046,9 @@ void initialize(lsdem_solver* s) {
   if (s->nsets > 0) {
     CK(s->gpos.alloc((size_t)s->nsets * std::max(n, 1)));
     CK(s->gkey.alloc((size_t)s->nsets * std::max(n, 1)));
-    CK(s->glist.alloc((size_t)s->nsets * std::max(n, 1)));
+    CK(s->glist.alloc((size_t)2 * s->nsets * std::max(n, 1)));
+    CK(s->img_list.alloc(s->cap_img));
+    CK(s->img_count.alloc(1));
     CK(s->gcount.alloc(1));
     CK(s->key2.alloc(std::max(n, 1)));
     CK(s->g2_idx.alloc(std::max(n, 1)));
@@ -1177,6 +1183,12 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.xb = s->xb.p;
   a.qb = s->qb.p;
   a.rec = s->rec.p;
+  // translated images with the lists on: from the image list, the wrap at the step's end
+  const bool img = reuse && s->nsets > 0 && !(s->periodic & 8);
+  a.gl.list = img ? s->img_list.p : nullptr;
+  a.gl.count = s->img_count.p;
+  a.gl.cap = (int)std::min<long long>(s->img_list.n, 0x7fffffff);
+  a.wrap_axes = img ? (s->periodic & 7) : 0;
   a.rec_s = s->rec_s.p;
   a.nbr = reuse ? s->nbr.p : nullptr;
   a.nbr_cnt = s->nbr_cnt.p;
@@ -1262,15 +1274,60 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
   }
   { PhaseTimer pt(s, 0); launch_integrate_first(a, st); }
   BucketScratch w{s->bk_counts.p, s->bk_fill.p, s->bk_offs.p, s->bk_scan.p, s->bk_big.p, s->bk_bigc.p, s->bk_tmp.p};
-  {
-    PhaseTimer pt(s, 1);
-    if (a.nbr) launch_rebuild(a, w, s->cell_idx.p, s->rb_sums.p, st);
-    else bucket_sort(a.P.key, a.P.n, s->pg.ncells, w, s->cell_idx.p, s->sorted_key.p, s->cell_start.p, s->cell_end.p, st);
-  }
   BucketScratch w2{s->bk2_counts.p, s->bk2_fill.p, s->bk2_offs.p, s->bk2_scan.p, s->bk2_big.p, s->bk2_bigc.p,
                    s->bk2_tmp.p};
+  {
+    PhaseTimer pt(s, 1);
+    const ImageSort im{w2, s->key2.p, s->g2_idx.p, s->cell_pk2.p};
+    if (a.nbr) launch_rebuild(a, w, im, s->cell_idx.p, s->rb_sums.p, st);
+    else bucket_sort(a.P.key, a.P.n, s->pg.ncells, w, s->cell_idx.p, s->sorted_key.p, s->cell_start.p, s->cell_end.p, st);
+  }
   const bool branch = s->nsets > 0 && !(s->periodic & 8) && !s->profiling;
-  if (branch) {
+  const int kinds = (s->W.n() > 0 ? 3 : 1) | (a.gl.list ? 4 : 0);
+  if (a.gl.list && !s->profiling) {
+    // Images from the list: their candidates run beside the particles', their pairs in the
+    // walls' screen beside the particles' screen, and one contact pass takes all.
+    cudaStream_t s2 = s->st2;
+    CK(cudaEventRecord(s->ev_fork, st));
+    CK(cudaStreamWaitEvent(s2, s->ev_fork, 0));
+    launch_image_candidates(a, s2);
+    launch_candidates(a, st);
+    if (s->precision == PREC_FP64) {
+      CK(cudaEventRecord(s->ev_join, s2));
+      CK(cudaStreamWaitEvent(st, s->ev_join, 0));
+      launch_narrowphase(a, kinds, st);
+    } else {
+      CK(cudaEventRecord(s->ev_fork, st));  // the wall pairs
+      CK(cudaStreamWaitEvent(s2, s->ev_fork, 0));
+      launch_narrowphase(a, kinds & 6, s2);
+      CK(cudaEventRecord(s->ev_join, s2));
+      launch_narrowphase(a, 1, st);
+      CK(cudaStreamWaitEvent(st, s->ev_join, 0));
+      launch_net_screen(a, 0, st);
+      launch_net_compact(a, 0, st);
+      launch_contact_pass(a, 0, st);
+    }
+    launch_wrap(a, st);
+  } else if (a.gl.list) {
+    {
+      PhaseTimer pt(s, 2);
+      launch_candidates(a, st);
+    }
+    {
+      PhaseTimer pt(s, 4);
+      launch_image_candidates(a, st);
+    }
+    { PhaseTimer pt(s, 3); launch_narrowphase(a, s->precision == PREC_FP64 ? kinds : (s->W.n() > 0 ? 3 : 1), st); }
+    if (s->precision != PREC_FP64) {
+      { PhaseTimer pt(s, 5); launch_narrowphase(a, 4, st); }
+      if (a.mlp_inf) { PhaseTimer pt(s, 10); launch_net_screen(a, 0, st); }
+      PhaseTimer pt(s, 8);
+      launch_net_compact(a, 0, st);
+      launch_contact_pass(a, 0, st);
+    }
+    PhaseTimer pt(s, 4);
+    launch_wrap(a, st);
+  } else if (branch) {
     // The periodic images run beside the particle candidates, screen and contact
     // pass, which read the pre-wrap positions: the image branch writes the wrapped
     // positions into pos_w and screens the images against them (its own sort scratch,
@@ -1332,16 +1389,16 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
     launch_bonds(a, b, st);
   }
   // kernels launched up to here: kick/drift/keys, cell sort and packing (11; one with
-  // neighbour lists), candidates, narrowphase; periodic:
-  // wrap/images, clamped keys, cell sort (9), image compaction + packing + candidates,
-  // ghost narrowphase; bonds. The precision forms add one contact pass per narrowphase
-  // and a separate wall screen; the learned form the network pass and the compaction
-  // after each screen.
+  // neighbour lists), candidates, narrowphase; periodic: image candidates and wrap, or
+  // (images searched every step) wrap/images, clamped keys, cell sort (9), image compaction +
+  // packing + candidates, ghost narrowphase; bonds. The precision forms add one contact pass
+  // (per narrowphase, where images are searched every step) and a separate screen for walls
+  // and images; the learned form the network pass and the compaction after each screen.
   const bool fp32 = s->precision != PREC_FP64;
   const int lrn = a.mlp_inf ? 2 : 0;
-  const int nf = fp32 ? 1 + (s->W.n() > 0 ? 1 : 0) + lrn : 0;
-  const int ng = fp32 ? 1 + lrn : 0;
-  if (a.P.n > 0) s->launches += (a.nbr ? 4 : 14) + nf + (s->nsets > 0 ? 15 + ng : 0) + (s->bonds.bonded.empty() ? 0 : 1);
+  const int nf = fp32 ? 1 + (s->W.n() > 0 || a.gl.list ? 1 : 0) + lrn : 0;
+  const int ng = a.gl.list ? 2 : 15 + (fp32 ? 1 + lrn : 0);
+  if (a.P.n > 0) s->launches += (a.nbr ? 4 : 14) + nf + (s->nsets > 0 ? ng : 0) + (s->bonds.bonded.empty() ? 0 : 1);
   CK(cudaGetLastError());
 }
 
@@ -1469,6 +1526,10 @@ bool plan_growth(lsdem_solver* s, const Status& st, long long last_contacts) {
     const int old = s->nbr_cap;
     up(s->nbr_cap, st.need_nbr, st.flags & OVF_NBR);
     if (s->nbr_cap != old) s->grow_nbr = true;
+    if (s->nsets > 0 && ((st.flags & OVF_IMG) || st.need_img * 5LL > s->cap_img * 4)) {
+      s->cap_img = std::max<long long>(s->cap_img * 2, st.need_img + st.need_img / 2 + 1024);
+      s->grow_img = changed = true;
+    }
   }
   const long long needc = std::max<long long>(st.need_contact, last_contacts);
   if ((st.flags & OVF_CONTACT) || needc * 5 > s->cap_c * 4) {
@@ -1506,6 +1567,10 @@ void grow(lsdem_solver* s) {
   if (s->grow_nbr) {
     CK(s->nbr.alloc((size_t)std::max(s->P.n(), 1) * s->nbr_cap));
     s->grow_nbr = false;
+  }
+  if (s->grow_img) {
+    CK(s->img_list.alloc((size_t)s->cap_img));
+    s->grow_img = false;
   }
   alloc_slots(s, true);
   if (s->grow_contacts) {

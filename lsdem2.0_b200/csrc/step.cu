@@ -15,7 +15,10 @@
 //   k_bonds            V-bond forces (contactKernel.cuh:138-199, contactKernel.cu:273-351)
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "kernels.h"
+#include "images.cuh"
 #include "separation.cuh"
 
 namespace lsdem {
@@ -116,7 +119,12 @@ __global__ void k_integrate_first(StepArgs a) {
       // among them, are within the 1e-6
       const float r = (float)P.radius[i];
       const float move = sqrtf((float)dot(m, m)) + (2.0f * sqrtf((float)dq) + 1e-6f) * r;
-      if (!(move * (1.0f + 1e-6f) <= a.move) || (key < 0) != (P.key[i] < 0)) atomicOr(a.reuse, 2);
+      // so does a body beyond a periodic face, whose wrap k_wrap does
+      const GridP& g = a.pg;
+      const bool beyond = ((a.wrap_axes & 1) && (x.x < g.mn.x || x.x >= g.mx.x)) ||
+                          ((a.wrap_axes & 2) && (x.y < g.mn.y || x.y >= g.mx.y)) ||
+                          ((a.wrap_axes & 4) && (x.z < g.mn.z || x.z >= g.mx.z));
+      if (!(move * (1.0f + 1e-6f) <= a.move) || (key < 0) != (P.key[i] < 0) || beyond) atomicOr(a.reuse, 2);
     }
     P.key[i] = key;
     if (a.reuse) {  // the candidate search's records
@@ -445,7 +453,7 @@ LD void order_slots(const StepArgs& a, int* out, int n) {
 // order, so that only the partners' records are gathered. A warp takes PER particles: as many
 // as leave half the resident warps busy, since with lists this short (0.3 entries a particle
 // in the settling configuration) a round of the warp's lanes is filled by a hundred of them
-// (300k settling particles: 43 us with 32, CAND_NEW us with 128).
+// (2M settling particles: 221 us with 32, 135 us with 128).
 template <int PER>
 __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
   constexpr int Q = PER < 32 ? 1 : PER / 32;  // particles per lane: t0 + lane + 32 q
@@ -691,6 +699,14 @@ void launch_candidates(const StepArgs& a, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Narrowphase.
 enum { KIND_PP = 0, KIND_WALL = 1, KIND_GHOST = 2 };
+
+// Position of the owner of a pair: image pairs take the wrapped one where the step's wrap has
+// yet to be done.
+template <int KIND>
+LD double3 owner_pos(const StepArgs& a, int A) {
+  const double3 x = a.P.pos[A];
+  return KIND == KIND_GHOST && a.wrap_axes ? wrap_pos(x, a.pg, a.wrap_axes) : x;
+}
 
 // The owner particle A of the warp.
 struct SelfCtx {
@@ -1085,6 +1101,7 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 2) k_narrowphase(StepArgs a) {
       do_pair<KIND_PP>(a, A, j, a.pp.id[(size_t)A * a.pp.cap + j], S, s_cl[warp], s_mask[warp], s_old[warp], FA, TA);
     for (int j = 0; j < nw; ++j)
       do_pair<KIND_WALL>(a, A, j, a.pw.id[(size_t)A * a.pw.cap + j], S, s_cl[warp], s_mask[warp], s_old[warp], FA, TA);
+    if (ngc > 0) S.x = owner_pos<KIND_GHOST>(a, A);
     for (int j = 0; j < ngc; ++j)
       do_pair<KIND_GHOST>(a, A, j, a.pgh.id[(size_t)A * a.pgh.cap + j], S, s_cl[warp], s_mask[warp], s_old[warp], FA, TA);
     FA = warp_sum3(FA);
@@ -1202,7 +1219,7 @@ LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape, int
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j)
       F.M[3 * i + j] = fmaf(rb[i], ra[j], fmaf(rb[3 + i], ra[3 + j], rb[6 + i] * ra[6 + j])) * scA;
-  const double3 d = a.P.pos[A] - P.x;
+  const double3 d = owner_pos<KIND>(a, A) - P.x;
   const float3 df = tof(d);
   F.dB = f3(fmaf(rb[0], df.x, fmaf(rb[3], df.y, rb[6] * df.z)), fmaf(rb[1], df.x, fmaf(rb[4], df.y, rb[7] * df.z)),
             fmaf(rb[2], df.x, fmaf(rb[5], df.y, rb[8] * df.z)));
@@ -1360,9 +1377,10 @@ LD bool cluster_may_hit_f(const PairF& F, float4 cn, float scA, float* up = null
   return !(ph > F.T + reach);
 }
 
+template <int KIND>
 LD SelfCtx self_ctx(const StepArgs& a, int A) {
   SelfCtx S;
-  S.x = a.P.pos[A]; S.v = a.P.vel[A]; S.w = a.P.angvel[A]; S.q = a.P.quat[A];
+  S.x = owner_pos<KIND>(a, A); S.v = a.P.vel[A]; S.w = a.P.angvel[A]; S.q = a.P.quat[A];
   S.sc = a.P.scale[A];
   const int sh = a.P.shape[A];
   S.n0 = a.S.node_off[sh]; S.nn = a.S.node_cnt[sh];
@@ -1382,13 +1400,13 @@ LD int partner_shape(const StepArgs& a, int pid) {
 // k_contacts_f; a pair without such nodes gets its empty contact segment here.
 template <int KIND, int SDFK, bool LRN>
 LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* s_cl, unsigned short* s_sub,
-                      unsigned* s_mask, unsigned (&cnt)[8]) {
+                      unsigned* s_mask, unsigned (&cnt)[8], unsigned& queued) {
   const int lane = threadIdx.x & 31;
   __syncwarp();  // the previous pair's write pass may still read s_cl / s_mask
   const int shA = a.P.shape[A];
   const int n0 = a.S.node_off[shA], nn = a.S.node_cnt[shA], cl0 = a.S.cl_off[shA], ncl = a.S.cl_cnt[shA];
   const float scA = (float)a.P.scale[A];
-  const double3 xA = a.P.pos[A];
+  const double3 xA = owner_pos<KIND>(a, A);
   PairF F;
   {
     const Partner P = load_partner<KIND>(a, pid);
@@ -1558,6 +1576,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
     }
   }
   cnt[5] += total;
+  queued += total;
   __syncwarp();
   const SlotView& cur = slots_of<KIND>(a, false);
   const size_t sidx = (size_t)A * cur.cap + slot;
@@ -1603,39 +1622,41 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
 // Particle-only screens fit 64 registers (8 blocks per SM); walls and images
 // need the window test's FP64 registers.
 template <int KINDS, int SDFK, bool LRN>
-__global__ void __launch_bounds__(NP_WARPS * 32, KINDS == 1 ? 8 : 5) k_screen_f(StepArgs a, int li) {
+__global__ void __launch_bounds__(NP_WARPS * 32, KINDS == 1 ? 8 : 5) k_screen_f(StepArgs a, int li, int kinds) {
   __shared__ int s_cl[NP_WARPS][MAXCL];
   __shared__ unsigned short s_sub[NP_WARPS][4 * MAXCL];
   __shared__ unsigned s_mask[NP_WARPS][MAXCL];
   const int warp = threadIdx.x >> 5;
   const int n0 = (KINDS & 1) ? min(a.pl.ctr[0], a.P.n * a.pp.cap) : 0;
-  const int n1 = (KINDS & 2) && a.pw.cap > 0 ? min(a.pl.ctr[1], a.P.n * a.pw.cap) : 0;
-  const int n2 = (KINDS & 4) ? min(a.pl.ctr[2], a.P.n * a.pgh.cap) : 0;
+  const int n1 = (kinds & KINDS & 2) && a.pw.cap > 0 ? min(a.pl.ctr[1], a.P.n * a.pw.cap) : 0;
+  const int n2 = (kinds & KINDS & 4) ? min(a.pl.ctr[2], a.P.n * a.pgh.cap) : 0;
   const int tot = n0 + n1 + n2;
   unsigned cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // warp-uniform screen counters
+  unsigned queued[3] = {0, 0, 0};              // nodes queued by partner kind
   for (int e = blockIdx.x * NP_WARPS + warp; e < tot; e += gridDim.x * NP_WARPS) {
     if ((KINDS & 1) && e < n0) {
       const int idx = __ldg(a.pl.list[0] + e);
       const int A = idx / a.pp.cap;
       screen_pair_f<KIND_PP, SDFK, LRN>(a, A, idx - A * a.pp.cap, __ldg(a.pp.id + idx), li, s_cl[warp], s_sub[warp],
-                                        s_mask[warp], cnt);
+                                        s_mask[warp], cnt, queued[0]);
     } else if ((KINDS & 2) && e < n0 + n1) {
       const int idx = a.pl.list[1][e - n0];
       const int A = idx / a.pw.cap;
       screen_pair_f<KIND_WALL, SDFK, LRN>(a, A, idx - A * a.pw.cap, a.pw.id[idx], li, s_cl[warp], s_sub[warp],
-                                          s_mask[warp], cnt);
+                                          s_mask[warp], cnt, queued[1]);
     } else if (KINDS & 4) {
       const int idx = __ldg(a.pl.list[2] + e - n0 - n1);
       const int A = idx / a.pgh.cap;
       screen_pair_f<KIND_GHOST, SDFK, LRN>(a, A, idx - A * a.pgh.cap, __ldg(a.pgh.id + idx), li, s_cl[warp], s_sub[warp],
-                                           s_mask[warp], cnt);
+                                           s_mask[warp], cnt, queued[2]);
     }
   }
   if (a.screen_stats && (threadIdx.x & 31) == 0) {
     for (int k = 0; k < 8; ++k)
       if (cnt[k]) atomicAdd(&a.screen_stats[k], (unsigned long long)cnt[k]);
-    // grid screen: nodes queued for the FP64 test by partner kind (one kind per launch)
-    if (!LRN && cnt[5]) atomicAdd(&a.screen_stats[8 + (KINDS == 1 ? 0 : (KINDS == 2 ? 1 : 2))], (unsigned long long)cnt[5]);
+    // grid screen: nodes queued for the FP64 test by partner kind
+    for (int k = 0; k < 3; ++k)
+      if (!LRN && queued[k]) atomicAdd(&a.screen_stats[8 + k], (unsigned long long)queued[k]);
   }
 }
 
@@ -1645,7 +1666,7 @@ template <int KIND>
 LD void contacts_pair(const StepArgs& a, int A, int slot, int start, int cnt, unsigned* s_mask, int* s_old) {
   const int lane = threadIdx.x & 31;
   const int pid = slots_of<KIND>(a, false).id[(size_t)A * slots_of<KIND>(a, false).cap + slot];
-  const SelfCtx S = self_ctx(a, A);
+  const SelfCtx S = self_ctx<KIND>(a, A);
   const Partner P = load_partner<KIND>(a, pid);
   const int* nodes = a.mb.node + start;
   const int nch = (cnt + 31) >> 5;
@@ -1844,8 +1865,8 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_net_compact(StepArgs a, int l
 }
 
 template <int KINDS, int SDFK, bool LRN>
-void launch_screen_k(const StepArgs& a, int li, dim3 g, dim3 b, cudaStream_t s) {
-  k_screen_f<KINDS, SDFK, LRN><<<g, b, 0, s>>>(a, li);
+void launch_screen_k(const StepArgs& a, int li, int kinds, dim3 g, dim3 b, cudaStream_t s) {
+  k_screen_f<KINDS, SDFK, LRN><<<g, b, 0, s>>>(a, li, kinds);
 }
 
 // Learned form: the network pass and the compaction after the screen of launch li.
@@ -1873,17 +1894,15 @@ void launch_net_compact(const StepArgs& a, int li, cudaStream_t s) {
 }
 
 template <bool LRN>
-// Particle and wall pairs in two launches: the particle-only screen fits 64 registers
-// (8 blocks per SM); the wall pairs (few) take the window test's FP64 registers.
+// Particle pairs, and wall and image pairs, in two launches: the particle-only screen fits 64
+// registers (8 blocks per SM); the others (few) take the window test's FP64 registers.
 void launch_screen(const StepArgs& a, int kinds, int li, dim3 g, dim3 b, cudaStream_t s) {
   if (a.precision == PREC_FP32_FP16) {
-    if (kinds & 1) launch_screen_k<1, PREC_FP32_FP16, LRN>(a, li, g, b, s);
-    if (kinds & 2) launch_screen_k<2, PREC_FP32_FP16, LRN>(a, li, g, b, s);
-    if (kinds & 4) launch_screen_k<4, PREC_FP32_FP16, LRN>(a, li, g, b, s);
+    if (kinds & 1) launch_screen_k<1, PREC_FP32_FP16, LRN>(a, li, kinds, g, b, s);
+    if (kinds & 6) launch_screen_k<6, PREC_FP32_FP16, LRN>(a, li, kinds, g, b, s);
   } else {
-    if (kinds & 1) launch_screen_k<1, PREC_FP32_BF16, LRN>(a, li, g, b, s);
-    if (kinds & 2) launch_screen_k<2, PREC_FP32_BF16, LRN>(a, li, g, b, s);
-    if (kinds & 4) launch_screen_k<4, PREC_FP32_BF16, LRN>(a, li, g, b, s);
+    if (kinds & 1) launch_screen_k<1, PREC_FP32_BF16, LRN>(a, li, kinds, g, b, s);
+    if (kinds & 6) launch_screen_k<6, PREC_FP32_BF16, LRN>(a, li, kinds, g, b, s);
   }
 }
 
@@ -1895,6 +1914,7 @@ void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s) {
   const dim3 g(blocks), b(NP_WARPS * 32);
   if (a.precision == PREC_FP64) {
     if (kinds == 3) k_narrowphase<3><<<g, b, 0, s>>>(a);
+    else if (kinds == 5) k_narrowphase<5><<<g, b, 0, s>>>(a);
     else if (kinds == 1) k_narrowphase<1><<<g, b, 0, s>>>(a);
     else if (kinds == 4) k_narrowphase<4><<<g, b, 0, s>>>(a);
     else k_narrowphase<7><<<g, b, 0, s>>>(a);
@@ -1902,7 +1922,7 @@ void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s) {
   }
   // precision form: the screen over the flat pair lists (launch_contact_pass
   // follows it); the grid is sized for the device, the list length is on it
-  const int li = kinds == 4 ? 1 : 0;
+  const int li = kinds == 4 && !a.gl.list ? 1 : 0;
   if (a.mlp_inf) launch_screen<true>(a, kinds, li, g, b, s);  // launch_net_screen and _compact follow
   else launch_screen<false>(a, kinds, li, g, b, s);
 }
@@ -1919,30 +1939,6 @@ void launch_contact_pass(const StepArgs& a, int li, cudaStream_t s) {
 // of PeriodicBoundaryXY2D::updateGhostSpatialGrid, PeriodicBoundary.h:215-288).
 // Ghost keys follow calculateGhostHashKernel (mySpatialGrid.cu:214-240),
 // including its z-upper test against the y bound.
-LD void ghost_image(double3 p, const GridP& g, int mask, double3& out) {
-  const int3 c = cell_of(p, g);
-  bool hit = true;
-  if (mask & 1) hit = hit && c.x == 0;
-  if (mask & 2) hit = hit && c.y == 0;
-  if (mask & 4) hit = hit && c.z == 0;
-  out = p;
-  if (hit) {
-    double3 off = d3(0., 0., 0.);
-    if (mask & 1) off = off + d3(g.mx.x - g.mn.x, 0., 0.);
-    if (mask & 2) off = off + d3(0., g.mx.y - g.mn.y, 0.);
-    if (mask & 4) off = off + d3(0., 0., g.mx.z - g.mn.z);
-    out += off;
-  }
-}
-LD int ghost_key(double3 p, const GridP& g) {
-  int3 c = cell_of(p, g);
-  bool out = false;
-  if (p.x < g.mn.x) { c.x = 0; out = true; } else if (p.x >= g.mx.x) { c.x = g.size.x - 1; out = true; }
-  if (p.y < g.mn.y) { c.y = 0; out = true; } else if (p.y >= g.mx.y) { c.y = g.size.y - 1; out = true; }
-  if (p.z < g.mn.z) { c.z = 0; out = true; } else if (p.z >= g.mx.y) { c.z = g.size.z - 1; out = true; }
-  return out ? lin3(c, g.size) : -1;
-}
-
 // Sector periodicity about the z axis through the domain minimum m: a particle
 // left of x = m.x (with y >= m.y) is turned by -90 degrees about that axis, one
 // below y = m.y (with x >= m.x) by +90 degrees: position about m, velocity and
@@ -2018,9 +2014,7 @@ __global__ void k_periodic(StepArgs a, int axes, double3* __restrict__ out) {
   const int n = a.P.n;
   for (int ax = 0; ax < 3; ++ax) {
     if (!((axes >> ax) & 1)) continue;
-    if (ax == 0) { const double L = g.mx.x - g.mn.x; if (p.x < g.mn.x) p.x += L; else if (p.x >= g.mx.x) p.x -= L; }
-    if (ax == 1) { const double L = g.mx.y - g.mn.y; if (p.y < g.mn.y) p.y += L; else if (p.y >= g.mx.y) p.y -= L; }
-    if (ax == 2) { const double L = g.mx.z - g.mn.z; if (p.z < g.mn.z) p.z += L; else if (p.z >= g.mx.z) p.z -= L; }
+    p = wrap_axis(p, g, ax);
     for (int s = 0; s < a.G.nsets; ++s)
       if (a.G.mask[s] == (1 << ax)) ghost_image(p, g, a.G.mask[s], a.G.gpos[(size_t)s * n + i]);
   }
@@ -2065,19 +2059,6 @@ __global__ void k_ghost_compact(StepArgs a) {
   if (vis) a.G.list[base + __popc(m & lanemask_lt())] = (int)t;
 }
 
-// Cell range along one axis of a ball (centre p, radius r) on the clamped grid,
-// intersected with [c - 2, c + 2].
-LD int axis_lo(double p, double mn, double inv, int size, double r, int c) {
-  int v = (int)floor((p - mn - r) * inv);
-  v = v < 0 ? 0 : (v > size - 1 ? size - 1 : v);
-  return v > c - 2 ? v : c - 2;
-}
-LD int axis_hi(double p, double mn, double inv, int size, double r, int c) {
-  int v = (int)floor((p - mn + r) * inv);
-  v = v < 0 ? 0 : (v > size - 1 ? size - 1 : v);
-  return v < c + 2 ? v : c + 2;
-}
-
 // Ghost partners, searched with one warp per visible image G: a node of A can
 // only reach G's cell window when A's clamped cell is within 2 cells of G's
 // cell, and only when A's bounding sphere reaches G's SDF grid box. The lanes
@@ -2095,10 +2076,7 @@ __global__ void k_ghost_candidates(StepArgs a, const int* __restrict__ g2_idx, c
     const double3 xg = a.G.gpos[t];
     const int cx = gk % g.size.x, cy = (gk / g.size.x) % g.size.y, cz = gk / (g.size.x * g.size.y);
     // circumradius of the image's SDF grid box about its centre
-    double3 lo, hi;
-    grid_box(a.P.origin[i], a.P.invh[i], a.S.gsize[a.P.shape[i]], lo, hi);
-    const double3 far = d3(fmax(fabs(lo.x), fabs(hi.x)), fmax(fabs(lo.y), fabs(hi.y)), fmax(fabs(lo.z), fabs(hi.z)));
-    const double Rg = len(far);
+    const double Rg = grid_reach(a, i);
     const int pid = (i << 3) | s;
     // A candidate lies within rmax + Rg of the image, so its clamped cell lies in
     // the per-axis cell range of that ball (edge cells are open outward: they
@@ -2164,6 +2142,93 @@ __global__ void k_ghost_candidates(StepArgs a, const int* __restrict__ g2_idx, c
   }
   need = __reduce_max_sync(FULL, need);
   if (lane == 0 && need > 0) atomicMax(&a.status->need_ghost, need);
+}
+
+// Image partners from the image list (k_rebuild, neighbours.cu): one thread per listed pair of
+// an owner A and an image, which stands at the particle moved by the domain or at the particle
+// itself (entry's high bit: moved). The pair is a candidate of this step when the image is
+// visible and stands so now, A's clamped cell is among the cells that k_ghost_candidates
+// walks for it, the spheres reach and no direction separates the two. Positions are the wrapped
+// ones. Writes the position and the cell of the images it passes on. (The image search of a step
+// was a wrap of all particles, a second cell sort and a walk, 18 launches beside the particles'
+// own: a step of 100k polydisperse particles took 199 us with them and takes 146 us now, one of
+// 2M settling particles 1105 and 665 us.)
+__global__ void __launch_bounds__(128) k_image_candidates(StepArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int m = min(*a.gl.count, a.gl.cap), n = a.P.n;
+  const GridP& g = a.pg;
+  const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
+  int need = 0;
+  for (int e0 = (blockIdx.x * blockDim.x + threadIdx.x) - lane; e0 < m; e0 += gridDim.x * blockDim.x) {
+    int slot = -1, A = 0;
+    if (e0 + lane < m) {
+      const int2 e = a.gl.list[e0 + lane];
+      A = e.x & 0x7fffffff;
+      const int i = e.y >> 3, s = e.y & 7;
+      const double3 base = image_base(a.P.pos[i], g, a.wrap_axes, a.G.mask[s]);
+      const bool hit = image_hit(base, g, a.G.mask[s]);
+      const double3 xg = hit ? base + image_offset(g, a.G.mask[s]) : base;
+      const int key = ghost_key(xg, g);
+      bool cand = key >= 0 && hit == (e.x < 0);
+      if (cand) {
+        const double3 xA = wrap_pos(a.P.pos[A], g, a.wrap_axes);
+        const int3 c = make_int3(key % g.size.x, (key / g.size.x) % g.size.y, key / (g.size.x * g.size.y));
+        const int3 cA = clamp_cell(cell_of(xA, g), g.size);
+        const double Rg = grid_reach(a, i);
+        const double reach = (a.rmax + Rg) * (1.0 + 1e-6) + coord_slack(xg, xg);
+        cand = cA.x >= axis_lo(xg.x, g.mn.x, g.inv.x, g.size.x, reach, c.x) &&
+               cA.x <= axis_hi(xg.x, g.mn.x, g.inv.x, g.size.x, reach, c.x) &&
+               cA.y >= axis_lo(xg.y, g.mn.y, g.inv.y, g.size.y, reach, c.y) &&
+               cA.y <= axis_hi(xg.y, g.mn.y, g.inv.y, g.size.y, reach, c.y) &&
+               cA.z >= axis_lo(xg.z, g.mn.z, g.inv.z, g.size.z, reach, c.z) &&
+               cA.z <= axis_hi(xg.z, g.mn.z, g.inv.z, g.size.z, reach, c.z);
+        if (cand) {
+          int kA, kB;
+          CandRec ra = cand_rec(a, A, kA), rb = cand_rec(a, i, kB);
+          ra.p = make_float4((float)xA.x, (float)xA.y, (float)xA.z, ra.p.w);
+          rb.p = make_float4((float)xg.x, (float)xg.y, (float)xg.z, 0.f);
+          const float R = (ra.p.w + (float)Rg) * (1.0f + 1e-5f) + 1e-6f * (n1_f(rb.p) + n1_f(ra.p));
+          cand = !(dist2_f(ra.p, rb.p) > R * R) &&
+                 !pair_separated(sup, ra.p, n1_f(ra.p), ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh);
+        }
+        if (cand) {
+          a.G.gpos[(size_t)s * n + i] = xg;  // the same from every entry of the image
+          a.G.gkey[(size_t)s * n + i] = key;
+          slot = atomicAdd(&a.pgh.cnt[A], 1);
+          if (slot < a.pgh.cap) a.pgh.id[(size_t)A * a.pgh.cap + slot] = e.y;
+          else atomicOr(&a.status->flags, OVF_GHOST);
+        }
+      }
+    }
+    need = max(need, slot + 1);
+    if (a.pl.ctr) {  // precision form: flat pair list
+      const bool ok = slot >= 0 && slot < a.pgh.cap;
+      const unsigned mk = __ballot_sync(FULL, ok);
+      int at = 0;
+      if (lane == 0 && mk) at = atomicAdd(&a.pl.ctr[2], __popc(mk));
+      at = __shfl_sync(FULL, at, 0);
+      if (ok) a.pl.list[2][at + __popc(mk & lanemask_lt())] = A * a.pgh.cap + slot;
+    }
+  }
+  need = __reduce_max_sync(FULL, need);
+  if (lane == 0 && need > 0) atomicMax(&a.status->need_ghost, need);
+}
+
+void launch_image_candidates(const StepArgs& a, cudaStream_t s) {
+  if (a.P.n > 0) k_image_candidates<<<std::min((a.P.n + 127) / 128, num_sms() * 4), 128, 0, s>>>(a);
+}
+
+// The step's wrap, in place after everything that reads the positions before it. A body beyond a
+// periodic face has set the rebuild flag (k_integrate_first), so most steps return at once.
+__global__ void k_wrap(StepArgs a) {
+  if (*a.reuse == 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.P.n) return;
+  const double3 x = a.P.pos[i], p = wrap_pos(x, a.pg, a.wrap_axes);
+  if (p.x != x.x || p.y != x.y || p.z != x.z) a.P.pos[i] = p;
+}
+void launch_wrap(const StepArgs& a, cudaStream_t s) {
+  if (a.P.n > 0) k_wrap<<<(a.P.n + 255) / 256, 256, 0, s>>>(a);
 }
 
 void launch_ghost_candidates(const StepArgs& a, const int* g2_idx, const int* g2_off, cudaStream_t s) {
