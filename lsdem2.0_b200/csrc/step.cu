@@ -931,10 +931,9 @@ LD bool node_hits(const StepArgs& a, const SelfCtx& S, const Partner& P, int ni)
 // Contact geometry, carried-over spring and linear contact force of one
 // admitted node (LSParticleContactDetectionKernel.cu:63-115, contactKernel.cu:75-117 /
 // :155-190 / :225-270); writes the contact at pos.
-template <int KIND>
 LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, const PairK& K, int ni, int ostart,
-                     int ocnt, bool staged, const int* s_old, int pos, bool can_write, double3& FA, double3& TA,
-                     double3& FB, double3& TB) {
+                     int ocnt, int pos, bool can_write, double3& FA, double3& TA, double3& FB, double3& TB,
+                     const int* s_old = nullptr) {
   const double3 w = node_world(a, S, ni);
   double ov, fx, fy, fz, cr[8];
   sdf_eval(w, P, ov, fx, fy, fz, cr);
@@ -947,7 +946,7 @@ LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, cons
   int lo = 0, hi = ocnt - 1;
   while (lo <= hi) {
     const int mid = (lo + hi) >> 1;
-    const int v = staged ? s_old[mid] : a.C_old.node[ostart + mid];
+    const int v = s_old ? s_old[mid] : a.C_old.node[ostart + mid];
     if (v == ni) { spring = a.C_old.spring[ostart + mid]; break; }
     if (v < ni) lo = mid + 1; else hi = mid - 1;
   }
@@ -1024,8 +1023,8 @@ LD void finish_pair(const StepArgs& a, int A, int slot, int pid, const SelfCtx& 
     const unsigned m = s_mask[k];
     if (m == 0) continue;
     if ((m >> lane) & 1u)
-      contact_node<KIND>(a, S, P, K, node_at(k), ostart, ocnt, staged, s_old,
-                         base + off + __popc(m & lanemask_lt()), can_write, FA, TA, FB, TB);
+      contact_node(a, S, P, K, node_at(k), ostart, ocnt, base + off + __popc(m & lanemask_lt()), can_write, FA, TA, FB,
+                   TB, staged ? s_old : nullptr);
     off += __popc(m);
   }
   if (KIND != KIND_WALL && !(KIND == KIND_GHOST && P.real == A)) {
@@ -1378,17 +1377,6 @@ LD bool cluster_may_hit_f(const PairF& F, float4 cn, float scA, float* up = null
 }
 
 template <int KIND>
-LD SelfCtx self_ctx(const StepArgs& a, int A) {
-  SelfCtx S;
-  S.x = owner_pos<KIND>(a, A); S.v = a.P.vel[A]; S.w = a.P.angvel[A]; S.q = a.P.quat[A];
-  S.sc = a.P.scale[A];
-  const int sh = a.P.shape[A];
-  S.n0 = a.S.node_off[sh]; S.nn = a.S.node_cnt[sh];
-  S.cl0 = a.S.cl_off[sh]; S.ncl = a.S.cl_cnt[sh];
-  return S;
-}
-
-template <int KIND>
 LD int partner_shape(const StepArgs& a, int pid) {
   if (KIND == KIND_WALL) return a.W.shape[pid];
   return a.P.shape[KIND == KIND_GHOST ? (pid >> 3) : pid];
@@ -1660,49 +1648,146 @@ __global__ void __launch_bounds__(NP_WARPS * 32, KINDS == 1 ? 8 : 5) k_screen_f(
   }
 }
 
-// Queued pairs of the screen, one warp each, in FP64: the reference's node test
-// on the screened nodes, then finish_pair (segment, history, forces).
-template <int KIND>
-LD void contacts_pair(const StepArgs& a, int A, int slot, int start, int cnt, unsigned* s_mask, int* s_old) {
-  const int lane = threadIdx.x & 31;
-  const int pid = slots_of<KIND>(a, false).id[(size_t)A * slots_of<KIND>(a, false).cap + slot];
-  const SelfCtx S = self_ctx<KIND>(a, A);
-  const Partner P = load_partner<KIND>(a, pid);
-  const int* nodes = a.mb.node + start;
-  const int nch = (cnt + 31) >> 5;
-  __syncwarp();  // the previous pair may still read s_mask / s_old
-  int total = 0;
-  for (int k = 0; k < nch; ++k) {
-    const int j = k * 32 + lane;
-    const bool hit = j < cnt && node_hits<KIND>(a, S, P, nodes[j]);
-    const unsigned m = __ballot_sync(FULL, hit);
-    if (lane == 0) s_mask[k] = m;
-    total += __popc(m);
-  }
-  __syncwarp();
-  double3 FA = d3(0., 0., 0.), TA = d3(0., 0., 0.);
-  finish_pair<KIND>(a, A, slot, pid, S, P, [&](int k) { return nodes[k * 32 + lane]; }, s_mask, s_old, nch, total,
-                    FA, TA);
-  FA = warp_sum3(FA);
-  TA = warp_sum3(TA);
-  if (lane == 0 && total > 0) {
-    atomic_add3(a.P.force, A, FA);
-    atomic_add3(a.P.torque, A, TA);
-  }
+// The partner of a pair whose kind is a value.
+LD Partner load_partner_of(const StepArgs& a, int kind, int pid) {
+  if (kind == KIND_WALL) return load_partner<KIND_WALL>(a, pid);
+  return kind == KIND_GHOST ? load_partner<KIND_GHOST>(a, pid) : load_partner<KIND_PP>(a, pid);
 }
 
-__global__ void __launch_bounds__(NP_WARPS * 32) k_contacts_f(StepArgs a, int li) {
-  __shared__ unsigned s_mask[NP_WARPS][MAXCL];
-  __shared__ int s_old[NP_WARPS][OLDCAP];
-  const int warp = threadIdx.x >> 5;
+// Queued pairs of the screen in FP64: the reference's node test on the screened nodes, then
+// each pair's contact segment, history and forces.
+//
+// A warp takes up to 32 pairs and runs their nodes, then their contacts, one lane each, whichever
+// pair they are of. A pair of a bed has 1.5 queued nodes and 0.7 contacts, so that a warp per
+// pair left 30 of its lanes idle through a chain of dependent loads, eight warps an SM (100k
+// bodies with 336k contacts: CON_OLD us that way, CON_NEW us now). With few pairs a warp takes
+// one, and the lanes are its nodes as before.
+// Between the two runs a pair's hits stand at the front of its part of the node queue, in node
+// order; one atomic per warp reserves the segments of its pairs.
+__global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int li) {
+  __shared__ int4 s_pair[NP_WARPS][32];   // {A, partner, first node, hits}
+  __shared__ int4 s_seg[NP_WARPS][32];    // {segment (-1: does not fit), old segment, its length, kind}
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int4* pair = s_pair[warp];
+  int4* seg = s_seg[warp];
   const int np = min(a.mb.ctr[1 + li], a.mb.pcap);
-  for (int p = blockIdx.x * NP_WARPS + warp; p < np; p += gridDim.x * NP_WARPS) {
-    const int4 e = a.mb.pair[(size_t)li * a.mb.pcap + p];
-    if (e.x < 0) continue;  // reserved by a pair whose nodes did not fit the queue
+  const int W = gridDim.x * NP_WARPS;
+  const int per = min(32, (np + W - 1) / W);
+  for (int p0 = (blockIdx.x * NP_WARPS + warp) * per; p0 < np; p0 += W * per) {
+    __syncwarp();  // the previous pairs' records are still read
+    int4 e = make_int4(-1, 0, 0, 0);  // A < 0: reserved by a pair whose nodes did not fit the queue
+    if (lane < per && p0 + lane < np) e = a.mb.pair[(size_t)li * a.mb.pcap + p0 + lane];
     const int kind = e.y >> 24, slot = e.y & 0xffffff;
-    if (kind == KIND_PP) contacts_pair<KIND_PP>(a, e.x, slot, e.z, e.w, s_mask[warp], s_old[warp]);
-    else if (kind == KIND_WALL) contacts_pair<KIND_WALL>(a, e.x, slot, e.z, e.w, s_mask[warp], s_old[warp]);
-    else contacts_pair<KIND_GHOST>(a, e.x, slot, e.z, e.w, s_mask[warp], s_old[warp]);
+    const SlotView& cur = kind == KIND_PP ? a.pp : (kind == KIND_WALL ? a.pw : a.pgh);
+    const SlotView& old = kind == KIND_PP ? a.pp_old : (kind == KIND_WALL ? a.pw_old : a.pgh_old);
+    const size_t sidx = e.x >= 0 ? (size_t)e.x * cur.cap + slot : 0;
+    const int pid = e.x >= 0 ? cur.id[sidx] : 0;
+    const int cnt = e.x >= 0 ? e.w : 0;
+    pair[lane] = make_int4(e.x, pid, e.z, 0);
+    seg[lane].w = kind;
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    int total = __shfl_sync(FULL, incl, 31);
+    __syncwarp();
+    for (int i0 = 0; i0 < total; i0 += 32) {
+      const int i = i0 + lane;
+      const int ow = lane_of(incl, i), first = __shfl_sync(FULL, incl - cnt, ow);
+      const int4 pr = pair[ow];
+      bool hit = false;
+      int ni = 0;
+      if (i < total) {
+        ni = a.mb.node[pr.z + i - first];
+        const int k = seg[ow].w;
+        SelfCtx S;
+        S.x = a.P.pos[pr.x];
+        if (k == KIND_GHOST && a.wrap_axes) S.x = wrap_pos(S.x, a.pg, a.wrap_axes);
+        S.q = a.P.quat[pr.x];
+        S.sc = a.P.scale[pr.x];
+        S.n0 = a.S.node_off[a.P.shape[pr.x]];
+        const Partner P = load_partner_of(a, k, pr.y);
+        const double3 w = node_world(a, S, ni);
+        const bool in = k == KIND_PP ? node_admitted<KIND_PP>(a, w, P)
+                                     : (k == KIND_WALL ? node_admitted<KIND_WALL>(a, w, P) : node_admitted<KIND_GHOST>(a, w, P));
+        double ov, fx, fy, fz, cr[8];
+        hit = in && sdf_eval(w, P, ov, fx, fy, fz, cr);
+      }
+      const unsigned m = __ballot_sync(FULL, hit);
+      const int at = pr.w + __popc(m & lanemask_lt() & (~0u << max(min(first - i0, 31), 0)));
+      const int nx = __shfl_down_sync(FULL, ow, 1);
+      __syncwarp();
+      if (hit) a.mb.node[pr.z + at] = ni;
+      if (i < total && (lane == 31 || nx != ow || i + 1 == total)) pair[ow].w = at + hit;
+      __syncwarp();
+    }
+    // segments, and the previous step's of the same pairs
+    const int h = pair[lane].w;
+    incl = h;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    total = __shfl_sync(FULL, incl, 31);
+    int base = 0;
+    if (lane == 0 && total > 0) base = atomicAdd(a.C.count, total);
+    base = __shfl_sync(FULL, base, 0) + incl - h;
+    if (e.x >= 0) {
+      const bool fits = base + h <= a.C.cap;
+      int ostart = 0, ocnt = 0;
+      if (h > 0 && old.cnt != nullptr) {
+        const int on = min(old.cnt[e.x], old.cap);
+        for (int j = 0; j < on; ++j) {
+          if (old.id[(size_t)e.x * old.cap + j] != pid) continue;
+          ostart = old.seg_start[(size_t)e.x * old.cap + j];
+          ocnt = old.seg_cnt[(size_t)e.x * old.cap + j];
+          break;
+        }
+      }
+      cur.seg_start[sidx] = base;
+      cur.seg_cnt[sidx] = fits ? h : 0;
+      if (!fits) atomicOr(&a.status->flags, OVF_CONTACT);
+      seg[lane] = make_int4(fits ? base : -1, ostart, ocnt, kind);
+    }
+    __syncwarp();
+    for (int i0 = 0; i0 < total; i0 += 32) {
+      const int i = i0 + lane;
+      const int ow = lane_of(incl, i), first = __shfl_sync(FULL, incl - h, ow);
+      double3 FA = d3(0., 0., 0.), TA = FA, FB = FA, TB = FA;
+      int A = -1, real = -1;
+      if (i < total) {
+        const int4 pr = pair[ow], sg = seg[ow];
+        const int k = sg.w;
+        A = pr.x;
+        SelfCtx S;
+        S.x = a.P.pos[A];
+        if (k == KIND_GHOST && a.wrap_axes) S.x = wrap_pos(S.x, a.pg, a.wrap_axes);
+        S.v = a.P.vel[A]; S.w = a.P.angvel[A]; S.q = a.P.quat[A];
+        S.sc = a.P.scale[A];
+        S.n0 = a.S.node_off[a.P.shape[A]];
+        const Partner P = load_partner_of(a, k, pr.y);
+        const PairK K = k == KIND_WALL ? pair_constants<KIND_WALL>(a, A, P) : pair_constants<KIND_PP>(a, A, P);
+        contact_node(a, S, P, K, a.mb.node[pr.z + i - first], sg.y, sg.z, sg.x + i - first, sg.x >= 0, FA, TA, FB, TB);
+        // an image of the owner itself takes no reaction
+        if (!(k == KIND_GHOST && P.real == A)) real = P.real;
+      }
+      const int ow0 = __shfl_sync(FULL, ow, 0);
+      if (__all_sync(FULL, i >= total || ow == ow0)) {  // one pair: one atomic per component
+        FA = warp_sum3(FA); TA = warp_sum3(TA); FB = warp_sum3(FB); TB = warp_sum3(TB);
+        if (lane > 0) A = real = -1;
+      }
+      if (A >= 0) {
+        atomic_add3(a.P.force, A, FA);
+        atomic_add3(a.P.torque, A, TA);
+      }
+      if (real >= 0) {
+        atomic_add3(a.P.force, real, FB);
+        atomic_add3(a.P.torque, real, TB);
+      }
+    }
   }
 }
 
@@ -1929,7 +2014,7 @@ void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s) {
 
 void launch_contact_pass(const StepArgs& a, int li, cudaStream_t s) {
   if (a.P.n <= 0 || a.precision == PREC_FP64) return;
-  k_contacts_f<<<num_sms() * 4, NP_WARPS * 32, 0, s>>>(a, li);
+  k_contacts_f<<<num_sms() * 3, NP_WARPS * 32, 0, s>>>(a, li);
 }
 
 // ---------------------------------------------------------------------------
