@@ -18,7 +18,7 @@ namespace lsdem {
 enum { FIX_GRADIENT = 1, FIX_SQRTF = 2 };
 
 // Overflow bits of the device status word.
-enum { OVF_PP = 1, OVF_WALL = 2, OVF_GHOST = 4, OVF_CONTACT = 8, OVF_NBR = 16, OVF_NET = 32, OVF_IMG = 64 };
+enum { OVF_PP = 1, OVF_WALL = 2, OVF_GHOST = 4, OVF_CONTACT = 8, OVF_NBR = 16, OVF_NET = 32, OVF_IMG = 64, OVF_QUEUE = 128 };
 
 // Largest demands seen during a batch (whether or not they overflowed), used
 // to grow capacities ahead of an overflow.
@@ -33,6 +33,7 @@ struct Status {
   int need_netq;     // learned form: largest rows of one shape's network queue
   int need_pend;     // learned form: largest count of nodes awaiting the network
   int need_img;      // largest length of the image list
+  int need_queue;    // largest demand of the contact pass's queue (nodes, twice the pairs)
   int errors;        // a bounded wait in a kernel gave up (results of the batch not valid)
 };
 
@@ -59,8 +60,9 @@ struct ShapeView {
   const uint4* cell16;
   const long long* cell_off;    // per shape, into cell16
   const float4* node_pos_f;     // FP32 copy of node_pos
-  const float* lip;             // 2 per shape, in spacings: largest |phi| difference of grid
-                                //   neighbours; largest gradient-norm bound of a grid cell
+  const float* lip;             // 3 per shape, in spacings: largest |phi| difference of grid
+                                //   neighbours; largest gradient-norm bound of a grid cell; of
+                                //   a cell where phi takes values in [0, LIP_BAND] spacings
   // support tables (cube map of SUP_M x SUP_M cells per face, per shape, template units,
   // rounded up): per cell the values at its four corner directions (p, q), (p + 1, q),
   // (p, q + 1), (p + 1, q + 1) of the largest projection of the nodes (sup_n) and of the
@@ -69,6 +71,8 @@ struct ShapeView {
   const float4* sup_s;
   const float* sup_r;           // per shape: largest |p| of the solid's grid cells, rounded up
 };
+
+constexpr double LIP_BAND = 8.0;
 
 // Arithmetic form of the narrowphase and contact forces.
 enum { PREC_FP64 = 0, PREC_FP32_FP16 = 1, PREC_FP32_BF16 = 2 };
@@ -103,8 +107,6 @@ struct BodyView {
   const double* invh;        // inverse grid spacing (scaled)
   const long long* node_base;  // global id of the first surface node (particles)
   int* key;                  // cell key of this step, -1 outside the domain
-  float4* rotm;              // precision form, particles: rows of the FP32 rotation matrix
-                             //   of quat (3 per body, written by k_integrate_first)
 };
 
 // Per-particle candidate slots of one partner kind, with the contact segment
@@ -166,7 +168,7 @@ void scan_i64(const long long* in, long long* out, long long n, long long* tmp, 
 void bucket_sort(const int* key, int n, int ncells, BucketScratch& w, int* sorted_idx, int* sorted_key, int* start,
                  int* end, cudaStream_t s, const int* gate = nullptr);
 
-// Precision form: nodes the FP32 screen could not reject, by pair, for the FP64
+// Nodes the FP32 screen could not reject, by pair, for the FP64
 // contact pass. One node cursor per step; one pair list per narrowphase launch
 // (0: particles and walls, 1: periodic images).
 struct MaybeView {
@@ -177,12 +179,12 @@ struct MaybeView {
   int* ctr;     // [0] node cursor, [1 + launch] pairs queued
 };
 
-// Precision form: flat lists of candidate pairs (A * cap + slot) per partner
+// Flat lists of candidate pairs (A * cap + slot) per partner
 // kind, appended by the candidate searches, so that the screen gives one warp
 // to each pair rather than to each owner particle.
 struct PairLists {
   int* list[3];  // particles, walls, images: n * cap entries each
-  int* ctr;      // [kind] entries appended this step (nullptr: lists not built)
+  int* ctr;      // [kind] entries appended this step
 };
 
 // Learned form, per narrowphase launch (0: particles and walls, 1: periodic images):
@@ -310,6 +312,7 @@ void mlp_infer(const MlpInfer* inf, const MlpNorm& nm, const double3* pts, int n
 void launch_integrate_first(const StepArgs& a, cudaStream_t s);
 void launch_candidates(const StepArgs& a, cudaStream_t s);
 void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s);
+bool one_screen(const StepArgs& a);  // all partner kinds of a step in one screen launch
 // precision form: FP64 contact pass over the pairs queued by the screen of
 // launch li (0: particles and walls, 1: periodic images)
 void launch_contact_pass(const StepArgs& a, int li, cudaStream_t s);

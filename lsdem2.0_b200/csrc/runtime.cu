@@ -281,7 +281,6 @@ struct BodyHost {
 struct BodyDev {
   DArr<double3> pos, vel, angvel, force, torque, origin;
   DArr<Quat> quat;
-  DArr<float4> rotm;  // precision form, particles: FP32 rotation matrix rows (written each step)
   DArr<double> invm, radius, kn, ks, mu, res, scale, invh;
   DArr<Sym6> invI;
   DArr<int> shape, key;
@@ -372,7 +371,8 @@ struct lsdem_solver {
   MlpTrainOpts mlp_opt;
   bool mlp_trained = false, mlp_on = false;
   DArr<int4> mb_pair;
-  long long mb_cap = 0, mb_pcap = 0;
+  long long mb_cap = 0, mb_pcap = 0, cap_mb = 0;
+  bool grow_mb = false;
   // learned form: network queues and pending nodes, per narrowphase launch
   struct NetDev {
     DArr<float4> row;
@@ -601,15 +601,15 @@ void alloc_slots(lsdem_solver* s, bool keep_unchanged = false) {
       CK(sl.seg_cnt.alloc(m));
       CK(sl.seg_cnt.zero(s->stream));
     }
-  // precision form: flat pair lists, one entry per slot
+  // flat pair lists, one entry per slot
   for (int k = 0; k < 3; ++k) {
     const int cap = s->slots[0][k].cap;
     const size_t m = (size_t)std::max(n, 1) * std::max(cap, 1);
-    if (s->precision == PREC_FP64 || cap == 0) { s->plist[k].release(); continue; }
-    if ((long long)n * cap > 0x7fffffffLL) throw Fail{LSDEM_ERR_NOMEM, "pair list index exceeds 32 bits"};
+    if (cap == 0) { s->plist[k].release(); continue; }
+    if ((long long)n * cap > 0xffffffffLL) throw Fail{LSDEM_ERR_NOMEM, "pair list index exceeds 32 bits"};
     if (s->plist[k].n != m) CK(s->plist[k].alloc(m));
   }
-  if (s->precision != PREC_FP64 && !s->pl_ctr.p) {
+  if (!s->pl_ctr.p) {
     CK(s->pl_ctr.alloc(4));
     CK(s->pl_ctr.zero(s->stream));
   }
@@ -657,10 +657,13 @@ void alloc_net(lsdem_solver* s) {
   s->net_dirty = false;
 }
 
-// Scratch of the precision form, sized with the contact capacity.
+// Queue of the screen: sized with the contact capacity in the precision forms, whose screens
+// leave the band of the 16-bit store to the FP64 test; the FP64 form's leaves little more than
+// the contacts themselves, of which few fill that capacity.
 void alloc_maybe(lsdem_solver* s) {
-  if (s->precision == PREC_FP64) return;
-  const long long cap = std::min<long long>(s->cap_c, 0x7fffffffLL);
+  const long long start = s->precision == PREC_FP64 ? std::max<long long>(1 << 16, 16LL * s->P.n()) : s->cap_c;
+  s->cap_mb = std::max(s->cap_mb, start);
+  const long long cap = std::min<long long>(s->cap_mb, 0x7fffffffLL);
   if (s->mb_cap == cap && s->mb_node.p) return;
   s->mb_cap = cap;
   s->mb_pcap = std::max<long long>(cap / 2, 1024);
@@ -705,8 +708,6 @@ void upload_bodies(lsdem_solver* s, BodyHost& H, BodyDev& D) {
   CK(D.shape.upload(H.shape.data(), n, st));
   CK(D.key.alloc(std::max<size_t>(n, 1)));
   if (!H.node_base.empty()) CK(D.node_base.upload(H.node_base.data(), n, st));
-  if (&D == &s->dP && s->precision != PREC_FP64) CK(D.rotm.alloc(3 * std::max<size_t>(n, 1)));
-  else D.rotm.release();
 }
 
 // Brings the host copies of the bodies' state up to date with the device after steps:
@@ -922,13 +923,14 @@ void initialize(lsdem_solver* s) {
     // per template, in spacings: the largest difference of neighbouring SDF values
     // (bound of each partial derivative of the trilinear interpolant per grid
     // unit) and the largest gradient-norm bound of a cell, sqrt of the sum over
-    // axes of the cell's largest edge difference squared
+    // axes of the cell's largest edge difference squared, over all cells and over those
+    // where phi takes values in [0, LIP_BAND] spacings
     std::vector<float> lip;
     for (const ShapeHost& sh : s->shapes) {
       const int nx = sh.size[0], ny = sh.size[1], nz = sh.size[2];
       const size_t sy = (size_t)nx, sz = (size_t)nx * ny;
       auto at = [&](int x, int y, int z) { return sh.sdf[(size_t)x + sy * y + sz * z]; };
-      double m = 0., g = 0.;
+      double m = 0., g = 0., gb = 0.;
       for (int z = 0; z + 1 < nz; ++z)
         for (int y = 0; y + 1 < ny; ++y)
           for (int x = 0; x + 1 < nx; ++x) {
@@ -940,15 +942,25 @@ void initialize(lsdem_solver* s) {
               e[2] = std::max(e[2], std::fabs(at(x + u, y + v, z + 1) - at(x + u, y + v, z)));
             }
             m = std::max(m, std::max(e[0], std::max(e[1], e[2])));
-            g = std::max(g, std::sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]));
+            const double ge = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
+            g = std::max(g, ge);
+            if (ge <= gb) continue;
+            double lo = 1e300, hi = -1e300;
+            for (int b = 0; b < 8; ++b) {
+              lo = std::min(lo, at(x + (b & 1), y + ((b >> 1) & 1), z + (b >> 2)));
+              hi = std::max(hi, at(x + (b & 1), y + ((b >> 1) & 1), z + (b >> 2)));
+            }
+            const double tol = 1e-9 * sh.h;
+            if (lo <= LIP_BAND * sh.h + tol && hi >= -tol) gb = ge;
           }
       lip.push_back((float)(m / sh.h * (1.0 + 1e-6)));
-      lip.push_back((float)(g / sh.h * (1.0 + 1e-6)));
+      lip.push_back((float)(std::sqrt(g) / sh.h * (1.0 + 1e-6)));
+      lip.push_back((float)(std::sqrt(gb) / sh.h * (1.0 + 1e-6)));
     }
     CK(s->s_lip.upload(lip.data(), lip.size(), st));
   }
   if (s->precision != PREC_FP64) {
-    // precision form: phi / h of each template in 16 bits, FP32 node copy
+    // precision form: phi / h of each template in 16 bits
     // cell-major 16-bit store: the 8 corners of cell (i, j, k) in 16 bytes, corner
     // c = dx + 2 dy + 4 dz at 16-bit lane c, cells x-fastest
     std::vector<uint4> cells;
@@ -977,11 +989,13 @@ void initialize(lsdem_solver* s) {
             cells.push_back(make_uint4(c[0] | c[1] << 16, c[2] | c[3] << 16, c[4] | c[5] << 16, c[6] | c[7] << 16));
           }
     }
+    CK(s->s_cell16.upload(cells.data(), cells.size(), st));
+    CK(s->s_cell_off.upload(cell_off.data(), cell_off.size(), st));
+  }
+  {
     std::vector<float4> nf(node_pos.size());
     for (size_t i = 0; i < node_pos.size(); ++i)
       nf[i] = make_float4((float)node_pos[i].x, (float)node_pos[i].y, (float)node_pos[i].z, 0.f);
-    CK(s->s_cell16.upload(cells.data(), cells.size(), st));
-    CK(s->s_cell_off.upload(cell_off.data(), cell_off.size(), st));
     CK(s->s_node_f.upload(nf.data(), nf.size(), st));
   }
   // node ids (LSBoundaryNode order: particle by particle, caller node order)
@@ -1065,7 +1079,8 @@ void initialize(lsdem_solver* s) {
     }
   }
   // history buffers
-  if (s->cap_c <= 0) s->cap_c = std::max<long long>(1 << 16, (long long)n * 128);
+  if (s->cap_c <= 0)  // the FP64 form's queue and pair lists come out of its share
+    s->cap_c = std::max<long long>(1 << 16, (long long)n * (s->precision == PREC_FP64 ? 120 : 128));
   alloc_slots(s);
   alloc_contacts(s, s->con[0], s->cap_c);
   alloc_contacts(s, s->con[1], s->cap_c);
@@ -1119,7 +1134,6 @@ StepArgs make_args(lsdem_solver* s, double dt) {
     v.quat = D.quat.p; v.invmass = D.invm.p; v.invI = D.invI.p; v.radius = D.radius.p; v.kn = D.kn.p;
     v.ks = D.ks.p; v.mu = D.mu.p; v.res = D.res.p; v.shape = D.shape.p; v.scale = D.scale.p;
     v.origin = D.origin.p; v.invh = D.invh.p; v.node_base = D.node_base.p; v.key = D.key.p;
-    v.rotm = D.rotm.p;
     return v;
   };
   a.P = bv(s->dP, s->P.n());
@@ -1197,9 +1211,9 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.pk_q = s->pk_q.p;
   a.mb.node = s->mb_node.p; a.mb.cap = (int)s->mb_cap;
   a.mb.pair = s->mb_pair.p; a.mb.pcap = (int)s->mb_pcap;
-  a.mb.ctr = s->precision == PREC_FP64 ? nullptr : s->mb_ctr.p;
+  a.mb.ctr = s->mb_ctr.p;
   for (int k = 0; k < 3; ++k) a.pl.list[k] = s->plist[k].p;
-  a.pl.ctr = s->precision == PREC_FP64 ? nullptr : s->pl_ctr.p;
+  a.pl.ctr = s->pl_ctr.p;
   a.screen_stats = s->scr_stats.p;
   const bool learned = s->mlp_on && s->mlp_trained && s->precision != PREC_FP64;
   a.mlp_inf = learned ? s->mlp_inf.p : nullptr;
@@ -1292,7 +1306,7 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
     CK(cudaStreamWaitEvent(s2, s->ev_fork, 0));
     launch_image_candidates(a, s2);
     launch_candidates(a, st);
-    if (s->precision == PREC_FP64) {
+    if (one_screen(a)) {
       CK(cudaEventRecord(s->ev_join, s2));
       CK(cudaStreamWaitEvent(st, s->ev_join, 0));
       launch_narrowphase(a, kinds, st);
@@ -1303,10 +1317,10 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
       CK(cudaEventRecord(s->ev_join, s2));
       launch_narrowphase(a, 1, st);
       CK(cudaStreamWaitEvent(st, s->ev_join, 0));
-      launch_net_screen(a, 0, st);
-      launch_net_compact(a, 0, st);
-      launch_contact_pass(a, 0, st);
     }
+    launch_net_screen(a, 0, st);
+    launch_net_compact(a, 0, st);
+    launch_contact_pass(a, 0, st);
     launch_wrap(a, st);
   } else if (a.gl.list) {
     {
@@ -1317,8 +1331,8 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
       PhaseTimer pt(s, 4);
       launch_image_candidates(a, st);
     }
-    { PhaseTimer pt(s, 3); launch_narrowphase(a, s->precision == PREC_FP64 ? kinds : (s->W.n() > 0 ? 3 : 1), st); }
-    if (s->precision != PREC_FP64) {
+    { PhaseTimer pt(s, 3); launch_narrowphase(a, kinds & 3, st); }
+    {
       { PhaseTimer pt(s, 5); launch_narrowphase(a, 4, st); }
       if (a.mlp_inf) { PhaseTimer pt(s, 10); launch_net_screen(a, 0, st); }
       PhaseTimer pt(s, 8);
@@ -1347,20 +1361,20 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
     launch_narrowphase(a2, 4, s2);
     launch_net_screen(a2, 1, s2);
     launch_net_compact(a2, 1, s2);
-    if (s->precision != PREC_FP64) launch_contact_pass(a2, 1, s2);
+    launch_contact_pass(a2, 1, s2);
     CK(cudaEventRecord(s->ev_join, s2));
     launch_candidates(a, st);
     launch_narrowphase(a, s->W.n() > 0 ? 3 : 1, st);
     launch_net_screen(a, 0, st);
     launch_net_compact(a, 0, st);
-    if (s->precision != PREC_FP64) launch_contact_pass(a, 0, st);
+    launch_contact_pass(a, 0, st);
     CK(cudaStreamWaitEvent(st, s->ev_join, 0));
     if (a.P.n > 0) CK(cudaMemcpyAsync(a.P.pos, s->pos_w.p, sizeof(double3) * a.P.n, cudaMemcpyDeviceToDevice, st));
   } else {
     { PhaseTimer pt(s, 2); launch_candidates(a, st); }
     { PhaseTimer pt(s, 3); launch_narrowphase(a, s->W.n() > 0 ? 3 : 1, st); }
     if (a.mlp_inf) { PhaseTimer pt(s, 10); launch_net_screen(a, 0, st); }
-    if (s->precision != PREC_FP64) {
+    {
       PhaseTimer pt(s, 8);
       launch_net_compact(a, 0, st);
       launch_contact_pass(a, 0, st);
@@ -1375,7 +1389,7 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
       }
       { PhaseTimer pt(s, 5); launch_narrowphase(a, 4, st); }
       if (a.mlp_inf) { PhaseTimer pt(s, 10); launch_net_screen(a, 1, st); }
-      if (s->precision != PREC_FP64) {
+      {
         PhaseTimer pt(s, 8);
         launch_net_compact(a, 1, st);
         launch_contact_pass(a, 1, st);
@@ -1391,13 +1405,12 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
   // kernels launched up to here: kick/drift/keys, cell sort and packing (11; one with
   // neighbour lists), candidates, narrowphase; periodic: image candidates and wrap, or
   // (images searched every step) wrap/images, clamped keys, cell sort (9), image compaction +
-  // packing + candidates, ghost narrowphase; bonds. The precision forms add one contact pass
-  // (per narrowphase, where images are searched every step) and a separate screen for walls
-  // and images; the learned form the network pass and the compaction after each screen.
-  const bool fp32 = s->precision != PREC_FP64;
+  // packing + candidates, ghost narrowphase; bonds. Also one contact pass (per narrowphase,
+  // where images are searched every step) and a separate screen for walls and images; the
+  // learned form adds the network pass and the compaction after each screen.
   const int lrn = a.mlp_inf ? 2 : 0;
-  const int nf = fp32 ? 1 + (s->W.n() > 0 || a.gl.list ? 1 : 0) + lrn : 0;
-  const int ng = a.gl.list ? 2 : 15 + (fp32 ? 1 + lrn : 0);
+  const int nf = 1 + ((s->W.n() > 0 || a.gl.list) && !one_screen(a) ? 1 : 0) + lrn;
+  const int ng = a.gl.list ? 2 : 15 + 1 + lrn;
   if (a.P.n > 0) s->launches += (a.nbr ? 4 : 14) + nf + (s->nsets > 0 ? ng : 0) + (s->bonds.bonded.empty() ? 0 : 1);
   CK(cudaGetLastError());
 }
@@ -1531,11 +1544,18 @@ bool plan_growth(lsdem_solver* s, const Status& st, long long last_contacts) {
       s->grow_img = changed = true;
     }
   }
-  const long long needc = std::max<long long>(st.need_contact, last_contacts);
-  if ((st.flags & OVF_CONTACT) || needc * 5 > s->cap_c * 4) {
+  // the precision forms' queue is sized with the contact capacity and grows with it
+  const bool queue_full = (st.flags & OVF_QUEUE) != 0, own = s->precision == PREC_FP64;
+  long long needc = std::max<long long>(st.need_contact, last_contacts);
+  if (!own && queue_full) needc = std::max<long long>(needc, st.need_queue);
+  if ((st.flags & OVF_CONTACT) || (!own && queue_full) || needc * 5 > s->cap_c * 4) {
     s->cap_c = std::max<long long>(s->cap_c * 2, needc + needc / 2 + 1024);
     changed = true;
     s->grow_contacts = true;
+  }
+  if (own && (queue_full || st.need_queue * 5LL > s->cap_mb * 4)) {
+    s->cap_mb = std::max<long long>(s->cap_mb * 2, st.need_queue + st.need_queue / 2LL + 1024);
+    s->grow_mb = changed = true;
   }
   if (changed) s->net_dirty = true;  // pair records are sized with the candidate slots
   // learned form: network rows per shape and pending nodes
@@ -1567,6 +1587,10 @@ void grow(lsdem_solver* s) {
   if (s->grow_nbr) {
     CK(s->nbr.alloc((size_t)std::max(s->P.n(), 1) * s->nbr_cap));
     s->grow_nbr = false;
+  }
+  if (s->grow_mb) {
+    alloc_maybe(s);
+    s->grow_mb = false;
   }
   if (s->grow_img) {
     CK(s->img_list.alloc((size_t)s->cap_img));

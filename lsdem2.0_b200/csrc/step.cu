@@ -1,4 +1,4 @@
-// Level-set DEM step kernels for sm_100a (FP64 "plain" form).
+// Level-set DEM step kernels for sm_100a.
 //
 // Kernel map against the reference hot path (paths relative to the reference root):
 //   k_integrate_first  half kick + drift + cell key (+ wall drift/key); replaces
@@ -7,9 +7,9 @@
 //                      calculateHashKernel (myUtility/mySpatialGrid.cu:4-26)
 //   k_candidates       particle-level candidate partners from the cell grid (new: replaces the
 //                      per-node 27-cell scan of LSParticleContactDetectionKernel.cu:44-61)
-//   k_narrowphase      node-vs-SDF tests (LSParticleContactDetectionKernel.cu:4-590), history
-//                      carry-over (…cu:280-289) and the linear contact force
-//                      (contactKernel.cuh:4-77, contactKernel.cu:46-271) fused in one pass
+//   k_screen_f         node-vs-SDF rejections (LSParticleContactDetectionKernel.cu:4-590), FP32
+//   k_contacts_f       node-vs-SDF tests of the rest, history carry-over (…cu:280-289) and the
+//                      linear contact force (contactKernel.cuh:4-77, contactKernel.cu:46-271)
 //   k_kick             second half kick (particleIntegrationKernel.cu:3-24)
 //   k_periodic         wrap + ghost images + ghost keys (mySpatialGrid.cu:28-56, 87-152, 214-240)
 //   k_bonds            V-bond forces (contactKernel.cuh:138-199, contactKernel.cu:273-351)
@@ -26,7 +26,6 @@ namespace lsdem {
 static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int NP_WARPS = 4;     // warps per narrowphase block
 static constexpr int MAXCL = 256;      // clusters of 32 nodes per shape (8192 nodes)
-static constexpr int OLDCAP = 256;     // previous-segment node ids staged in shared memory per warp
 
 LD unsigned lanemask_lt() {
   unsigned m;
@@ -97,12 +96,6 @@ __global__ void k_integrate_first(StepArgs a) {
     q = quat_integrate(q, w, a.dt);
     P.pos[i] = x;
     P.quat[i] = q;
-    if (P.rotm) {  // precision form: FP32 rotation matrix (columns are rotate(q, e_j))
-      const double3 c0 = rotate(q, d3(1., 0., 0.)), c1 = rotate(q, d3(0., 1., 0.)), c2 = rotate(q, d3(0., 0., 1.));
-      P.rotm[3 * i] = make_float4((float)c0.x, (float)c1.x, (float)c2.x, 0.f);
-      P.rotm[3 * i + 1] = make_float4((float)c0.y, (float)c1.y, (float)c2.y, 0.f);
-      P.rotm[3 * i + 2] = make_float4((float)c0.z, (float)c1.z, (float)c2.z, 0.f);
-    }
     P.force[i] = d3(0., 0., 0.);
     P.torque[i] = d3(0., 0., 0.);
     const int key = hash_key(x, a.pg);
@@ -189,7 +182,7 @@ LD void grid_box(const double3 o, double invh, int3 gs, double3& lo, double3& hi
 // box; for a node position p in the box |p - q| <= |p - l| (projection onto a
 // convex set does not expand distances), the segment p-q stays in the box, and
 // along it phi changes by at most the template's cell gradient-norm bound per
-// grid unit (lip[2 sh + 1] spacings per spacing). phi(q) is the FP64 trilinear
+// grid unit (lip[3 sh + 1] spacings per spacing). phi(q) is the FP64 trilinear
 // value of the grid, as the node test computes it, with a rounding margin.
 LD bool wall_far(const StepArgs& a, int w, double3 l, double reach) {
   const int sh = a.W.shape[w];
@@ -214,7 +207,7 @@ LD bool wall_far(const StepArgs& a, int w, double3 l, double reach) {
     acc += (v0 * (1.0 - fx) + v1 * fx) * (dy ? fy : 1.0 - fy) * (dz ? fz : 1.0 - fz);
   }
   const double phi = sc * acc;
-  const double bound = (double)a.S.lip[2 * sh + 1] * reach * (1.0 + 1e-9) + 1e-12 * sc * cmax + 1e-300;
+  const double bound = (double)a.S.lip[3 * sh + 1] * reach * (1.0 + 1e-9) + 1e-12 * sc * cmax + 1e-300;
   return phi > bound;
 }
 
@@ -231,7 +224,7 @@ LD void append_pairs(int* list, int* ctr, int A, int cap, int cnt) {
   int base = 0;
   if (lane == 31 && tot > 0) base = atomicAdd(ctr, tot);
   base = __shfl_sync(FULL, base, 31) + incl - cnt;
-  for (int j = 0; j < cnt; ++j) list[base + j] = A * cap + j;
+  for (int j = 0; j < cnt; ++j) list[base + j] = (int)((unsigned)A * cap + j);
 }
 
 // Centres and bounding radii in a sorted order (idx), FP32, for the candidate
@@ -414,13 +407,11 @@ LD int wall_candidates(const StepArgs& a, const WallBox* box, int A, double3 xA,
   return nw;
 }
 
-// End of a candidate kernel (all lanes of the warp): the flat pair lists of the precision
-// forms, the largest demands, one atomic per warp.
+// End of a candidate kernel (all lanes of the warp): the flat pair lists, the largest demands,
+// one atomic per warp.
 LD void candidates_done(const StepArgs& a, int A, bool on, int n, int nw) {
-  if (a.pl.ctr) {
-    append_pairs(a.pl.list[0], &a.pl.ctr[0], A, a.pp.cap, on ? min(n, a.pp.cap) : 0);
-    if (a.pw.cap > 0) append_pairs(a.pl.list[1], &a.pl.ctr[1], A, a.pw.cap, on ? min(nw, a.pw.cap) : 0);
-  }
+  append_pairs(a.pl.list[0], &a.pl.ctr[0], A, a.pp.cap, on ? min(n, a.pp.cap) : 0);
+  if (a.pw.cap > 0) append_pairs(a.pl.list[1], &a.pl.ctr[1], A, a.pw.cap, on ? min(nw, a.pw.cap) : 0);
   n = __reduce_max_sync(FULL, n);
   nw = __reduce_max_sync(FULL, nw);
   if ((threadIdx.x & 31) == 0) {
@@ -840,21 +831,6 @@ LD bool node_admitted(const StepArgs& a, double3 w, const Partner& P) {
   }
 }
 
-// Conservative cluster cull: false only when no node of the cluster can pass.
-template <int KIND>
-LD bool cluster_may_hit(double3 wc, double rad, const Partner& P) {
-  const double slack = coord_slack(wc, P.x);
-  if (KIND == KIND_PP) {
-    const double R = (P.r + rad) * (1.0 + 1e-9) + slack;
-    return len2(wc - P.x) <= R * R;
-  } else {
-    const double3 l = rotate_inv(wc - P.x, P.q);
-    double3 lo, hi;
-    grid_box(P.o, P.invh, P.gs, lo, hi);
-    return box_dist(l, lo, hi) <= rad * (1.0 + 1e-9) + slack + 1e-12 * len(hi - lo);
-  }
-}
-
 LD double sqrt_damp(double v, int flags) { return (flags & FIX_SQRTF) ? sqrt(v) : (double)sqrtf((float)v); }
 
 template <int KIND>
@@ -918,22 +894,11 @@ LD const SlotView& slots_of(const StepArgs& a, bool old) {
   return old ? a.pgh_old : a.pgh;
 }
 
-// The reference's per-node test in FP64: admission, then node inside the
-// partner's SDF grid with phi <= 0.
-template <int KIND>
-LD bool node_hits(const StepArgs& a, const SelfCtx& S, const Partner& P, int ni) {
-  const double3 w = node_world(a, S, ni);
-  if (!node_admitted<KIND>(a, w, P)) return false;
-  double ov, fx, fy, fz, cr[8];
-  return sdf_eval(w, P, ov, fx, fy, fz, cr);
-}
-
 // Contact geometry, carried-over spring and linear contact force of one
 // admitted node (LSParticleContactDetectionKernel.cu:63-115, contactKernel.cu:75-117 /
 // :155-190 / :225-270); writes the contact at pos.
 LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, const PairK& K, int ni, int ostart,
-                     int ocnt, int pos, bool can_write, double3& FA, double3& TA, double3& FB, double3& TB,
-                     const int* s_old = nullptr) {
+                     int ocnt, int pos, bool can_write, double3& FA, double3& TA, double3& FB, double3& TB) {
   const double3 w = node_world(a, S, ni);
   double ov, fx, fy, fz, cr[8];
   sdf_eval(w, P, ov, fx, fy, fz, cr);
@@ -946,7 +911,7 @@ LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, cons
   int lo = 0, hi = ocnt - 1;
   while (lo <= hi) {
     const int mid = (lo + hi) >> 1;
-    const int v = s_old ? s_old[mid] : a.C_old.node[ostart + mid];
+    const int v = a.C_old.node[ostart + mid];
     if (v == ni) { spring = a.C_old.spring[ostart + mid]; break; }
     if (v < ni) lo = mid + 1; else hi = mid - 1;
   }
@@ -970,161 +935,19 @@ LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, cons
   TB += cross(pc - P.x, -F);
 }
 
-// Second half of a pair, shared by both arithmetic forms: given the ballots of
-// admitted nodes per chunk of 32 (s_mask; node_at(k) is this lane's node of
-// chunk k, chunks in ascending node order), one
-// atomic reserves a contiguous segment ordered by node, the previous step's
-// segment of the same pair is located, and the contacts are evaluated and
-// written in FP64. The partner's reaction is reduced over the warp and added
-// with one atomic per component.
-template <int KIND, class NodeAt>
-LD void finish_pair(const StepArgs& a, int A, int slot, int pid, const SelfCtx& S, const Partner& P,
-                    NodeAt node_at, const unsigned* s_mask, int* s_old, int nsurv, int total, double3& FA,
-                    double3& TA) {
-  const int lane = threadIdx.x & 31;
-  const SlotView& cur = slots_of<KIND>(a, false);
-  const size_t sidx = (size_t)A * cur.cap + slot;
-  int base = 0;
-  if (lane == 0 && total > 0) base = atomicAdd(a.C.count, total);
-  base = __shfl_sync(FULL, base, 0);
-  const bool can_write = (base + total <= a.C.cap);
-  if (lane == 0) {
-    cur.seg_start[sidx] = base;
-    cur.seg_cnt[sidx] = can_write ? total : 0;
-    if (!can_write) atomicOr(&a.status->flags, OVF_CONTACT);
-  }
-  if (total == 0) return;
-  // previous segment of the same pair
-  const SlotView& old = slots_of<KIND>(a, true);
-  int ostart = 0, ocnt = 0;
-  if (old.cnt != nullptr) {
-    const int on = old.cnt[A] < old.cap ? old.cnt[A] : old.cap;
-    for (int j0 = 0; j0 < on; j0 += 32) {
-      const int j = j0 + lane;
-      const bool match = j < on && old.id[(size_t)A * old.cap + j] == pid;
-      const unsigned m = __ballot_sync(FULL, match);
-      if (m) {
-        const int src = j0 + __ffs(m) - 1;
-        ostart = old.seg_start[(size_t)A * old.cap + src];
-        ocnt = old.seg_cnt[(size_t)A * old.cap + src];
-        break;
-      }
-    }
-  }
-  // the previous segment's node ids in shared memory (binary-searched by every contact)
-  const bool staged = ocnt <= OLDCAP;
-  if (staged)
-    for (int j = lane; j < ocnt; j += 32) s_old[j] = a.C_old.node[ostart + j];
-  __syncwarp();
-  const PairK K = pair_constants<KIND>(a, A, P);
-  double3 FB = d3(0., 0., 0.), TB = d3(0., 0., 0.);
-  int off = 0;
-  for (int k = 0; k < nsurv; ++k) {
-    const unsigned m = s_mask[k];
-    if (m == 0) continue;
-    if ((m >> lane) & 1u)
-      contact_node(a, S, P, K, node_at(k), ostart, ocnt, base + off + __popc(m & lanemask_lt()), can_write, FA, TA, FB,
-                   TB, staged ? s_old : nullptr);
-    off += __popc(m);
-  }
-  if (KIND != KIND_WALL && !(KIND == KIND_GHOST && P.real == A)) {
-    FB = warp_sum3(FB);
-    TB = warp_sum3(TB);
-    if (lane == 0) {
-      atomic_add3(a.P.force, P.real, FB);
-      atomic_add3(a.P.torque, P.real, TB);
-    }
-  }
-}
-
-// Processes one (A, partner) pair with the whole warp in FP64: cluster culling,
-// then a first sweep over the surviving clusters that ballots the admitted
-// nodes, then finish_pair.
-template <int KIND>
-LD void do_pair(const StepArgs& a, int A, int slot, int pid, const SelfCtx& S, int* s_cl, unsigned* s_mask,
-                int* s_old, double3& FA, double3& TA) {
-  const int lane = threadIdx.x & 31;
-  __syncwarp();  // the previous pair's second sweep may still read s_cl / s_mask
-  const Partner P = load_partner<KIND>(a, pid);
-  // cluster culling
-  int nsurv = 0;
-  for (int c0 = 0; c0 < S.ncl; c0 += 32) {
-    const int c = c0 + lane;
-    bool keep = false;
-    if (c < S.ncl) {
-      const double4 sp = a.S.cl_sphere[S.cl0 + c];
-      const double3 wc = rotate(S.q, d3(sp.x, sp.y, sp.z) * S.sc) + S.x;
-      keep = cluster_may_hit<KIND>(wc, sp.w * S.sc, P);
-    }
-    const unsigned m = __ballot_sync(FULL, keep);
-    if (keep) s_cl[nsurv + __popc(m & lanemask_lt())] = c;
-    nsurv += __popc(m);
-  }
-  __syncwarp();
-  // sweep 1: admission + SDF test
-  int total = 0;
-  for (int k = 0; k < nsurv; ++k) {
-    const int ni = s_cl[k] * 32 + lane;
-    const bool hit = ni < S.nn && node_hits<KIND>(a, S, P, ni);
-    const unsigned m = __ballot_sync(FULL, hit);
-    if (lane == 0) s_mask[k] = m;
-    total += __popc(m);
-  }
-  __syncwarp();
-  finish_pair<KIND>(a, A, slot, pid, S, P, [&](int k) { return s_cl[k] * 32 + lane; }, s_mask, s_old, nsurv, total,
-                    FA, TA);
-}
-
-template <int KINDS>
-__global__ void __launch_bounds__(NP_WARPS * 32, 2) k_narrowphase(StepArgs a) {
-  __shared__ int s_cl[NP_WARPS][MAXCL];
-  __shared__ unsigned s_mask[NP_WARPS][MAXCL];
-  __shared__ int s_old[NP_WARPS][OLDCAP];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int ng_max = 0;
-  for (int A = blockIdx.x * NP_WARPS + warp; A < a.P.n; A += gridDim.x * NP_WARPS) {
-    const int npp = (KINDS & 1) ? a.pp.cnt[A] : 0;
-    const int nw = (KINDS & 2) ? (a.pw.cap > 0 ? a.pw.cnt[A] : 0) : 0;
-    const int ng = (KINDS & 4) ? a.pgh.cnt[A] : 0;
-    ng_max = ng > ng_max ? ng : ng_max;
-    const int ngc = ng < a.pgh.cap ? ng : a.pgh.cap;
-    if (npp + nw + ngc == 0) continue;
-    SelfCtx S;
-    S.x = a.P.pos[A]; S.v = a.P.vel[A]; S.w = a.P.angvel[A]; S.q = a.P.quat[A];
-    S.sc = a.P.scale[A];
-    const int sh = a.P.shape[A];
-    S.n0 = a.S.node_off[sh]; S.nn = a.S.node_cnt[sh];
-    S.cl0 = a.S.cl_off[sh]; S.ncl = a.S.cl_cnt[sh];
-    double3 FA = d3(0., 0., 0.), TA = d3(0., 0., 0.);
-    for (int j = 0; j < npp; ++j)
-      do_pair<KIND_PP>(a, A, j, a.pp.id[(size_t)A * a.pp.cap + j], S, s_cl[warp], s_mask[warp], s_old[warp], FA, TA);
-    for (int j = 0; j < nw; ++j)
-      do_pair<KIND_WALL>(a, A, j, a.pw.id[(size_t)A * a.pw.cap + j], S, s_cl[warp], s_mask[warp], s_old[warp], FA, TA);
-    if (ngc > 0) S.x = owner_pos<KIND_GHOST>(a, A);
-    for (int j = 0; j < ngc; ++j)
-      do_pair<KIND_GHOST>(a, A, j, a.pgh.id[(size_t)A * a.pgh.cap + j], S, s_cl[warp], s_mask[warp], s_old[warp], FA, TA);
-    FA = warp_sum3(FA);
-    TA = warp_sum3(TA);
-    if (lane == 0) {
-      atomic_add3(a.P.force, A, FA);
-      atomic_add3(a.P.torque, A, TA);
-    }
-  }
-  if ((KINDS & 4) && lane == 0 && ng_max > 0) atomicMax(&a.status->need_ghost, ng_max);
-}
-
 // ---------------------------------------------------------------------------
-// Precision form: certified FP32 screening on 16-bit SDF templates.
+// Certified FP32 screening.
 //
 // Almost every node the narrowphase visits is rejected (outside the partner's
-// bounding sphere or cell window, or phi > 0). The precision form makes those
-// rejections in FP32 against SDF templates stored as phi / h in FP16 or BF16,
-// and rejects a node only when error bounds prove that the FP64 test
-// (node_hits) rejects it too. Every node it cannot reject is decided by
-// node_hits itself, and every contact is evaluated by the FP64 code of
-// finish_pair. Pair lists, contact segments and forces are therefore those of
-// the FP64 form; the 16-bit store and FP32 arithmetic only make the rejections
-// cheaper.
+// bounding sphere or cell window, or phi > 0). Those rejections are made in FP32,
+// in the precision forms against SDF templates stored as phi / h in FP16 or BF16, in
+// the FP64 form against the FP64 templates, and a node is rejected only when error
+// bounds prove that the FP64 test (k_contacts_f) rejects it too. Every node the screen
+// cannot reject is decided by that test, and every contact is evaluated in FP64. Pair
+// lists, contact segments and forces of all forms are therefore the same; the 16-bit
+// store only makes the rejections cheaper. (The FP64 form ran its cluster cull and node test
+// in FP64, one warp per owner at 255 registers, with no cull by phi: a step of a bed of 20,000
+// bodies took 961 us that way and takes 392 us.)
 //
 // Per pair, the owner's node offsets n (template units) map to the partner's
 // frame by l = M n + dB, M = R_B^T R_A scale_A, dB = R_B^T (xA - xB), and to its
@@ -1137,9 +960,10 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 2) k_narrowphase(StepArgs a) {
 // node distance x scale_A, and g adds u |g|_1 + invh u |origin|_1; EPS_F = 1.6e-5
 // (~270u) bounds all of it with a wide margin: el = EPS_F (N1 + 2 |d|_1) in
 // length, eg = invh (el + EPS_F |origin|_1) + EPS_F (sizes summed) in grid units
-// per axis. The 16-bit corners c differ from the FP64 values v by at most
+// per axis. The corners c differ from the FP64 values v by at most
 // Q |v| (Q = 2^-11 for FP16, 2^-8 for BF16, round to nearest, plus the FP32
-// rounding of phi / h and of the interpolation); an error eg in the grid point
+// rounding of phi / h and of the interpolation; these alone, below 16u, from the FP64
+// templates); an error eg in the grid point
 // moves the piecewise-trilinear phi / h by at most 3 L eg, L = the largest
 // difference of neighbouring grid values of the partner's template in spacings;
 // and every corner of the cell lies within 3 L of the interpolated value. So
@@ -1153,10 +977,13 @@ LD float3 tof(double3 v) { return f3((float)v.x, (float)v.y, (float)v.z); }
 LD double3 tod(float3 v) { return d3(v.x, v.y, v.z); }
 
 static constexpr float EPS_F = 1.6e-5f;
+static constexpr float PHI_BAND = (float)LIP_BAND;
 
 // relative bound of the 16-bit store and FP32 interpolation error (with margin)
 template <int SDFK>
-LD constexpr float quant16() { return SDFK == PREC_FP32_BF16 ? 3.95e-3f + 1e-6f : 4.95e-4f + 1e-6f; }
+LD constexpr float quant16() {
+  return SDFK == PREC_FP32_BF16 ? 3.95e-3f + 1e-6f : (SDFK == PREC_FP32_FP16 ? 4.95e-4f + 1e-6f : 2e-6f);
+}
 
 // Constants of one screened pair.
 struct PairF {
@@ -1172,8 +999,11 @@ struct PairF {
   float T;           // rejection threshold of phi / h
   float Tq;          // 1 / (1 - Q')
   float gmax;        // gradient-norm bound of phi / h per grid unit
+  float gband;       // the same over the cells where phi / h takes values in [0, PHI_BAND]
   int sy, sz;        // cell strides
   const uint4* cells;
+  const double* sdf; // FP64 form: grid values, their factor ih to phi / h (strides sy, sz of the grid)
+  float ih;
   int key;           // walls and images: the partner's cell key
   float RA[9];       // walls and images: R_A scale_A (world offsets of the nodes)
   float n1w;         // walls and images: error bound of the world node offset
@@ -1183,34 +1013,21 @@ struct PairF {
   int pshape;
 };
 
-// Rotation matrix columns of q (the images of the unit axes under rotate()).
-LD void rot_cols(Quat q, double3 c[3]) {
-  c[0] = rotate(q, d3(1., 0., 0.));
-  c[1] = rotate(q, d3(0., 1., 0.));
-  c[2] = rotate(q, d3(0., 0., 1.));
-}
-
 template <int KIND, int SDFK>
-LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape, int pidx) {
+LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape) {
   PairF F;
-  // rows of R_A (FP32, from the step's matrices) and of R_B (particles likewise;
-  // walls from their quaternion)
+  // R_A and R_B (row-major), each column rotated by one lane in FP64 and rounded
   float ra[9], rb[9];
   {
-    const float4 r0 = __ldg(a.P.rotm + 3 * A), r1 = __ldg(a.P.rotm + 3 * A + 1), r2 = __ldg(a.P.rotm + 3 * A + 2);
-    ra[0] = r0.x; ra[1] = r0.y; ra[2] = r0.z; ra[3] = r1.x; ra[4] = r1.y; ra[5] = r1.z;
-    ra[6] = r2.x; ra[7] = r2.y; ra[8] = r2.z;
-  }
-  if (KIND == KIND_WALL || (KIND == KIND_GHOST && a.G.sector)) {
-    double3 cb[3];
-    rot_cols(P.q, cb);
+    const int lane = threadIdx.x & 31, ax = lane % 3;
+    const double3 u = d3(ax == 0 ? 1. : 0., ax == 1 ? 1. : 0., ax == 2 ? 1. : 0.);
+    const double3 c = rotate(lane < 3 ? a.P.quat[A] : P.q, u);
+    const float cx = (float)c.x, cy = (float)c.y, cz = (float)c.z;
+#pragma unroll
     for (int j = 0; j < 3; ++j) {
-      rb[j] = (float)cb[j].x; rb[3 + j] = (float)cb[j].y; rb[6 + j] = (float)cb[j].z;
+      ra[j] = __shfl_sync(FULL, cx, j); ra[3 + j] = __shfl_sync(FULL, cy, j); ra[6 + j] = __shfl_sync(FULL, cz, j);
+      rb[j] = __shfl_sync(FULL, cx, 3 + j); rb[3 + j] = __shfl_sync(FULL, cy, 3 + j); rb[6 + j] = __shfl_sync(FULL, cz, 3 + j);
     }
-  } else {
-    const float4 r0 = __ldg(a.P.rotm + 3 * pidx), r1 = __ldg(a.P.rotm + 3 * pidx + 1), r2 = __ldg(a.P.rotm + 3 * pidx + 2);
-    rb[0] = r0.x; rb[1] = r0.y; rb[2] = r0.z; rb[3] = r1.x; rb[4] = r1.y; rb[5] = r1.z;
-    rb[6] = r2.x; rb[7] = r2.y; rb[8] = r2.z;
   }
   const int shA = a.P.shape[A];
   const float scA = (float)a.P.scale[A];
@@ -1235,15 +1052,23 @@ LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape, int
   const float eg = F.invh * (el + EPS_F * (fabsf(F.cg.x) + fabsf(F.cg.y) + fabsf(F.cg.z)) / F.invh) +
                    EPS_F * (float)(P.gs.x + P.gs.y + P.gs.z);
   F.eg = eg;
-  const float L = a.S.lip[2 * pshape];
+  const float L = a.S.lip[3 * pshape];
   const float Q = quant16<SDFK>();
   const float Qp = Q / (1.0f - Q);
   F.Tq = 1.0f / (1.0f - Qp);
   F.T = (3.0f * L * Qp + 3.0f * L * eg + 1e-7f) * F.Tq * (1.0f + 1e-5f);
-  F.gmax = a.S.lip[2 * pshape + 1];
-  F.sy = P.gs.x - 1;
-  F.sz = (P.gs.x - 1) * (P.gs.y - 1);
-  F.cells = a.S.cell16 + a.S.cell_off[pshape];
+  F.gmax = a.S.lip[3 * pshape + 1];
+  F.gband = a.S.lip[3 * pshape + 2];
+  if (SDFK == PREC_FP64) {
+    F.sy = P.gs.x;
+    F.sz = P.gs.x * P.gs.y;
+    F.sdf = P.sdf;
+    F.ih = (float)(P.invh * P.sc);  // 1 / template spacing
+  } else {
+    F.sy = P.gs.x - 1;
+    F.sz = (P.gs.x - 1) * (P.gs.y - 1);
+    F.cells = a.S.cell16 + a.S.cell_off[pshape];
+  }
   F.key = P.key;
   if (KIND != KIND_PP) {
     for (int k = 0; k < 9; ++k) F.RA[k] = ra[k] * scA;
@@ -1296,6 +1121,18 @@ LD float phi16_at(const uint4* cells, int sy, int sz, float gx, float gy, float 
 }
 template <int SDFK>
 LD float phi16(const PairF& F, float gx, float gy, float gz) {
+  if (SDFK == PREC_FP64) {
+    const int i0 = __float2int_rd(gx), j0 = __float2int_rd(gy), k0 = __float2int_rd(gz);
+    const double* b = F.sdf + (k0 * F.sz + j0 * F.sy + i0);
+    const float fx = gx - floorf(gx), fy = gy - floorf(gy), fz = gz - floorf(gz);
+    float c[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) c[k] = (float)__ldg(b + (k & 1) + (k & 2 ? F.sy : 0) + (k & 4 ? F.sz : 0));
+    const float x0 = fmaf(fx, c[1] - c[0], c[0]), x1 = fmaf(fx, c[3] - c[2], c[2]);
+    const float x2 = fmaf(fx, c[5] - c[4], c[4]), x3 = fmaf(fx, c[7] - c[6], c[6]);
+    const float y0 = fmaf(fy, x1 - x0, x0), y1 = fmaf(fy, x3 - x2, x2);
+    return fmaf(fz, y1 - y0, y0) * F.ih;
+  }
   return phi16_at<SDFK>(F.cells, F.sy, F.sz, gx, gy, gz);
 }
 
@@ -1345,7 +1182,11 @@ LD bool node_may_hit_f(const StepArgs& a, double3 xA, const PairF& F, float4 nd,
 //    sqrt(3) m (projection onto a convex set does not expand distances), the
 //    segment p-q lies in the box, and along it phi / h changes by at most gmax
 //    per grid unit, so phi(q) - gmax (rad + sqrt(3) m) > 0 proves phi > 0 at
-//    every node of the cluster.
+//    every node of the cluster. On the way down to phi = 0 the last stretch from
+//    min(phi(q), PHI_BAND) lies in cells where phi / h takes values in [0, PHI_BAND], so
+//    when the distance times their bound gband is below PHI_BAND, gband serves in place of
+//    gmax, which the medial surface sets (1.73 against 1.15 for a rounded box, 1.14 against
+//    1.07 for an ellipsoid).
 //  With up != nullptr (learned form), *up receives an estimate of the largest phi / h
 //  over the cluster's nodes (phi at q plus gmax times the reach; +inf when phi at q is
 //  not looked up): where it is below the network's rejection threshold the network would
@@ -1370,7 +1211,9 @@ LD bool cluster_may_hit_f(const PairF& F, float4 cn, float scA, float* up = null
   if (F.ux < 4.f * m || F.uy < 4.f * m || F.uz < 4.f * m) return true;
   const float qx = fminf(fmaxf(gx, m), F.ux - m), qy = fminf(fmaxf(gy, m), F.uy - m),
               qz = fminf(fmaxf(gz, m), F.uz - m);
-  const float reach = (F.gmax * (radh + 2.8f * m) + 1e-6f) * F.Tq * (1.0f + 1e-6f);
+  const float dist = radh + 2.8f * m;
+  const float g = F.gband * dist * (1.0f + 1e-6f) < PHI_BAND ? F.gband : F.gmax;
+  const float reach = (g * dist + 1e-6f) * F.Tq * (1.0f + 1e-6f);
   const float ph = phi16<SDFK>(F, qx, qy, qz);
   if (up) *up = ph + reach;
   return !(ph > F.T + reach);
@@ -1386,7 +1229,7 @@ LD int partner_shape(const StepArgs& a, int pid) {
 // surviving clusters. The nodes the screen cannot reject are written, in node
 // order, to the precision-form node buffer and the pair is queued for
 // k_contacts_f; a pair without such nodes gets its empty contact segment here.
-template <int KIND, int SDFK, bool LRN>
+template <int KIND, int SDFK, bool LRN, bool STATS>
 LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* s_cl, unsigned short* s_sub,
                       unsigned* s_mask, unsigned (&cnt)[8], unsigned& queued) {
   const int lane = threadIdx.x & 31;
@@ -1398,7 +1241,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
   PairF F;
   {
     const Partner P = load_partner<KIND>(a, pid);
-    F = make_pair_f<KIND, SDFK>(a, A, P, partner_shape<KIND>(a, pid), KIND == KIND_GHOST ? (pid >> 3) : pid);
+    F = make_pair_f<KIND, SDFK>(a, A, P, partner_shape<KIND>(a, pid));
   }
   int nsurv = 0;
   for (int c0 = 0; c0 < ncl; c0 += 32) {
@@ -1431,7 +1274,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
     nsub += __popc(m);
   }
   const int nch = (nsub + 3) >> 2;
-  cnt[0] += 1; cnt[1] += ncl; cnt[2] += nsurv; cnt[7] += nsub;
+  if (STATS) { cnt[0] += 1; cnt[1] += ncl; cnt[2] += nsurv; cnt[7] += nsub; }
   __syncwarp();
   // this lane's node in chunk k (nn when none)
   auto node_of = [&](int k) {
@@ -1455,7 +1298,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
       const int ni = node_of(k);
       const int j = 4 * k + (lane >> 3);
       const bool marked = j < nsub && (s_sub[j] & 0x8000);
-      cnt[4] += __popc(__ballot_sync(FULL, ni < nn));
+      if (STATS) cnt[4] += __popc(__ballot_sync(FULL, ni < nn));
       bool need = false, may = false, looked = false;
       if (ni < nn) {
         const float4 nd = __ldg(a.S.node_pos_f + n0 + ni);
@@ -1472,7 +1315,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
           need = adm && !(lo < -F.eg || hi >= F.eg);
         }
       }
-      cnt[3] += __popc(__ballot_sync(FULL, looked));
+      if (STATS) cnt[3] += __popc(__ballot_sync(FULL, looked));
       const unsigned mn = __ballot_sync(FULL, need), md = __ballot_sync(FULL, may);
       if (lane == 0) {
         s_mask[k] = mn;
@@ -1554,17 +1397,16 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
   } else {
     for (int k = 0; k < nch; ++k) {
       const int ni = node_of(k);
-      cnt[4] += __popc(__ballot_sync(FULL, ni < nn));
+      if (STATS) cnt[4] += __popc(__ballot_sync(FULL, ni < nn));
       bool may = false, looked = false;
       if (ni < nn) may = node_may_hit_f<KIND, SDFK>(a, xA, F, __ldg(a.S.node_pos_f + n0 + ni), looked);
-      cnt[3] += __popc(__ballot_sync(FULL, looked));
+      if (STATS) cnt[3] += __popc(__ballot_sync(FULL, looked));
       const unsigned m = __ballot_sync(FULL, may);
       if (lane == 0) s_mask[k] = m;
       total += __popc(m);
     }
   }
-  cnt[5] += total;
-  queued += total;
+  if (STATS) { cnt[5] += total; queued += total; }
   __syncwarp();
   const SlotView& cur = slots_of<KIND>(a, false);
   const size_t sidx = (size_t)A * cur.cap + slot;
@@ -1587,9 +1429,9 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
       // the pair index is reserved: mark its entry empty so that the contact pass skips it
       // (the node queue is full; the batch re-runs with grown capacities)
       if (pi < a.mb.pcap) a.mb.pair[(size_t)li * a.mb.pcap + pi] = make_int4(-1, 0, 0, 0);
-      atomicOr(&a.status->flags, OVF_CONTACT);
+      atomicOr(&a.status->flags, OVF_QUEUE);
       const long long need = start + total > 2LL * (pi + 1) ? start + total : 2LL * (pi + 1);
-      atomicMax(&a.status->need_contact, (int)(need < 0x7fffffff ? need : 0x7fffffff));
+      atomicMax(&a.status->need_queue, (int)(need < 0x7fffffff ? need : 0x7fffffff));
     }
     cur.seg_start[sidx] = 0;
     cur.seg_cnt[sidx] = 0;
@@ -1609,37 +1451,37 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
 // particle, wall, image order.
 // Particle-only screens fit 64 registers (8 blocks per SM); walls and images
 // need the window test's FP64 registers.
-template <int KINDS, int SDFK, bool LRN>
+template <int KINDS, int SDFK, bool LRN, bool STATS>
 __global__ void __launch_bounds__(NP_WARPS * 32, KINDS == 1 ? 8 : 5) k_screen_f(StepArgs a, int li, int kinds) {
   __shared__ int s_cl[NP_WARPS][MAXCL];
   __shared__ unsigned short s_sub[NP_WARPS][4 * MAXCL];
   __shared__ unsigned s_mask[NP_WARPS][MAXCL];
   const int warp = threadIdx.x >> 5;
-  const int n0 = (KINDS & 1) ? min(a.pl.ctr[0], a.P.n * a.pp.cap) : 0;
-  const int n1 = (kinds & KINDS & 2) && a.pw.cap > 0 ? min(a.pl.ctr[1], a.P.n * a.pw.cap) : 0;
-  const int n2 = (kinds & KINDS & 4) ? min(a.pl.ctr[2], a.P.n * a.pgh.cap) : 0;
+  const int n0 = (KINDS & 1) ? a.pl.ctr[0] : 0;
+  const int n1 = (kinds & KINDS & 2) && a.pw.cap > 0 ? a.pl.ctr[1] : 0;
+  const int n2 = (kinds & KINDS & 4) ? a.pl.ctr[2] : 0;
   const int tot = n0 + n1 + n2;
   unsigned cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // warp-uniform screen counters
   unsigned queued[3] = {0, 0, 0};              // nodes queued by partner kind
   for (int e = blockIdx.x * NP_WARPS + warp; e < tot; e += gridDim.x * NP_WARPS) {
     if ((KINDS & 1) && e < n0) {
-      const int idx = __ldg(a.pl.list[0] + e);
+      const unsigned idx = __ldg(a.pl.list[0] + e);
       const int A = idx / a.pp.cap;
-      screen_pair_f<KIND_PP, SDFK, LRN>(a, A, idx - A * a.pp.cap, __ldg(a.pp.id + idx), li, s_cl[warp], s_sub[warp],
+      screen_pair_f<KIND_PP, SDFK, LRN, STATS>(a, A, idx - A * a.pp.cap, __ldg(a.pp.id + idx), li, s_cl[warp], s_sub[warp],
                                         s_mask[warp], cnt, queued[0]);
     } else if ((KINDS & 2) && e < n0 + n1) {
-      const int idx = a.pl.list[1][e - n0];
+      const unsigned idx = a.pl.list[1][e - n0];
       const int A = idx / a.pw.cap;
-      screen_pair_f<KIND_WALL, SDFK, LRN>(a, A, idx - A * a.pw.cap, a.pw.id[idx], li, s_cl[warp], s_sub[warp],
+      screen_pair_f<KIND_WALL, SDFK, LRN, STATS>(a, A, idx - A * a.pw.cap, a.pw.id[idx], li, s_cl[warp], s_sub[warp],
                                           s_mask[warp], cnt, queued[1]);
     } else if (KINDS & 4) {
-      const int idx = __ldg(a.pl.list[2] + e - n0 - n1);
+      const unsigned idx = __ldg(a.pl.list[2] + e - n0 - n1);
       const int A = idx / a.pgh.cap;
-      screen_pair_f<KIND_GHOST, SDFK, LRN>(a, A, idx - A * a.pgh.cap, __ldg(a.pgh.id + idx), li, s_cl[warp], s_sub[warp],
+      screen_pair_f<KIND_GHOST, SDFK, LRN, STATS>(a, A, idx - A * a.pgh.cap, __ldg(a.pgh.id + idx), li, s_cl[warp], s_sub[warp],
                                            s_mask[warp], cnt, queued[2]);
     }
   }
-  if (a.screen_stats && (threadIdx.x & 31) == 0) {
+  if (STATS && (threadIdx.x & 31) == 0) {
     for (int k = 0; k < 8; ++k)
       if (cnt[k]) atomicAdd(&a.screen_stats[k], (unsigned long long)cnt[k]);
     // grid screen: nodes queued for the FP64 test by partner kind
@@ -1660,7 +1502,7 @@ LD Partner load_partner_of(const StepArgs& a, int kind, int pid) {
 // A warp takes up to 32 pairs and runs their nodes, then their contacts, one lane each, whichever
 // pair they are of. A pair of a bed has 1.5 queued nodes and 0.7 contacts, so that a warp per
 // pair left 30 of its lanes idle through a chain of dependent loads, eight warps an SM (100k
-// bodies with 336k contacts: CON_OLD us that way, CON_NEW us now). With few pairs a warp takes
+// bodies with 336k contacts: 2325 us that way, 150 us now). With few pairs a warp takes
 // one, and the lanes are its nodes as before.
 // Between the two runs a pair's hits stand at the front of its part of the node queue, in node
 // order; one atomic per warp reserves the segments of its pairs.
@@ -1671,6 +1513,8 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
   int4* pair = s_pair[warp];
   int4* seg = s_seg[warp];
   const int np = min(a.mb.ctr[1 + li], a.mb.pcap);
+  if (blockIdx.x == 0 && threadIdx.x == 0)  // this step's demand, for the capacity planning
+    atomicMax(&a.status->need_queue, max(a.mb.ctr[0], min(np, 0x3fffffff) * 2));
   const int W = gridDim.x * NP_WARPS;
   const int per = min(32, (np + W - 1) / W);
   for (int p0 = (blockIdx.x * NP_WARPS + warp) * per; p0 < np; p0 += W * per) {
@@ -1931,9 +1775,9 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_net_compact(StepArgs a, int l
         a.mb.pair[(size_t)li * a.mb.pcap + pi] = make_int4(e.x, e.y, start, total);
       } else {
         if (pi < a.mb.pcap) a.mb.pair[(size_t)li * a.mb.pcap + pi] = make_int4(-1, 0, 0, 0);
-        atomicOr(&a.status->flags, OVF_CONTACT);
+        atomicOr(&a.status->flags, OVF_QUEUE);
         const long long need = start + total > 2LL * (pi + 1) ? start + total : 2LL * (pi + 1);
-        atomicMax(&a.status->need_contact, (int)(need < 0x7fffffff ? need : 0x7fffffff));
+        atomicMax(&a.status->need_queue, (int)(need < 0x7fffffff ? need : 0x7fffffff));
       }
     }
     start = __shfl_sync(FULL, start, 0);
@@ -1949,9 +1793,13 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_net_compact(StepArgs a, int l
   if (a.screen_stats && lane == 0 && queued) atomicAdd(&a.screen_stats[5], (unsigned long long)queued);
 }
 
+bool one_screen(const StepArgs& a) { return a.P.n <= num_sms() * 20; }
+
 template <int KINDS, int SDFK, bool LRN>
 void launch_screen_k(const StepArgs& a, int li, int kinds, dim3 g, dim3 b, cudaStream_t s) {
-  k_screen_f<KINDS, SDFK, LRN><<<g, b, 0, s>>>(a, li, kinds);
+  // the counters' ballots are compiled in only where they are asked for
+  if (a.screen_stats) k_screen_f<KINDS, SDFK, LRN, true><<<g, b, 0, s>>>(a, li, kinds);
+  else k_screen_f<KINDS, SDFK, LRN, false><<<g, b, 0, s>>>(a, li, kinds);
 }
 
 // Learned form: the network pass and the compaction after the screen of launch li.
@@ -1978,42 +1826,38 @@ void launch_net_compact(const StepArgs& a, int li, cudaStream_t s) {
   k_net_compact<<<num_sms() * 16, NP_WARPS * 32, 0, s>>>(a, li);
 }
 
-template <bool LRN>
 // Particle pairs, and wall and image pairs, in two launches: the particle-only screen fits 64
 // registers (8 blocks per SM); the others (few) take the window test's FP64 registers.
+// A system of no more particles than the warps that are resident at 96 registers takes one
+// launch: there a launch counts more than occupancy (2,000 ellipsoids on a floor: 54.3 us per step
+// with two, 46.1 us with one).
+template <int SDFK, bool LRN>
 void launch_screen(const StepArgs& a, int kinds, int li, dim3 g, dim3 b, cudaStream_t s) {
-  if (a.precision == PREC_FP32_FP16) {
-    if (kinds & 1) launch_screen_k<1, PREC_FP32_FP16, LRN>(a, li, kinds, g, b, s);
-    if (kinds & 6) launch_screen_k<6, PREC_FP32_FP16, LRN>(a, li, kinds, g, b, s);
-  } else {
-    if (kinds & 1) launch_screen_k<1, PREC_FP32_BF16, LRN>(a, li, kinds, g, b, s);
-    if (kinds & 6) launch_screen_k<6, PREC_FP32_BF16, LRN>(a, li, kinds, g, b, s);
-  }
-}
-
-void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s) {
-  if (a.P.n <= 0) return;
-  int want = (a.P.n + NP_WARPS - 1) / NP_WARPS;
-  int cap = num_sms() * 16;
-  int blocks = want < cap ? want : cap;
-  const dim3 g(blocks), b(NP_WARPS * 32);
-  if (a.precision == PREC_FP64) {
-    if (kinds == 3) k_narrowphase<3><<<g, b, 0, s>>>(a);
-    else if (kinds == 5) k_narrowphase<5><<<g, b, 0, s>>>(a);
-    else if (kinds == 1) k_narrowphase<1><<<g, b, 0, s>>>(a);
-    else if (kinds == 4) k_narrowphase<4><<<g, b, 0, s>>>(a);
-    else k_narrowphase<7><<<g, b, 0, s>>>(a);
+  if ((kinds & 1) && (kinds & 6) && one_screen(a)) {
+    launch_screen_k<7, SDFK, LRN>(a, li, kinds, g, b, s);
     return;
   }
-  // precision form: the screen over the flat pair lists (launch_contact_pass
-  // follows it); the grid is sized for the device, the list length is on it
+  if (kinds & 1) launch_screen_k<1, SDFK, LRN>(a, li, kinds, g, b, s);
+  if (kinds & 6) launch_screen_k<6, SDFK, LRN>(a, li, kinds, g, b, s);
+}
+
+// The screen over the flat pair lists (launch_contact_pass, in the learned form after
+// launch_net_screen and _compact, follows it); the grid is sized for the device, the list length
+// is on it.
+void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s) {
+  if (a.P.n <= 0) return;
+  // walls and images come on top of a small system's particle pairs
+  const dim3 g(std::min((2 * a.P.n + NP_WARPS - 1) / NP_WARPS, num_sms() * 16)), b(NP_WARPS * 32);
   const int li = kinds == 4 && !a.gl.list ? 1 : 0;
-  if (a.mlp_inf) launch_screen<true>(a, kinds, li, g, b, s);  // launch_net_screen and _compact follow
-  else launch_screen<false>(a, kinds, li, g, b, s);
+  if (a.precision == PREC_FP64) launch_screen<PREC_FP64, false>(a, kinds, li, g, b, s);
+  else if (a.precision == PREC_FP32_FP16 && a.mlp_inf) launch_screen<PREC_FP32_FP16, true>(a, kinds, li, g, b, s);
+  else if (a.precision == PREC_FP32_FP16) launch_screen<PREC_FP32_FP16, false>(a, kinds, li, g, b, s);
+  else if (a.mlp_inf) launch_screen<PREC_FP32_BF16, true>(a, kinds, li, g, b, s);
+  else launch_screen<PREC_FP32_BF16, false>(a, kinds, li, g, b, s);
 }
 
 void launch_contact_pass(const StepArgs& a, int li, cudaStream_t s) {
-  if (a.P.n <= 0 || a.precision == PREC_FP64) return;
+  if (a.P.n <= 0) return;
   k_contacts_f<<<num_sms() * 3, NP_WARPS * 32, 0, s>>>(a, li);
 }
 
@@ -2064,12 +1908,6 @@ LD void sector_wrap_images(const StepArgs& a, int i, double3& p) {
   if (turned) {
     a.P.vel[i] = v;
     a.P.quat[i] = q;
-    if (a.P.rotm) {
-      const double3 c0 = rotate(q, d3(1., 0., 0.)), c1 = rotate(q, d3(0., 1., 0.)), c2 = rotate(q, d3(0., 0., 1.));
-      a.P.rotm[3 * i] = make_float4((float)c0.x, (float)c1.x, (float)c2.x, 0.f);
-      a.P.rotm[3 * i + 1] = make_float4((float)c0.y, (float)c1.y, (float)c2.y, 0.f);
-      a.P.rotm[3 * i + 2] = make_float4((float)c0.z, (float)c1.z, (float)c2.z, 0.f);
-    }
   }
   double3 gp[3] = {p, p, p}, gv[3] = {v, v, v};
   Quat gq[3] = {q, q, q};
@@ -2212,7 +2050,7 @@ __global__ void k_ghost_candidates(StepArgs a, const int* __restrict__ g2_idx, c
               }
             }
             need = max(need, slot + 1);
-            if (a.pl.ctr) {  // precision form: flat pair list
+            {  // flat pair list
               const bool ok = slot >= 0 && slot < a.pgh.cap;
               const unsigned m = __ballot_sync(FULL, ok);
               int base = 0;
@@ -2286,13 +2124,13 @@ __global__ void __launch_bounds__(128) k_image_candidates(StepArgs a) {
       }
     }
     need = max(need, slot + 1);
-    if (a.pl.ctr) {  // precision form: flat pair list
+    {  // flat pair list
       const bool ok = slot >= 0 && slot < a.pgh.cap;
       const unsigned mk = __ballot_sync(FULL, ok);
       int at = 0;
       if (lane == 0 && mk) at = atomicAdd(&a.pl.ctr[2], __popc(mk));
       at = __shfl_sync(FULL, at, 0);
-      if (ok) a.pl.list[2][at + __popc(mk & lanemask_lt())] = A * a.pgh.cap + slot;
+      if (ok) a.pl.list[2][at + __popc(mk & lanemask_lt())] = (int)((unsigned)A * a.pgh.cap + slot);
     }
   }
   need = __reduce_max_sync(FULL, need);
