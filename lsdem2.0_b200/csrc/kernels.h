@@ -235,6 +235,7 @@ struct StepArgs {
   double dt;
   double3 gravity;
   int flags;        // FIX_* bits
+  int kick;         // the step before it left its second half kick to this one
   int precision;    // PREC_*
   double rmax;      // largest particle bounding radius
   MaybeView mb;
@@ -251,8 +252,9 @@ struct StepArgs {
   int nshapes;
   // Neighbour lists (exact, optional): *reuse is set non-zero when a point of a particle
   // may have moved more than `move` since the last list build; the cell sort and
-  // the list rebuild run only then. The step's kick clears it.
+  // the list rebuild run only then. Two flags by history parity: a step clears the next one's.
   int* reuse;
+  int* reuse_next;
   float move;             // 0.4 skin
   float skin;             // neighbour-list margin beyond the candidate reach (length)
   double3* xb;            // particle order: position at the last list build
@@ -311,6 +313,19 @@ void mlp_infer(const MlpInfer* inf, const MlpNorm& nm, const double3* pts, int n
 
 void launch_integrate_first(const StepArgs& a, cudaStream_t s);
 void launch_candidates(const StepArgs& a, cudaStream_t s);
+// Copies taken aside at the start of a batch.
+struct CopySeg {
+  const unsigned* src;
+  unsigned* dst;
+  long long words;
+};
+struct BackupArgs {
+  CopySeg seg[12];
+  int nseg;
+  SlotView from[3], to[3];  // cnt nullptr: none
+  int n;
+};
+void launch_backup(const BackupArgs& b, cudaStream_t s);
 void launch_narrowphase(const StepArgs& a, int kinds, cudaStream_t s);
 bool one_screen(const StepArgs& a);  // all partner kinds of a step in one screen launch
 // precision form: FP64 contact pass over the pairs queued by the screen of

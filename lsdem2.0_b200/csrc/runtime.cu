@@ -332,7 +332,7 @@ struct lsdem_solver {
   // profiling or contact recording; `graph_gen` changes whenever a step's arguments or
   // launch configuration may change (initialize, capacity growth, setters)
   struct StepGraph { cudaGraphExec_t exec = nullptr; uint64_t key = 0; long long launches = 0; };
-  StepGraph sgraph[2];
+  StepGraph sgraph[2][2];  // [history parity][with the last step's kick]
   long long graph_gen = 0;
   bool graphs = true;
   cudaStream_t gstream = nullptr;  // blocking stream for replay when the solver runs on the legacy stream
@@ -1022,7 +1022,8 @@ void initialize(lsdem_solver* s) {
     // particle moved 0.4 of it (pairs approach by at most twice that)
     const double sr = 0.1 * s->rmax_p;
     s->skin = (float)sr;
-    CK(s->reuse.alloc(1));
+    CK(s->reuse.alloc(2));
+    CK(s->reuse.zero(st));
     CK(s->xb.alloc(std::max(n, 1)));
     CK(s->qb.alloc(std::max(n, 1)));
     CK(s->rec.alloc(2 * (size_t)std::max(n, 1)));
@@ -1191,7 +1192,8 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.precision = s->precision;
   a.rmax = s->rmax_p;
   const bool reuse = s->reuse_on && s->reuse.p;
-  a.reuse = reuse ? s->reuse.p : nullptr;
+  a.reuse = reuse ? s->reuse.p + s->hp : nullptr;
+  a.reuse_next = reuse ? s->reuse.p + (1 - s->hp) : nullptr;
   a.move = 0.4f * s->skin;
   a.skin = s->skin;
   a.xb = s->xb.p;
@@ -1277,9 +1279,10 @@ void resolve_profile(lsdem_solver* s, bool keep) {
 // One time step in the reference order (LSSolver.h:1000-1011, 1104-1128).
 // The launches of one step up to the external-force hook: integration, cell sort,
 // candidates, narrowphase and contact forces, periodic images, bonds.
-void step_pre(lsdem_solver* s, double dt, bool record) {
+void step_pre(lsdem_solver* s, double dt, bool record, bool kick) {
   cudaStream_t st = s->stream;
   StepArgs a = make_args(s, dt);
+  a.kick = kick ? 1 : 0;
   if (record) {
     ContactsDev& c = s->con[1 - s->hp];
     ensure_geom(s, c);
@@ -1415,64 +1418,76 @@ void step_pre(lsdem_solver* s, double dt, bool record) {
   CK(cudaGetLastError());
 }
 
-// The rest of a step after the hook: the second half kick.
-void step_post(lsdem_solver* s, double dt) {
-  StepArgs a = make_args(s, dt);
-  { PhaseTimer pt(s, 7); launch_kick(a, s->stream); }
-  if (a.P.n > 0) s->launches += 1;
-  CK(cudaGetLastError());
+// The rest of a step after the hook: the second half kick, or (later) that of the next step's
+// first kernel.
+void step_post(lsdem_solver* s, double dt, bool later) {
+  if (!later) {
+    StepArgs a = make_args(s, dt);
+    { PhaseTimer pt(s, 7); launch_kick(a, s->stream); }
+    if (a.P.n > 0) s->launches += 1;
+    CK(cudaGetLastError());
+  }
   s->hp = 1 - s->hp;
 }
 
-void step_once(lsdem_solver* s, double dt, bool record, lsdem_hook hook, void* user, double t) {
-  step_pre(s, dt, record);
-  if (hook) hook(user, t);
-  step_post(s, dt);
-}
-
 // Snapshot of everything a batch may change, taken at the batch start.
-void backup_state(lsdem_solver* s);
-void backup(lsdem_solver* s) {
-  backup_state(s);
-  backup_history(s);
-}
-
-// Body state and bond flags (what one step changes besides the new contact list).
-void backup_state(lsdem_solver* s) {
-  cudaStream_t st = s->stream;
-  const size_t n = (size_t)s->P.n(), nw = (size_t)s->W.n();
-  // backup buffers grow geometrically (never per batch: a free synchronises the device)
-  auto cp = [&](auto& dst, auto& src, size_t m) {
+// Arrays of a backup in one launch; the buffers grow geometrically (never per batch: a free
+// synchronises the device).
+struct Backup {
+  lsdem_solver* s;
+  BackupArgs b{};
+  template <class T>
+  void add(DArr<T>& dst, const DArr<T>& src, size_t m) {
     if (dst.n < m) CK(dst.alloc(std::max(m + m / 2, (size_t)1024)));
-    if (m) CK(cudaMemcpyAsync(dst.p, src.p, m * sizeof(*src.p), cudaMemcpyDeviceToDevice, st));
-  };
-  cp(s->bk_pos, s->dP.pos, n); cp(s->bk_vel, s->dP.vel, n); cp(s->bk_angvel, s->dP.angvel, n);
-  cp(s->bk_quat, s->dP.quat, n); cp(s->bk_force, s->dP.force, n); cp(s->bk_torque, s->dP.torque, n);
-  cp(s->bk_wpos, s->dW.pos, nw); cp(s->bk_wquat, s->dW.quat, nw);
-  cp(s->bk_bonded, s->b_bonded, s->bonds.bonded.size());
-}
-
-// The contact history of the last step (candidate slots with their contact segments,
-// contact nodes and springs) into the backup buffers.
-void backup_history(lsdem_solver* s) {
-  cudaStream_t st = s->stream;
-  const size_t n = (size_t)s->P.n();
-  auto cp = [&](auto& dst, auto& src, size_t m) {
-    if (dst.n < m) CK(dst.alloc(std::max(m + m / 2, (size_t)1024)));
-    if (m) CK(cudaMemcpyAsync(dst.p, src.p, m * sizeof(*src.p), cudaMemcpyDeviceToDevice, st));
-  };
-  for (int k = 0; k < 3; ++k) {
-    SlotsDev& sl = s->slots[s->hp][k];
-    s->bk_cap[k] = sl.cap;
-    if (!sl.cnt.p) continue;
-    cp(s->bk_slot[k][0], sl.cnt, n);
-    cp(s->bk_slot[k][1], sl.id, n * sl.cap);
-    cp(s->bk_slot[k][2], sl.seg_start, n * sl.cap);
-    cp(s->bk_slot[k][3], sl.seg_cnt, n * sl.cap);
+    if (m) b.seg[b.nseg++] = CopySeg{(const unsigned*)src.p, (unsigned*)dst.p, (long long)(m * sizeof(T) / 4)};
   }
-  const size_t nc = (size_t)s->hist_count;
-  cp(s->bk_cnode, s->con[s->hp].node, nc);
-  cp(s->bk_cspring, s->con[s->hp].spring, nc);
+  // Body state and bond flags (what one step changes besides the new contact list).
+  void state() {
+    const size_t n = (size_t)s->P.n(), nw = (size_t)s->W.n();
+    add(s->bk_pos, s->dP.pos, n); add(s->bk_vel, s->dP.vel, n); add(s->bk_angvel, s->dP.angvel, n);
+    add(s->bk_quat, s->dP.quat, n); add(s->bk_force, s->dP.force, n); add(s->bk_torque, s->dP.torque, n);
+    add(s->bk_wpos, s->dW.pos, nw); add(s->bk_wquat, s->dW.quat, nw);
+    add(s->bk_bonded, s->b_bonded, s->bonds.bonded.size());
+  }
+  // The contact history of the last step: candidate slots with their contact segments, contact
+  // nodes and springs.
+  void history() {
+    const size_t n = (size_t)s->P.n();
+    b.n = (int)n;
+    for (int k = 0; k < 3; ++k) {
+      SlotsDev& sl = s->slots[s->hp][k];
+      s->bk_cap[k] = sl.cap;
+      if (!sl.cnt.p || n == 0) continue;
+      for (int q = 0; q < 4; ++q) {
+        const size_t m = q == 0 ? n : n * sl.cap;
+        auto& d = s->bk_slot[k][q];
+        if (d.n < m) CK(d.alloc(std::max(m + m / 2, (size_t)1024)));
+      }
+      b.from[k] = SlotView{sl.cap, sl.cnt.p, sl.id.p, sl.seg_start.p, sl.seg_cnt.p};
+      b.to[k] = SlotView{sl.cap, s->bk_slot[k][0].p, s->bk_slot[k][1].p, s->bk_slot[k][2].p, s->bk_slot[k][3].p};
+    }
+    const size_t nc = (size_t)s->hist_count;
+    add(s->bk_cnode, s->con[s->hp].node, nc);
+    add(s->bk_cspring, s->con[s->hp].spring, nc);
+  }
+  void run() { launch_backup(b, s->stream); }
+};
+
+void backup(lsdem_solver* s) {
+  Backup b{s};
+  b.state();
+  b.history();
+  b.run();
+}
+void backup_state(lsdem_solver* s) {
+  Backup b{s};
+  b.state();
+  b.run();
+}
+void backup_history(lsdem_solver* s) {
+  Backup b{s};
+  b.history();
+  b.run();
 }
 
 void restore_state(lsdem_solver* s, int hp0);
@@ -1616,14 +1631,14 @@ cudaEvent_t step_start(lsdem_solver* s) {
   return e;
 }
 
-// One step replayed from a CUDA graph: the launches of step_once captured once per
-// history parity and key (the generation of the step's arguments, dt, capacities),
+// One step replayed from a CUDA graph: the launches of step_pre captured once per
+// history parity, kick and key (the generation of the step's arguments, dt, capacities),
 // then launched as one unit, which removes the per-launch host cost and most of the
 // gaps between the step's ~30 short kernels. On the legacy default stream (which
 // cannot be captured) the graph runs on a private blocking stream: the legacy stream
 // and blocking streams are ordered with each other both ways, so the copies, events
 // and app kernels on the legacy stream keep their order around the step.
-static void step_graph_pre(lsdem_solver* s, double dt) {
+static void step_graph_pre(lsdem_solver* s, double dt, bool kick) {
   const int hp = s->hp;
   uint64_t key = 1469598103934665603ull;
   auto mix = [&](uint64_t v) { key = (key ^ v) * 1099511628211ull; };
@@ -1637,7 +1652,7 @@ static void step_graph_pre(lsdem_solver* s, double dt) {
   mix((uint64_t)s->cap_netq); mix((uint64_t)s->cap_pend); mix((uint64_t)(uintptr_t)s->net[0].row.p);
   if (!s->stream && !s->gstream) CK(cudaStreamCreate(&s->gstream));
   cudaStream_t gs = s->stream ? s->stream : s->gstream;
-  lsdem_solver::StepGraph& G = s->sgraph[hp];
+  lsdem_solver::StepGraph& G = s->sgraph[hp][kick];
   if (!G.exec || G.key != key) {
     if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
     const long long l0 = s->launches;
@@ -1646,7 +1661,7 @@ static void step_graph_pre(lsdem_solver* s, double dt) {
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(gs, cudaStreamCaptureModeRelaxed));
     try {
-      step_pre(s, dt, false);
+      step_pre(s, dt, false, kick);
     } catch (...) {
       cudaStreamEndCapture(gs, &graph);
       if (graph) cudaGraphDestroy(graph);
@@ -1668,12 +1683,6 @@ static void step_graph_pre(lsdem_solver* s, double dt) {
   s->launches += G.launches;
 }
 
-static void step_graph(lsdem_solver* s, double dt, lsdem_hook hook, void* user, double t) {
-  step_graph_pre(s, dt);
-  if (hook) hook(user, t);
-  step_post(s, dt);
-}
-
 // Steps with an external-force hook: each step's capacity status is read before its hook
 // runs (one host synchronisation per step, as the reference's per-step count reads), and a
 // step that overflowed is re-run with grown capacities first, so the hook runs exactly once
@@ -1691,11 +1700,11 @@ static int run_steps_hooked(lsdem_solver* s, double dt, long long nsteps, lsdem_
     for (int attempt = 0;; ++attempt) {
       CK(cudaMemsetAsync(s->status.p, 0, sizeof(Status), st));
       if (s->force_reuse && s->reuse.p) {  // sort and rebuild in this step
-        CK(cudaMemsetAsync(s->reuse.p, 0xff, sizeof(int), st));
+        CK(cudaMemsetAsync(s->reuse.p + s->hp, 0xff, sizeof(int), st));
         s->force_reuse = false;
       }
-      if (s->graphs && !rec && !s->profiling && s->P.n() > 0) step_graph_pre(s, dt);
-      else step_pre(s, dt, rec);
+      if (s->graphs && !rec && !s->profiling && s->P.n() > 0) step_graph_pre(s, dt, false);
+      else step_pre(s, dt, rec, false);
       // this step's contacts are in the buffer of the other parity until step_post
       CK(cudaMemcpyAsync(s->h_status, s->status.p, sizeof(Status), cudaMemcpyDeviceToHost, st));
       CK(cudaMemcpyAsync(s->h_count, s->con[1 - s->hp].count.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1713,7 +1722,7 @@ static int run_steps_hooked(lsdem_solver* s, double dt, long long nsteps, lsdem_
     }
     const long long count = *s->h_count;
     hook(user, s->time);
-    step_post(s, dt);
+    step_post(s, dt, false);
     if (ea) {
       cudaEvent_t eb = pool_event(s);
       CK(cudaEventRecord(eb, st));
@@ -1762,13 +1771,15 @@ int run_steps(lsdem_solver* s, double dt, long long nsteps, lsdem_hook hook, voi
         cudaEvent_t ea = nullptr;
         if (s->step_timing) ea = (k == 0 && attempt == 0) ? first : step_start(s);
         if (s->force_reuse && s->reuse.p) {  // sort and rebuild in this step
-          CK(cudaMemsetAsync(s->reuse.p, 0xff, sizeof(int), st));
+          CK(cudaMemsetAsync(s->reuse.p + s->hp, 0xff, sizeof(int), st));
           s->force_reuse = false;
         }
-        if (s->graphs && !rec && !s->profiling && s->P.n() > 0)
-          step_graph(s, dt, hook, user, t);
-        else
-          step_once(s, dt, rec, hook, user, t);
+        // inside a batch the second half kick rides on the next step's first kernel (the phase
+        // profile keeps it a phase of its own)
+        const bool kick = k > 0 && !s->profiling, later = k + 1 < B && !s->profiling;
+        if (s->graphs && !rec && !s->profiling && s->P.n() > 0) step_graph_pre(s, dt, kick);
+        else step_pre(s, dt, rec, kick);
+        step_post(s, dt, later);
         if (ea) {
           cudaEvent_t eb = pool_event(s);
           CK(cudaEventRecord(eb, st));
@@ -1860,8 +1871,9 @@ void lsdem_destroy(lsdem_solver* s) {
   if (!s) return;
   if (s->ready) cudaStreamSynchronize(s->stream);
   if (s->vtu) vtu_free(s->vtu);
-  for (auto& g : s->sgraph)
-    if (g.exec) cudaGraphExecDestroy(g.exec);
+  for (auto& h : s->sgraph)
+    for (auto& g : h)
+      if (g.exec) cudaGraphExecDestroy(g.exec);
   if (s->gstream) cudaStreamDestroy(s->gstream);
   if (s->st2) cudaStreamDestroy(s->st2);
   if (s->ev_fork) cudaEventDestroy(s->ev_fork);
