@@ -1040,30 +1040,52 @@ struct PairF {
   const uint4* cells;
   const double* sdf; // FP64 form: grid values, their factor ih to phi / h (strides sy, sz of the grid)
   float ih;
-  int key;           // walls and images: the partner's cell key
-  float RA[9];       // walls and images: R_A scale_A (world offsets of the nodes)
-  float n1w;         // walls and images: error bound of the world node offset
-  // learned SDF: u = l * ms - mc (network input), phi / h = y * mtoh, threshold Tn
+  // the owner
+  int A, slot, n0, nn, cl0, ncl;  // particle, slot; first node, nodes, first cluster, clusters
+  float scA;
+};
+// Walls and images: the partner's cell key, R_A scale_A (world offsets of the nodes), their error
+// bound, the owner's position.
+template <bool WIN>
+struct PairWin {};
+template <>
+struct PairWin<true> {
+  int key;
+  float RA[9];
+  float n1w;
+  double3 xA;
+};
+// Learned SDF: u = l * ms - mc (network input), phi / h = y * mtoh, threshold Tn.
+template <bool LRN>
+struct PairNet {};
+template <>
+struct PairNet<true> {
   float ms, mtoh, Tn;
   float3 mc;
   int pshape;
 };
+template <bool WIN, bool LRN>
+struct PairX : PairF, PairWin<WIN>, PairNet<LRN> {};
 
-template <int KIND, int SDFK>
-LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape) {
-  PairF F;
-  // R_A and R_B (row-major), each column rotated by one lane in FP64 and rounded
+template <int KIND>
+LD int partner_shape(const StepArgs& a, int pid) {
+  if (KIND == KIND_WALL) return a.W.shape[pid];
+  return a.P.shape[KIND == KIND_GHOST ? (pid >> 3) : pid];
+}
+
+template <int KIND, int SDFK, bool WIN, bool LRN>
+LD void make_pair_f(const StepArgs& a, int A, int slot, int pid, PairX<WIN, LRN>& F) {
+  const Partner P = load_partner<KIND>(a, pid);
+  const int pshape = partner_shape<KIND>(a, pid);
+  // R_A and R_B (row-major), rotated in FP64 and rounded
   float ra[9], rb[9];
-  {
-    const int lane = threadIdx.x & 31, ax = lane % 3;
-    const double3 u = d3(ax == 0 ? 1. : 0., ax == 1 ? 1. : 0., ax == 2 ? 1. : 0.);
-    const double3 c = rotate(lane < 3 ? a.P.quat[A] : P.q, u);
-    const float cx = (float)c.x, cy = (float)c.y, cz = (float)c.z;
+  const Quat qA = a.P.quat[A];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      ra[j] = __shfl_sync(FULL, cx, j); ra[3 + j] = __shfl_sync(FULL, cy, j); ra[6 + j] = __shfl_sync(FULL, cz, j);
-      rb[j] = __shfl_sync(FULL, cx, 3 + j); rb[3 + j] = __shfl_sync(FULL, cy, 3 + j); rb[6 + j] = __shfl_sync(FULL, cz, 3 + j);
-    }
+  for (int j = 0; j < 3; ++j) {
+    const double3 u = d3(j == 0 ? 1. : 0., j == 1 ? 1. : 0., j == 2 ? 1. : 0.);
+    const double3 ca = rotate(qA, u), cb = rotate(P.q, u);
+    ra[j] = (float)ca.x; ra[3 + j] = (float)ca.y; ra[6 + j] = (float)ca.z;
+    rb[j] = (float)cb.x; rb[3 + j] = (float)cb.y; rb[6 + j] = (float)cb.z;
   }
   const int shA = a.P.shape[A];
   const float scA = (float)a.P.scale[A];
@@ -1071,8 +1093,8 @@ LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape) {
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j)
       F.M[3 * i + j] = fmaf(rb[i], ra[j], fmaf(rb[3 + i], ra[3 + j], rb[6 + i] * ra[6 + j])) * scA;
-  const double3 d = owner_pos<KIND>(a, A) - P.x;
-  const float3 df = tof(d);
+  const double3 xA = owner_pos<KIND>(a, A);
+  const float3 df = tof(xA - P.x);
   F.dB = f3(fmaf(rb[0], df.x, fmaf(rb[3], df.y, rb[6] * df.z)), fmaf(rb[1], df.x, fmaf(rb[4], df.y, rb[7] * df.z)),
             fmaf(rb[2], df.x, fmaf(rb[5], df.y, rb[8] * df.z)));
   F.invh = (float)P.invh;
@@ -1105,13 +1127,19 @@ LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape) {
     F.sz = (P.gs.x - 1) * (P.gs.y - 1);
     F.cells = a.S.cell16 + a.S.cell_off[pshape];
   }
-  F.key = P.key;
-  if (KIND != KIND_PP) {
+  F.A = A;
+  F.slot = slot;
+  F.scA = scA;
+  F.n0 = a.S.node_off[shA]; F.nn = a.S.node_cnt[shA];
+  F.cl0 = a.S.cl_off[shA]; F.ncl = a.S.cl_cnt[shA];
+  if constexpr (WIN) {
+    F.key = P.key;
     for (int k = 0; k < 9; ++k) F.RA[k] = ra[k] * scA;
     F.n1w = EPS_F * N1;
+    F.xA = xA;
   }
-  F.pshape = pshape;
-  if (a.mlp_inf) {
+  if constexpr (LRN) {
+    F.pshape = pshape;
     // partner frame (length) -> template units (/ scale) -> network input
     const MlpNorm nm = a.mlp_norm[pshape];
     const double ht = 1.0 / (P.invh * P.sc);  // template spacing
@@ -1120,7 +1148,6 @@ LD PairF make_pair_f(const StepArgs& a, int A, const Partner& P, int pshape) {
     F.mtoh = (float)(nm.R / ht);
     F.Tn = a.mlp_band[pshape];
   }
-  return F;
 }
 
 LD float3 mulf(const float* M, float x, float y, float z) {
@@ -1191,13 +1218,13 @@ LD int window_state(const StepArgs& a, double3 x, float3 ra, float e0, int key) 
 
 // FP32 screen of one node (offset nd, template units): false only when the
 // FP64 test (node_hits) certainly rejects it.
-template <int KIND, int SDFK>
-LD bool node_may_hit_f(const StepArgs& a, double3 xA, const PairF& F, float4 nd, bool& looked) {
+template <int KIND, int SDFK, class FX>
+LD bool node_may_hit_f(const StepArgs& a, const FX& F, float4 nd, bool& looked) {
   const float3 l = mulf(F.M, nd.x, nd.y, nd.z) + F.dB;
-  if (KIND == KIND_PP) {
+  if constexpr (KIND == KIND_PP) {
     if (l.x * l.x + l.y * l.y + l.z * l.z > F.R2) return false;
   } else {
-    if (window_state<KIND>(a, xA, mulf(F.RA, nd.x, nd.y, nd.z), F.n1w, F.key) == 0) return false;
+    if (window_state<KIND>(a, F.xA, mulf(F.RA, nd.x, nd.y, nd.z), F.n1w, F.key) == 0) return false;
   }
   const float gx = fmaf(l.x, F.invh, F.cg.x), gy = fmaf(l.y, F.invh, F.cg.y), gz = fmaf(l.z, F.invh, F.cg.z);
   // the FP64 test rejects g < 0 or g >= size - 1 on any axis
@@ -1255,37 +1282,25 @@ LD bool cluster_may_hit_f(const PairF& F, float4 cn, float scA, float* up = null
   return !(ph > F.T + reach);
 }
 
-template <int KIND>
-LD int partner_shape(const StepArgs& a, int pid) {
-  if (KIND == KIND_WALL) return a.W.shape[pid];
-  return a.P.shape[KIND == KIND_GHOST ? (pid >> 3) : pid];
-}
 
 // Screens one (A, partner) pair: cluster cull, then the node screen over the
 // surviving clusters. The nodes the screen cannot reject are written, in node
 // order, to the precision-form node buffer and the pair is queued for
 // k_contacts_f; a pair without such nodes gets its empty contact segment here.
-template <int KIND, int SDFK, bool LRN, bool STATS>
-LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* s_cl, unsigned short* s_sub,
-                      unsigned* s_mask, unsigned (&cnt)[8], unsigned& queued) {
+template <int KIND, int SDFK, bool LRN, bool STATS, class FX>
+LD void screen_pair_f(const StepArgs& a, const FX& F, int li, unsigned char* s_cl, unsigned short* s_sub, unsigned* s_mask,
+                      unsigned* s_dir, unsigned (&cnt)[8], unsigned& queued) {
   const int lane = threadIdx.x & 31;
   __syncwarp();  // the previous pair's write pass may still read s_cl / s_mask
-  const int shA = a.P.shape[A];
-  const int n0 = a.S.node_off[shA], nn = a.S.node_cnt[shA], cl0 = a.S.cl_off[shA], ncl = a.S.cl_cnt[shA];
-  const float scA = (float)a.P.scale[A];
-  const double3 xA = owner_pos<KIND>(a, A);
-  PairF F;
-  {
-    const Partner P = load_partner<KIND>(a, pid);
-    F = make_pair_f<KIND, SDFK>(a, A, P, partner_shape<KIND>(a, pid));
-  }
+  const int A = F.A, slot = F.slot, n0 = F.n0, nn = F.nn, cl0 = F.cl0, ncl = F.ncl;
+  const float scA = F.scA;
   int nsurv = 0;
   for (int c0 = 0; c0 < ncl; c0 += 32) {
     const int c = c0 + lane;
     bool keep = false;
     if (c < ncl) keep = cluster_may_hit_f<KIND, SDFK>(F, __ldg(a.S.cl_sphere_f + cl0 + c), scA);
     const unsigned m = __ballot_sync(FULL, keep);
-    if (keep) s_cl[nsurv + __popc(m & lanemask_lt())] = c;
+    if (keep) s_cl[nsurv + __popc(m & lanemask_lt())] = (unsigned char)c;
     nsurv += __popc(m);
   }
   __syncwarp();
@@ -1303,7 +1318,8 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
       const float4 sp = __ldg(a.S.sub_sphere + 4 * cl0 + sid);
       float up = INFINITY;
       keep = sp.w >= 0.f && cluster_may_hit_f<KIND, SDFK>(F, sp, scA, LRN ? &up : nullptr);
-      if (LRN && up <= F.Tn) sid |= 0x8000;
+      if constexpr (LRN)
+        if (up <= F.Tn) sid |= 0x8000;
     }
     const unsigned m = __ballot_sync(FULL, keep);
     if (keep) s_sub[nsub + __popc(m & lanemask_lt())] = (unsigned short)sid;
@@ -1320,7 +1336,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
     return ni < nn ? ni : nn;
   };
   int total = 0;
-  if (LRN) {
+  if constexpr (LRN) {
     // Learned form: the nodes the partner's bounds cannot reject go to the network of the
     // partner's shape (k_net_screen, tensor cores), which decides with the grid test of
     // the nodes it keeps, unless their sub-cluster is marked (then the grid test runs
@@ -1328,7 +1344,6 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
     // pending (the marked ones with a passing verdict already; k_net_compact queues the
     // survivors for the FP64 pass); a pair without takes the plain screen's tail.
     const NetView& Q = a.net[li];
-    unsigned* s_dir = reinterpret_cast<unsigned*>(s_cl);  // the cluster list is spent
     int tnet = 0, tdir = 0;
     for (int k = 0; k < nch; ++k) {
       const int ni = node_of(k);
@@ -1339,12 +1354,12 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
       if (ni < nn) {
         const float4 nd = __ldg(a.S.node_pos_f + n0 + ni);
         if (marked) {
-          may = node_may_hit_f<KIND, SDFK>(a, xA, F, nd, looked);
+          may = node_may_hit_f<KIND, SDFK>(a, F, nd, looked);
         } else {
           const float3 l = mulf(F.M, nd.x, nd.y, nd.z) + F.dB;
           bool adm;
-          if (KIND == KIND_PP) adm = !(l.x * l.x + l.y * l.y + l.z * l.z > F.R2);
-          else adm = window_state<KIND>(a, xA, mulf(F.RA, nd.x, nd.y, nd.z), F.n1w, F.key) != 0;
+          if constexpr (KIND == KIND_PP) adm = !(l.x * l.x + l.y * l.y + l.z * l.z > F.R2);
+          else adm = window_state<KIND>(a, F.xA, mulf(F.RA, nd.x, nd.y, nd.z), F.n1w, F.key) != 0;
           const float gx = fmaf(l.x, F.invh, F.cg.x), gy = fmaf(l.y, F.invh, F.cg.y), gz = fmaf(l.z, F.invh, F.cg.z);
           const float lo = fminf(gx, fminf(gy, gz));
           const float hi = fmaxf(gx - F.ux, fmaxf(gy - F.uy, gz - F.uz));
@@ -1435,7 +1450,7 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
       const int ni = node_of(k);
       if (STATS) cnt[4] += __popc(__ballot_sync(FULL, ni < nn));
       bool may = false, looked = false;
-      if (ni < nn) may = node_may_hit_f<KIND, SDFK>(a, xA, F, __ldg(a.S.node_pos_f + n0 + ni), looked);
+      if (ni < nn) may = node_may_hit_f<KIND, SDFK>(a, F, __ldg(a.S.node_pos_f + n0 + ni), looked);
       if (STATS) cnt[3] += __popc(__ballot_sync(FULL, looked));
       const unsigned m = __ballot_sync(FULL, may);
       if (lane == 0) s_mask[k] = m;
@@ -1483,38 +1498,59 @@ LD void screen_pair_f(const StepArgs& a, int A, int slot, int pid, int li, int* 
   }
 }
 
-// One warp per listed pair: the flat pair lists of the kinds in KINDS, in
+// A warp takes up to SCREEN_PAIRS pairs at a time: its lanes form their constants (about 350
+// instructions of a pair's 1,100 when the whole warp formed them for each), then it screens them one by
+// one. The flat pair lists of the kinds in KINDS, in
 // particle, wall, image order.
 // Particle-only screens fit 64 registers (8 blocks per SM); walls and images
 // need the window test's FP64 registers.
+static constexpr int SCREEN_PAIRS = 8;
 template <int KINDS, int SDFK, bool LRN, bool STATS>
 __global__ void __launch_bounds__(NP_WARPS * 32, KINDS == 1 ? 8 : 5) k_screen_f(StepArgs a, int li, int kinds) {
-  __shared__ int s_cl[NP_WARPS][MAXCL];
+  __shared__ unsigned char s_cl[NP_WARPS][MAXCL];
   __shared__ unsigned short s_sub[NP_WARPS][4 * MAXCL];
   __shared__ unsigned s_mask[NP_WARPS][MAXCL];
-  const int warp = threadIdx.x >> 5;
+  __shared__ unsigned s_dir[NP_WARPS][LRN ? MAXCL : 1];
+  __shared__ PairX<KINDS != 1, LRN> s_pair[NP_WARPS][SCREEN_PAIRS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (KINDS & 1) ? a.pl.ctr[0] : 0;
   const int n1 = (kinds & KINDS & 2) && a.pw.cap > 0 ? a.pl.ctr[1] : 0;
   const int n2 = (kinds & KINDS & 4) ? a.pl.ctr[2] : 0;
   const int tot = n0 + n1 + n2;
   unsigned cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // warp-uniform screen counters
   unsigned queued[3] = {0, 0, 0};              // nodes queued by partner kind
-  for (int e = blockIdx.x * NP_WARPS + warp; e < tot; e += gridDim.x * NP_WARPS) {
-    if ((KINDS & 1) && e < n0) {
-      const unsigned idx = __ldg(a.pl.list[0] + e);
-      const int A = idx / a.pp.cap;
-      screen_pair_f<KIND_PP, SDFK, LRN, STATS>(a, A, idx - A * a.pp.cap, __ldg(a.pp.id + idx), li, s_cl[warp], s_sub[warp],
-                                        s_mask[warp], cnt, queued[0]);
-    } else if ((KINDS & 2) && e < n0 + n1) {
-      const unsigned idx = a.pl.list[1][e - n0];
-      const int A = idx / a.pw.cap;
-      screen_pair_f<KIND_WALL, SDFK, LRN, STATS>(a, A, idx - A * a.pw.cap, a.pw.id[idx], li, s_cl[warp], s_sub[warp],
-                                          s_mask[warp], cnt, queued[1]);
-    } else if (KINDS & 4) {
-      const unsigned idx = __ldg(a.pl.list[2] + e - n0 - n1);
-      const int A = idx / a.pgh.cap;
-      screen_pair_f<KIND_GHOST, SDFK, LRN, STATS>(a, A, idx - A * a.pgh.cap, __ldg(a.pgh.id + idx), li, s_cl[warp], s_sub[warp],
-                                           s_mask[warp], cnt, queued[2]);
+  const int W = gridDim.x * NP_WARPS;
+  const int per = max(1, min(SCREEN_PAIRS, tot / W));
+  for (int e0 = (blockIdx.x * NP_WARPS + warp) * per; e0 < tot; e0 += W * per) {
+    __syncwarp();  // the previous pairs' records may still be read
+    const int e = e0 + lane;
+    if (lane < per && e < tot) {
+      auto& F = s_pair[warp][lane];
+      if ((KINDS & 1) && e < n0) {
+        const unsigned idx = __ldg(a.pl.list[0] + e);
+        const int A = idx / a.pp.cap;
+        make_pair_f<KIND_PP, SDFK>(a, A, idx - A * a.pp.cap, __ldg(a.pp.id + idx), F);
+      } else if ((KINDS & 2) && e < n0 + n1) {
+        const unsigned idx = a.pl.list[1][e - n0];
+        const int A = idx / a.pw.cap;
+        make_pair_f<KIND_WALL, SDFK>(a, A, idx - A * a.pw.cap, a.pw.id[idx], F);
+      } else if (KINDS & 4) {
+        const unsigned idx = __ldg(a.pl.list[2] + e - n0 - n1);
+        const int A = idx / a.pgh.cap;
+        make_pair_f<KIND_GHOST, SDFK>(a, A, idx - A * a.pgh.cap, __ldg(a.pgh.id + idx), F);
+      }
+    }
+    __syncwarp();
+    for (int p = 0; p < per && e0 + p < tot; ++p) {
+      const auto& F = s_pair[warp][p];
+      if ((KINDS & 1) && e0 + p < n0) {
+        screen_pair_f<KIND_PP, SDFK, LRN, STATS>(a, F, li, s_cl[warp], s_sub[warp], s_mask[warp], s_dir[warp], cnt, queued[0]);
+      } else if constexpr ((KINDS & 6) != 0) {
+        if ((KINDS & 2) && e0 + p < n0 + n1)
+          screen_pair_f<KIND_WALL, SDFK, LRN, STATS>(a, F, li, s_cl[warp], s_sub[warp], s_mask[warp], s_dir[warp], cnt, queued[1]);
+        else
+          screen_pair_f<KIND_GHOST, SDFK, LRN, STATS>(a, F, li, s_cl[warp], s_sub[warp], s_mask[warp], s_dir[warp], cnt, queued[2]);
+      }
     }
   }
   if (STATS && (threadIdx.x & 31) == 0) {
