@@ -259,6 +259,9 @@ struct StepArgs {
   float skin;             // neighbour-list margin beyond the candidate reach (length)
   double3* xb;            // particle order: position at the last list build
   float4* qb;             // particle order: orientation at the last list build
+  unsigned char* kin;     // particle order: in a cell, as the last list build expects it
+  int cross;              // 1: the build lists bodies that crossed a periodic face where they stand
+                          //   from the next step on (xb is that position), too
   float4* rec;            // particle order, 2 per particle, written with the drift: FP32 centre and
                           //   cell key; FP32 orientation
   ImageList gl;
@@ -272,8 +275,8 @@ struct StepArgs {
 };
 
 // Neighbour lists: when *a.reuse is set, the cell sort of the keys into sorted_idx and the
-// lists (neighbours.cu); sums: REBUILD_SUMS entries.
-// With a.gl.list the image list, too, from a second sort of the wrapped positions.
+// lists (neighbours.cu); sums: REBUILD_SUMS + 1 entries.
+// With a.gl.list the image list, too.
 constexpr int REBUILD_SUMS = 4096;
 struct ImageSort {
   BucketScratch w;

@@ -86,7 +86,64 @@ LD void grid_cell_sort(cg::grid_group& grid, const int* key, int n, int ncells, 
       __syncthreads();
     }
   }
-  grid.sync();
+  if (nbig > 0 || nmid > 0) grid.sync();
+}
+
+// Bounding spheres within reach + skin, with a margin beyond the FP32 rounding of the step's test.
+LD bool in_reach(const StepArgs& a, float4 pa, float n1a, float4 pb) {
+  const float Rs = __fmul_rn(__fmaf_rn(1e-5f, __fadd_rn(n1a, n1_f(pb)), __fadd_rn(reach_f(pa, n1a, pb), a.skin)),
+                             1.0f + 1e-4f);
+  return !(dist2_f(pa, pb) > __fmul_rn(Rs, Rs));
+}
+
+// Bodies that crossed a periodic face in this step: they stand in no cell, and from the next step
+// on in the domain at their wrapped position. Their pairs there are added to the lists now, so
+// that the next step, which finds them moved by the domain, needs no rebuild of its own. One
+// warp per such body; list[0, m) holds them. (Only where the domain is wide enough that a
+// body cannot be near both positions: a.cross.)
+LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* list, int m) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
+  const int n = a.P.n;
+  const GridP& g = a.pg;
+  const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
+  const bool sep = a.S.sup_n != nullptr;
+  const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
+  for (int v = tid >> 5; v < m; v += T >> 5) {
+    const int W = __ldcg(list + v);
+    const double3 xw = wrap_pos(a.P.pos[W], g, a.wrap_axes);
+    int key;
+    CandRec rw = cand_rec(a, W, key);
+    rw.p = make_float4((float)xw.x, (float)xw.y, (float)xw.z, rw.p.w);
+    const float n1w = n1_f(rw.p);
+    auto add = [&](int B, float4 pB) {
+      if (!in_reach(a, rw.p, n1w, pB)) return;
+      CandRec rb = cand_rec(a, B, key);
+      rb.p = pB;
+      const bool first = W < B;
+      const CandRec &r0 = first ? rw : rb, &r1 = first ? rb : rw;
+      if (sep && pair_separated<2>(sup, r0.p, n1_f(r0.p), r0.q, r0.sc, r0.sh, r1.p, r1.q, r1.sc, r1.sh, gap)) return;
+      const int A = first ? W : B, at = atomicAdd(&a.nbr_cnt[A], 1);
+      if (at >= 0 && at < a.nbr_cap) a.nbr[(size_t)at * n + A] = first ? B : W;
+      if (at >= a.nbr_cap) {
+        atomicMax(&a.status->need_nbr, at + 1);
+        atomicOr(&a.status->flags, OVF_NBR);
+      }
+    };
+    const double R = a.P.radius[W] + a.rmax + (double)a.skin;
+    const double ext = 1.001 * R + 1e-4 * (fabs(xw.x) + fabs(xw.y) + fabs(xw.z) + 4.0 * R);
+    const int3 lo = ball_cell(xw - d3(ext, ext, ext), g), hi = ball_cell(xw + d3(ext, ext, ext), g);
+    for (int z = lo.z; z <= hi.z; ++z)
+      for (int y = lo.y; y <= hi.y; ++y) {
+        const int h0 = lin3(make_int3(lo.x, y, z), g.size);
+        const int st = __ldcg(w.offs + h0 + 1), en = __ldcg(w.offs + h0 + (hi.x - lo.x) + 2);
+        for (int k = st + lane; k < en; k += 32) add(a.pk_meta[k].y, a.cell_pk[k]);
+      }
+    for (int u = v + 1 + lane; u < m; u += 32) {  // the other bodies of the list, once
+      const int B = __ldcg(list + u);
+      const double3 x = wrap_pos(a.P.pos[B], g, a.wrap_axes);
+      add(B, make_float4((float)x.x, (float)x.y, (float)x.z, __ldg(a.rec_s + B).x));
+    }
+  }
 }
 
 // The image list: owners A and images that some step before the next rebuild may find as
@@ -95,36 +152,50 @@ LD void grid_cell_sort(cg::grid_group& grid, const int* key, int n, int ncells, 
 // outside the domain, or above the y bound, which the image keys test z against); in between,
 // bodies keep their side of the domain's faces, or the lists are rebuilt. The search is that of
 // k_ghost_candidates with the list's margin.
-LD void grid_image_list(cg::grid_group& grid, const StepArgs& a, const ImageSort& im, int* sums, int* sw) {
+LD void grid_image_list(cg::grid_group& grid, const StepArgs& a, const BucketScratch& w1, const int* idx1,
+                        const ImageSort& im, int* sums, int* sw) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
   const int n = a.P.n;
   const GridP& g = a.pg;
-  for (int i = tid; i < n; i += T)
-    im.key[i] = lin3(clamp_cell(cell_of(wrap_pos(a.P.pos[i], g, a.wrap_axes), g), g.size), g.size);
   if (tid == 0) *a.G.count = *a.gl.count = 0;
+  // The owners are searched in the cells of their wrapped positions. Those of bodies in a cell are
+  // the particle sort's own; the bodies in no cell are tested one by one with every image while
+  // they are few (the crossers of a step), and all bodies sorted again otherwise (a second sort
+  // was a third of a rebuild of 100k particles).
+  const int n0 = __ldcg(w1.offs + 1), nL = n - __ldcg(w1.offs + g.ncells + 1);
+  const bool resort = n0 + nL > 64;
   grid.sync();
-  grid_cell_sort(grid, im.key, n, g.ncells, im.w, im.idx, sums, sw);
-  const double m = 0.4 * (double)a.skin * 1.01;
-  for (int k = tid; k < n; k += T) {
-    const int B = __ldcg(im.idx + k);
-    const double3 p = wrap_pos(a.P.pos[B], g, a.wrap_axes);
-    im.pk[k] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)a.P.radius[B]);
+  if (resort) {
+    for (int i = tid; i < n; i += T)
+      im.key[i] = lin3(clamp_cell(cell_of(wrap_pos(a.P.pos[i], g, a.wrap_axes), g), g.size), g.size);
+    grid.sync();
+    grid_cell_sort(grid, im.key, n, g.ncells, im.w, im.idx, sums, sw);
+    for (int k = tid; k < n; k += T) {
+      const int B = __ldcg(im.idx + k);
+      const double3 p = wrap_pos(a.P.pos[B], g, a.wrap_axes);
+      im.pk[k] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)a.P.radius[B]);
+    }
   }
+  const int* offs = resort ? im.w.offs : w1.offs;
+  const int* idx = resort ? im.idx : idx1;
+  const float4* pk = resort ? im.pk : a.cell_pk;
+  const double m = 0.4 * (double)a.skin * 1.01;
   for (int i0 = tid - lane; i0 < n; i0 += T) {
     const int i = i0 + lane;
     double3 x = d3(0., 0., 0.);
     if (i < n) x = a.P.pos[i];
     for (int s = 0; s < a.G.nsets; ++s) {
       bool on[2] = {false, false};  // in place, moved
-      if (i < n) {
+      // (with a.cross also where a body beyond a face stands from the next step on)
+      for (int q = 0; i < n && q < (a.cross ? 2 : 1); ++q) {
         const int mask = a.G.mask[s];
-        const double3 p = image_base(x, g, a.wrap_axes, mask);
+        const double3 p = q == 0 ? image_base(x, g, a.wrap_axes, mask) : wrap_pos(x, g, a.wrap_axes);
         const double ux = fabs((p.x - g.mn.x) * g.inv.x), uy = fabs((p.y - g.mn.y) * g.inv.y),
                      uz = fabs((p.z - g.mn.z) * g.inv.z);
         const double ex = m * g.inv.x + 1e-9, ey = m * g.inv.y + 1e-9, ez = m * g.inv.z + 1e-9;
-        on[1] = (!(mask & 1) || ux < 1.0 + ex) && (!(mask & 2) || uy < 1.0 + ey) && (!(mask & 4) || uz < 1.0 + ez);
+        on[1] = on[1] || ((!(mask & 1) || ux < 1.0 + ex) && (!(mask & 2) || uy < 1.0 + ey) && (!(mask & 4) || uz < 1.0 + ez));
         const bool stays = ((mask & 1) && ux >= 1.0 - ex) || ((mask & 2) && uy >= 1.0 - ey) || ((mask & 4) && uz >= 1.0 - ez);
-        on[0] = stays && (ghost_key(p, g) >= 0 || p.z >= g.mx.y - m);
+        on[0] = on[0] || (stays && (ghost_key(p, g) >= 0 || p.z >= g.mx.y - m));
       }
       for (int v = 0; v < 2; ++v) {
         const unsigned b = __ballot_sync(FULL, on[v]);
@@ -142,39 +213,49 @@ LD void grid_image_list(cg::grid_group& grid, const StepArgs& a, const ImageSort
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
   for (int v = tid >> 5; v < nimg; v += T >> 5) {  // one warp per image
     const int t = __ldcg(a.G.list + v), moved = t & 1, s = (t >> 1) / n, i = (t >> 1) % n;
-    double3 xg = image_base(a.P.pos[i], g, a.wrap_axes, a.G.mask[s]);
-    if (moved) xg += image_offset(g, a.G.mask[s]);
+    const double3 base = image_base(a.P.pos[i], g, a.wrap_axes, a.G.mask[s]), xw = wrap_pos(a.P.pos[i], g, a.wrap_axes);
     const double Rg = grid_reach(a, i);
-    const double r = (a.rmax + Rg + (double)a.skin) * 1.001 + 1e-4 * (fabs(xg.x) + fabs(xg.y) + fabs(xg.z));
-    const int3 lo = ball_cell(xg - d3(r, r, r), g), hi = ball_cell(xg + d3(r, r, r), g);
     int kB;
     CandRec rb = cand_rec(a, i, kB);
-    rb.p = make_float4((float)xg.x, (float)xg.y, (float)xg.z, 0.f);
-    const float n1g = n1_f(rb.p), Rgs = (float)Rg + a.skin;
-    for (int z = lo.z; z <= hi.z; ++z) {
-      for (int y = lo.y; y <= hi.y; ++y) {
-        const int h0 = lin3(make_int3(lo.x, y, z), g.size);
-        const int st = __ldcg(im.w.offs + h0 + 1), en = __ldcg(im.w.offs + h0 + (hi.x - lo.x) + 2);
-        for (int k0 = st; k0 < en; k0 += 32) {
-          const int k = k0 + lane;
-          bool keep = false;
-          int A = 0;
-          if (k < en) {
-            const float4 pa = im.pk[k];
-            const float R = (pa.w + Rgs) * (1.0f + 1e-4f) + 1e-5f * (n1g + n1_f(pa));
-            if (!(dist2_f(pa, rb.p) > R * R)) {
-              A = __ldcg(im.idx + k);
-              int kA;
-              const CandRec ra = cand_rec(a, A, kA);
-              keep = !(sep && pair_separated<2>(sup, pa, n1_f(pa), ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh, gap));
-            }
-          }
-          const unsigned b = __ballot_sync(FULL, keep);
-          int at = 0;
-          if (lane == 0 && b) at = atomicAdd(a.gl.count, __popc(b));
-          at = __shfl_sync(FULL, at, 0) + __popc(b & ((1u << lane) - 1u));
-          if (keep && at < a.gl.cap) a.gl.list[at] = make_int2(A | (moved ? (int)0x80000000u : 0), (i << 3) | s);
+    const float Rgs = (float)Rg + a.skin;
+    // the second position only where the body crosses a face of an axis the set does not wrap
+    const int places = a.cross && (base.x != xw.x || base.y != xw.y || base.z != xw.z) ? 2 : 1;
+    for (int q = 0; q < places; ++q) {
+      double3 xg = q == 0 ? base : xw;
+      if (moved) xg += image_offset(g, a.G.mask[s]);
+      const double r = (a.rmax + Rg + (double)a.skin) * 1.001 + 1e-4 * (fabs(xg.x) + fabs(xg.y) + fabs(xg.z));
+      const int3 lo = ball_cell(xg - d3(r, r, r), g), hi = ball_cell(xg + d3(r, r, r), g);
+      rb.p = make_float4((float)xg.x, (float)xg.y, (float)xg.z, 0.f);
+      const float n1g = n1_f(rb.p);
+      // one owner per lane (A < 0: none)
+      auto add = [&](int A, float4 pa) {
+        bool keep = false;
+        const float R = (pa.w + Rgs) * (1.0f + 1e-4f) + 1e-5f * (n1g + n1_f(pa));
+        if (A >= 0 && !(dist2_f(pa, rb.p) > R * R)) {
+          int kA;
+          const CandRec ra = cand_rec(a, A, kA);
+          keep = !(sep && pair_separated<2>(sup, pa, n1_f(pa), ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh, gap));
         }
+        const unsigned b = __ballot_sync(FULL, keep);
+        int at = 0;
+        if (lane == 0 && b) at = atomicAdd(a.gl.count, __popc(b));
+        at = __shfl_sync(FULL, at, 0) + __popc(b & ((1u << lane) - 1u));
+        if (keep && at < a.gl.cap) a.gl.list[at] = make_int2(A | (moved ? (int)0x80000000u : 0), (i << 3) | s);
+      };
+      for (int z = lo.z; z <= hi.z; ++z) {
+        for (int y = lo.y; y <= hi.y; ++y) {
+          const int h0 = lin3(make_int3(lo.x, y, z), g.size);
+          const int st = __ldcg(offs + h0 + 1), en = __ldcg(offs + h0 + (hi.x - lo.x) + 2);
+          for (int k0 = st; k0 < en; k0 += 32) {
+            const int k = min(k0 + lane, en - 1);
+            add(k0 + lane < en ? __ldcg(idx + k) : -1, pk[k]);
+          }
+        }
+      }
+      for (int k0 = 0; !resort && k0 < n0 + nL; k0 += 32) {  // the bodies in no cell
+        const int k = min(k0 + lane, n0 + nL - 1), A = __ldcg(idx1 + (k < n0 ? k : n - nL + k - n0));
+        const double3 x = wrap_pos(a.P.pos[A], g, a.wrap_axes);
+        add(k0 + lane < n0 + nL ? A : -1, make_float4((float)x.x, (float)x.y, (float)x.z, __ldg(a.rec_s + A).x));
       }
     }
   }
@@ -194,6 +275,9 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
   const int n = a.P.n;
+  int* cross_n = sums + REBUILD_SUMS;
+  int* cross_list = w.tmp;  // the sort's, free after it
+  if (tid == 0) *cross_n = 0;
   grid_cell_sort(grid, a.P.key, n, a.pg.ncells, w, sorted_idx, sums, sw);
   if (tid == 0) atomicAdd(&a.status->builds, 1);
   for (int k = tid; k < n; k += T) pack_cell(a, k, __ldcg(sorted_idx + k));
@@ -238,7 +322,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
     cnt[lane] = 0;
     while (__any_sync(FULL, r < rows || k < en)) {
       int m = 0;
-      while (m < RB_BUF) {
+      while (m <= RB_BUF - 4) {
         if (k >= en) {
           if (r >= rows) break;
           // the cells of a row are contiguous in the sorted order
@@ -248,11 +332,13 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
           ++r;
           continue;
         }
-        const float4 pb = a.cell_pk[k];
-        const float Rs = __fmul_rn(__fmaf_rn(1e-5f, __fadd_rn(n1a, n1_f(pb)), __fadd_rn(reach_f(pa, n1a, pb), a.skin)),
-                                   1.0f + 1e-4f);
-        if (!(dist2_f(pa, pb) > __fmul_rn(Rs, Rs)) && a.pk_meta[k].y > A) buf[32 * m++ + lane] = k;
-        ++k;
+        float4 pb[4];  // four bodies' loads in flight
+#pragma unroll
+        for (int u = 0; u < 4; ++u) pb[u] = a.cell_pk[min(k + u, en - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k + u < en && in_reach(a, pa, n1a, pb[u]) && a.pk_meta[k + u].y > A) buf[32 * m++ + lane] = k + u;
+        k += 4;
       }
       int incl = m;
 #pragma unroll
@@ -291,7 +377,12 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
       a.nbr_cnt[A] = nl <= a.nbr_cap ? nl : -1;
       if (nl > a.nbr_cap) atomicOr(&a.status->flags, OVF_NBR);
       need = max(need, nl);
-      a.xb[A] = xA;
+      // where the body stands from the next step on
+      const double3 xw = a.cross ? wrap_pos(xA, a.pg, a.wrap_axes) : xA;
+      a.xb[A] = xw;
+      const int k0 = a.pk_meta[t].x, kw = a.cross && k0 < 0 ? hash_key(xw, a.pg) : k0;
+      a.kin[A] = kw >= 0;
+      if (k0 < 0 && kw >= 0) cross_list[atomicAdd(cross_n, 1)] = A;
       const Quat q = a.P.quat[A];
       a.qb[A] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
     }
@@ -299,7 +390,11 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   }
   need = __reduce_max_sync(FULL, need);
   if (lane == 0 && need > 0) atomicMax(&a.status->need_nbr, need);
-  if (a.gl.list) grid_image_list(grid, a, im, sums, sw);
+  if (a.cross) {
+    grid.sync();
+    grid_cross_lists(a, w, cross_list, __ldcg(cross_n));
+  }
+  if (a.gl.list) grid_image_list(grid, a, w, sorted_idx, im, sums, sw);
 }
 
 void launch_rebuild(const StepArgs& a, const BucketScratch& w, const ImageSort& img, int* sorted_idx, int* sums,

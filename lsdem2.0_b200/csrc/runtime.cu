@@ -313,6 +313,7 @@ struct lsdem_solver {
   int flags = 0;
   int precision = PREC_FP64;
   double rmax_p = 0.;        // largest particle bounding radius (set at initialize)
+  double rg_max = 0.;        // largest distance of a particle's grid corner from its centre
   std::string err;
   // model
   std::vector<ShapeHost> shapes;
@@ -402,6 +403,7 @@ struct lsdem_solver {
   bool grow_nbr = false;
   DArr<int> reuse;
   DArr<double3> xb;
+  DArr<unsigned char> kin;
   DArr<float4> qb, rec, rec_s;  // orientation at the last rebuild; FP32 records of the search
   DArr<int> nbr, nbr_cnt, rb_sums;
   DArr<int2> img_list;       // image list (k_rebuild)
@@ -1011,6 +1013,15 @@ void initialize(lsdem_solver* s) {
   double rp = 0., rw = 0.;
   for (double r : s->P.radius) rp = std::max(rp, r);
   s->rmax_p = rp;
+  s->rg_max = 0.;
+  for (int i = 0; i < s->P.n(); ++i) {
+    double r2 = 0.;
+    for (int k = 0; k < 3; ++k) {
+      const double o = s->P.origin[3 * i + k], e = o + (s->shapes[s->P.shape[i]].size[k] - 1) / s->P.invh[i];
+      r2 += std::max(o * o, e * e);
+    }
+    s->rg_max = std::max(s->rg_max, std::sqrt(r2));
+  }
   for (double r : s->W.radius) rw = std::max(rw, r);
   set_grid(s->pg, s->dmin, s->dmax, s->P.n() ? 2.0 * rp : 0.0);
   set_grid(s->wg, s->dmin, s->dmax, s->W.n() ? 2.0 * rw : 0.0);
@@ -1035,7 +1046,8 @@ void initialize(lsdem_solver* s) {
     }
     CK(s->rec_s.upload(rs.data(), rs.size(), st));
     CK(cudaStreamSynchronize(st));  // rs goes out of scope
-    CK(s->rb_sums.alloc(REBUILD_SUMS));
+    CK(s->rb_sums.alloc(REBUILD_SUMS + 1));
+    CK(s->kin.alloc(std::max(n, 1)));
     CK(s->nbr_cnt.alloc(std::max(n, 1)));
     CK(s->pk_meta.alloc(std::max(n, 1)));
     CK(s->pk_q.alloc(std::max(n, 1)));
@@ -1198,6 +1210,7 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.skin = s->skin;
   a.xb = s->xb.p;
   a.qb = s->qb.p;
+  a.kin = s->kin.p;
   a.rec = s->rec.p;
   // translated images with the lists on: from the image list, the wrap at the step's end
   const bool img = reuse && s->nsets > 0 && !(s->periodic & 8);
@@ -1205,6 +1218,11 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.gl.count = s->img_count.p;
   a.gl.cap = (int)std::min<long long>(s->img_list.n, 0x7fffffff);
   a.wrap_axes = img ? (s->periodic & 7) : 0;
+  // wide along every periodic axis: no body or image is near another at two positions a domain apart
+  const double wide = 8.0 * s->rmax_p, L[3] = {s->pg.mx.x - s->pg.mn.x, s->pg.mx.y - s->pg.mn.y, s->pg.mx.z - s->pg.mn.z};
+  a.cross = img ? 1 : 0;
+  for (int ax = 0; ax < 3; ++ax)
+    if (((s->periodic >> ax) & 1) && !(L[ax] > wide + 2.0 * s->rg_max)) a.cross = 0;
   a.rec_s = s->rec_s.p;
   a.nbr = reuse ? s->nbr.p : nullptr;
   a.nbr_cnt = s->nbr_cnt.p;

@@ -127,7 +127,7 @@ __global__ void k_integrate_first(StepArgs a) {
       const bool beyond = ((a.wrap_axes & 1) && (x.x < g.mn.x || x.x >= g.mx.x)) ||
                           ((a.wrap_axes & 2) && (x.y < g.mn.y || x.y >= g.mx.y)) ||
                           ((a.wrap_axes & 4) && (x.z < g.mn.z || x.z >= g.mx.z));
-      if (!(move * (1.0f + 1e-6f) <= a.move) || (key < 0) != (P.key[i] < 0) || beyond) atomicOr(a.reuse, 2);
+      if (!(move * (1.0f + 1e-6f) <= a.move) || (key >= 0) != (a.kin[i] != 0) || beyond) atomicOr(a.reuse, 2);
     }
     P.key[i] = key;
     if (a.reuse) {  // the candidate search's records
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const int A = t0 + lane + 32 * q;
-      listed[q] = lane < PER && A < a.P.n ? max(a.nbr_cnt[A], 0) : 0;
+      listed[q] = lane < PER && A < a.P.n ? min(max(a.nbr_cnt[A], 0), a.nbr_cap) : 0;
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
