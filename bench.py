@@ -97,17 +97,11 @@ def _bf16_peak():
 NET_FLOP = 8704
 
 
-# Algorithmic bytes of the narrowphase kernel of each form.
-# FP64 form, k_narrowphase (detection and forces fused): per owner particle (pose,
-# velocities, slot counts, force/torque write: 208 B), per candidate pair (partner id,
-# pose, velocities, shape and material scalars, segment bookkeeping, reaction atomics:
-# 236 B) and per contact (node id, FP64 spring read and write, history lookup: 56 B).
-# Precision forms, k_screen_f (the screen; contacts are evaluated by the separate
-# FP64 contact pass): per owner particle (pose, scale, shape, slot count: 72 B) and
+# Algorithmic bytes of k_screen_f (the screen of every form; contacts are evaluated by the
+# separate FP64 contact pass): per owner particle (pose, scale, shape, slot count: 72 B) and
 # per candidate pair (partner id, pose, radius, grid origin and spacing, shape,
-# segment words: 120 B).
-B_PARTICLE = 208
-B_PAIR = 236
+# segment words: 120 B). B_CONTACT: per contact of a step (node id, FP64 spring read and
+# write, history lookup).
 B_CONTACT = 56
 B_PARTICLE_SCREEN = 72
 B_PAIR_SCREEN = 120
@@ -774,13 +768,8 @@ def main():
         avg_ms = (np_ms + g_ms) / max(1, np_calls + g_calls)
         # a step runs the particle/wall launch and the image launch: per-launch bytes = per-step / 2
         launches_per_step = 2 if g_calls else 1
-        if prec == 0:
-            kernel = "k_narrowphase"
-            bytes_launch = (B_PARTICLE * n * launches_per_step + B_PAIR * pairs + B_CONTACT * stats["contacts"]) / \
-                launches_per_step
-        else:
-            kernel = "k_screen_f"
-            bytes_launch = (B_PARTICLE_SCREEN * n * launches_per_step + B_PAIR_SCREEN * pairs) / launches_per_step
+        kernel = "k_screen_f"
+        bytes_launch = (B_PARTICLE_SCREEN * n * launches_per_step + B_PAIR_SCREEN * pairs) / launches_per_step
         # DRAM bytes per launch: the capture's measured traffic scaled by algorithmic bytes
         # (its excess over them is the 16-bit template store read once per step after the
         # L2 flush, so the scaling overstates it for larger cases: an upper estimate)

@@ -346,20 +346,21 @@ int lsdem_write_vtu(lsdem_solver* s, const char* dir, unsigned long long frame, 
  * the step's launches up to the external-force hook (captured once per history
  * parity and re-captured when the step's arguments change; on the legacy default
  * stream the replay runs on a private blocking stream, ordered with it both ways);
- * the hook and the second half kick follow the replay. on = 0 launches every kernel
+ * the hook and the second half kick follow the replay, or, without a hook and inside a
+ * batch, the kick is part of the next step's. on = 0 launches every kernel
  * of every step instead. Default on. No counterpart in the reference (which
  * launches each kernel and synchronises with the host every step). */
 int lsdem_set_graphs(lsdem_solver* s, int on);
 
-/* Neighbour lists (exact; default on): the candidate search tests, per particle, the
- * bodies it found within its reach plus a margin (a tenth of the largest bounding
- * radius) at the last rebuild, keeping those whose cell is in its cell window and
- * which pass the same bounding-sphere test, in the walk's order. The cell sort and the
- * rebuild run only in steps where a particle moved 0.04 of the largest bounding
- * radius since the last rebuild (a periodic wrap included). The candidate pairs,
- * their order and so every result are the same as with on = 0, which sorts and walks
- * the 27 cells every step as the reference does (LSSolver.h:1000-1011,
- * mySpatialGrid.cu, LSParticleContactDetectionKernel.cu). */
+/* Neighbour lists (default on): the candidate search tests, per particle, the bodies that
+ * its last rebuild found within its reach plus a margin (a tenth of the largest bounding
+ * radius) and not provably 0.8 of the margin apart, with the step's own tests and in the
+ * walk's order. The cell sort and the rebuild run only in steps where a point of a body
+ * may have moved 0.04 of the largest bounding radius since the last rebuild, a body
+ * entered or left the domain, or one crossed a periodic face. Contacts and results are
+ * the same as with on = 0, which sorts and walks the 27 cells every step as the
+ * reference does (LSSolver.h:1000-1011, mySpatialGrid.cu,
+ * LSParticleContactDetectionKernel.cu). */
 int lsdem_set_neighbour_lists(lsdem_solver* s, int on);
 
 /* Snapshot of the dynamic state (no counterpart in the reference, which writes its
