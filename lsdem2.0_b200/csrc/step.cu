@@ -481,6 +481,12 @@ LD void order_slots(const StepArgs& a, int* out, int n) {
 // as leave half the resident warps busy, since with lists this short (0.3 entries a particle
 // in the settling configuration) a round of the warp's lanes is filled by a hundred of them
 // (2M settling particles: 221 us with 32, 135 us with 128).
+//
+// Walls: with 8 particles a warp, a lane per particle would leave three of four lanes without
+// a wall to test, after the pairs' chain of loads; the walls take blocks of their own there,
+// all lanes busy, beside the pairs' (2000 bodies over a floor: 39.8 -> 39.0 us a step; 12k
+// bonded ones 61.5 -> 60.0). With 32 and more, every lane has a particle and the pairs' blocks
+// fill the chip, so that they test the walls themselves.
 template <int PER>
 __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
   constexpr int Q = PER < 32 ? 1 : PER / 32;  // particles per lane: t0 + lane + 32 q
@@ -491,6 +497,17 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
   int* pre = s_pre[threadIdx.x >> 5];
   int* cnt = s_cnt[threadIdx.x >> 5];
   const int t0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER;
+  if (PER < 32 && t0 >= a.P.n) {
+    // a small system's walls, in blocks of their own beside the pairs': one lane per particle
+    const int A = (blockIdx.x - (a.P.n + 4 * PER - 1) / (4 * PER)) * blockDim.x + threadIdx.x;
+    if (blockIdx.x * 4 * PER < (unsigned)a.P.n) return;  // the last pair block's idle warps
+    if ((int)threadIdx.x < min(a.W.n, WALLS_SH)) load_wall_box(a, threadIdx.x, s_wall[threadIdx.x]);
+    __syncthreads();
+    const bool on = A < a.P.n;
+    const int nw = on ? wall_candidates(a, s_wall, A, a.P.pos[A], a.P.radius[A]) : 0;
+    candidates_done(a, A, on, 0, nw);
+    return;
+  }
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const int cap = a.pp.cap;
   int total = 0;
@@ -565,7 +582,8 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
     }
     __syncwarp();
   }
-  if (a.W.n > 0) {
+  const bool walls = PER >= 32 && a.W.n > 0;
+  if (walls) {
     if ((int)threadIdx.x < min(a.W.n, WALLS_SH)) load_wall_box(a, threadIdx.x, s_wall[threadIdx.x]);
     __syncthreads();
   }
@@ -579,7 +597,7 @@ __global__ void __launch_bounds__(128) k_candidates(StepArgs a) {
       if (((moved[q] >> lane) & 1u) && n <= cap) order_slots(a, a.pp.id + (size_t)A * cap, n);
       a.pp.cnt[A] = n < cap ? n : cap;
       if (n > cap) atomicOr(&a.status->flags, OVF_PP);
-      if (a.W.n > 0) nw = wall_candidates(a, s_wall, A, a.P.pos[A], a.P.radius[A]);
+      if (walls) nw = wall_candidates(a, s_wall, A, a.P.pos[A], a.P.radius[A]);
     }
     candidates_done(a, A, on, n, nw);
   }
@@ -716,7 +734,7 @@ void launch_candidates(const StepArgs& a, cudaStream_t s) {
     const int half = num_sms() * 10;  // warps
     if (a.P.n >= half * 128) k_candidates<128><<<(a.P.n + 511) / 512, 128, 0, s>>>(a);
     else if (a.P.n >= half * 32) k_candidates<32><<<(a.P.n + 127) / 128, 128, 0, s>>>(a);
-    else k_candidates<8><<<(a.P.n + 31) / 32, 128, 0, s>>>(a);
+    else k_candidates<8><<<(a.P.n + 31) / 32 + (a.W.n > 0 ? (a.P.n + 127) / 128 : 0), 128, 0, s>>>(a);
     return;
   }
   k_pack_cells<<<(a.P.n + 255) / 256, 256, 0, s>>>(a, a.cell_idx);
