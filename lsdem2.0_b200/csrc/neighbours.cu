@@ -97,13 +97,16 @@ LD bool in_reach(const StepArgs& a, float4 pa, float n1a, float4 pb) {
 }
 
 // Bodies that crossed a periodic face in this step: they stand in no cell, and from the next step
-// on in the domain at their wrapped position. Their pairs there are added to the lists now, so
-// that the next step, which finds them moved by the domain, needs no rebuild of its own. One
-// warp per such body; list[0, m) holds them. (Only where the domain is wide enough that a
-// body cannot be near both positions: a.cross.)
-LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* list, int m) {
+// on at their wrapped position, in the domain or outside it along another axis. Their pairs there
+// are added to the lists now, so that the next step, which finds them moved by the domain, needs no
+// rebuild of its own. The partners of such a body are bodies in a cell, and the crossers that
+// will be; it is itself a partner, of any body of smaller index, once it is in a cell, so that the
+// bodies in no cell are looked through, too. One warp per such body; list[0, m) holds them.
+// (Only where the domain is wide enough that a body cannot be near both positions: a.cross.)
+LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* idx, const int* list, int m) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
   const int n = a.P.n;
+  const int n0 = __ldcg(w.offs + 1), nL = n - __ldcg(w.offs + a.pg.ncells + 1);  // in no cell
   const GridP& g = a.pg;
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const bool sep = a.S.sup_n != nullptr;
@@ -116,7 +119,7 @@ LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* l
     rw.p = make_float4((float)xw.x, (float)xw.y, (float)xw.z, rw.p.w);
     const float n1w = n1_f(rw.p);
     auto add = [&](int B, float4 pB) {
-      if (!in_reach(a, rw.p, n1w, pB)) return;
+      if (!__ldcg(a.kin + max(W, B)) || !in_reach(a, rw.p, n1w, pB)) return;
       CandRec rb = cand_rec(a, B, key);
       rb.p = pB;
       const bool first = W < B;
@@ -142,6 +145,11 @@ LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* l
       const int B = __ldcg(list + u);
       const double3 x = wrap_pos(a.P.pos[B], g, a.wrap_axes);
       add(B, make_float4((float)x.x, (float)x.y, (float)x.z, __ldg(a.rec_s + B).x));
+    }
+    for (int u = lane; u < n0 + nL; u += 32) {  // the bodies in no cell that did not cross
+      const int k = u < n0 ? u : n - nL + u - n0, B = __ldcg(idx + k);
+      const double3 x = a.P.pos[B], p = wrap_pos(x, g, a.wrap_axes);
+      if (p.x == x.x && p.y == x.y && p.z == x.z) add(B, a.cell_pk[k]);
     }
   }
 }
@@ -382,7 +390,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
       a.xb[A] = xw;
       const int k0 = a.pk_meta[t].x, kw = a.cross && k0 < 0 ? hash_key(xw, a.pg) : k0;
       a.kin[A] = kw >= 0;
-      if (k0 < 0 && kw >= 0) cross_list[atomicAdd(cross_n, 1)] = A;
+      if (k0 < 0 && (xw.x != xA.x || xw.y != xA.y || xw.z != xA.z)) cross_list[atomicAdd(cross_n, 1)] = A;
       const Quat q = a.P.quat[A];
       a.qb[A] = make_float4((float)q.q0, (float)q.q1, (float)q.q2, (float)q.q3);
     }
@@ -392,7 +400,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   if (lane == 0 && need > 0) atomicMax(&a.status->need_nbr, need);
   if (a.cross) {
     grid.sync();
-    grid_cross_lists(a, w, cross_list, __ldcg(cross_n));
+    grid_cross_lists(a, w, sorted_idx, cross_list, __ldcg(cross_n));
   }
   if (a.gl.list) grid_image_list(grid, a, w, sorted_idx, im, sums, sw);
 }
