@@ -83,7 +83,9 @@ constexpr int SUP_CELLS = 6 * SUP_M * SUP_M;
 constexpr int SUP_VERTS = 6 * (SUP_M + 1) * (SUP_M + 1);
 void launch_support_tables(int nshapes, const double3* node_pos, const int* node_off, const int* node_cnt,
                            const double4* pts, const long long* pts_off, float* vtx, float4* sup_n, float4* sup_s,
-                           float* sup_r, cudaStream_t s);
+                           float* sup_r, float* sup_t, cudaStream_t s);  // sup_t: zero; the largest |p| of the solid
+// sup_t: nullptr without images
+void launch_turn_radius(int n, const float4* rec_s, const float* sup_t, float* turn, cudaStream_t s);
 
 // A set of rigid bodies (particles or walls).
 struct BodyView {
@@ -256,6 +258,7 @@ struct StepArgs {
   int* reuse;
   int* reuse_next;
   float move;             // 0.4 skin
+  const float* turn;      // particle order: largest distance from the centre of a point that counts
   float skin;             // neighbour-list margin beyond the candidate reach (length)
   double3* xb;            // particle order: position at the last list build
   float4* qb;             // particle order: orientation at the last list build

@@ -416,7 +416,7 @@ struct lsdem_solver {
   DArr<double4> sup_pts;
   DArr<long long> sup_off;
   DArr<float4> sup_n, sup_s;
-  DArr<float> sup_r, sup_vtx;
+  DArr<float> sup_r, sup_t, sup_vtx, turn;
   int nbr_cap = 24;
   float skin = 0.f;
   long long builds = 0;      // steps that sorted and rebuilt the lists (lists on)
@@ -890,9 +890,11 @@ void initialize(lsdem_solver* s) {
     CK(s->sup_n.alloc((size_t)ns * SUP_CELLS));
     CK(s->sup_s.alloc((size_t)ns * SUP_CELLS));
     CK(s->sup_r.alloc((size_t)std::max(ns, 1)));
+    CK(s->sup_t.alloc((size_t)std::max(ns, 1)));
+    CK(s->sup_t.zero(st));
     CK(s->sup_vtx.alloc((size_t)2 * ns * SUP_VERTS));
     launch_support_tables(ns, s->s_node_pos.p, s->s_node_off.p, s->s_node_cnt.p, s->sup_pts.p, s->sup_off.p,
-                          s->sup_vtx.p, s->sup_n.p, s->sup_s.p, s->sup_r.p, st);
+                          s->sup_vtx.p, s->sup_n.p, s->sup_s.p, s->sup_r.p, s->sup_t.p, st);
     CK(cudaGetLastError());
   }
   {
@@ -1045,6 +1047,8 @@ void initialize(lsdem_solver* s) {
       rs[i] = make_float4((float)s->P.radius[i], (float)s->P.scale[i], shape, 0.f);
     }
     CK(s->rec_s.upload(rs.data(), rs.size(), st));
+    CK(s->turn.alloc(std::max(n, 1)));
+    launch_turn_radius(n, s->rec_s.p, (s->periodic & 7) ? s->sup_t.p : nullptr, s->turn.p, st);
     CK(cudaStreamSynchronize(st));  // rs goes out of scope
     CK(s->rb_sums.alloc(REBUILD_SUMS + 1));
     CK(s->kin.alloc(std::max(n, 1)));
@@ -1207,6 +1211,7 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.reuse = reuse ? s->reuse.p + s->hp : nullptr;
   a.reuse_next = reuse ? s->reuse.p + (1 - s->hp) : nullptr;
   a.move = 0.4f * s->skin;
+  a.turn = s->turn.p;
   a.skin = s->skin;
   a.xb = s->xb.p;
   a.qb = s->qb.p;

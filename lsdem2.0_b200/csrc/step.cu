@@ -120,7 +120,7 @@ __global__ void k_integrate_first(StepArgs a) {
       // a point of the body at distance p from its centre has moved by at most |m| + 2 |dq| p
       // (|dq| is 2 sin(angle / 4), its chord 2 sin(angle / 2) p); FP32 roundings, that of qb
       // among them, are within the 1e-6
-      const float r = (float)P.radius[i];
+      const float r = a.turn[i];
       const float move = sqrtf((float)dot(m, m)) + (2.0f * sqrtf((float)dq) + 1e-6f) * r;
       // so does a body beyond a periodic face, whose wrap k_wrap does
       const GridP& g = a.pg;
@@ -150,6 +150,19 @@ void launch_integrate_first(const StepArgs& a, cudaStream_t s) {
   int n = a.P.n + a.W.n;
   if (n < 1) n = 1;
   k_integrate_first<<<(n + 255) / 256, 256, 0, s>>>(a);
+}
+
+// Radius within which a body's points count for the lists. A node of another body counts against a
+// body only within its bounding radius, but against its images wherever their grid's solid reaches.
+__global__ void k_turn_radius(int n, const float4* __restrict__ rec_s, const float* __restrict__ sup_t,
+                              float* __restrict__ turn) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 s = rec_s[i];
+  turn[i] = sup_t ? fmaxf(s.x, s.y * sup_t[__float_as_int(s.z)]) : s.x;
+}
+void launch_turn_radius(int n, const float4* rec_s, const float* sup_t, float* turn, cudaStream_t s) {
+  if (n > 0) k_turn_radius<<<(n + 255) / 256, 256, 0, s>>>(n, rec_s, sup_t, turn);
 }
 
 __global__ void k_kick(StepArgs a) {
@@ -307,7 +320,7 @@ __constant__ double SUP_L[8] = {0.0, 0.5, 0.7, 0.85, 1.0, 1.2, 1.5, 2.5};
 __global__ void k_support_vertices(int nshapes, const double3* __restrict__ node_pos, const int* __restrict__ node_off,
                                    const int* __restrict__ node_cnt, const double4* __restrict__ pts,
                                    const long long* __restrict__ pts_off, float* __restrict__ vtx,
-                                   float* __restrict__ sup_r) {
+                                   float* __restrict__ sup_r, int* __restrict__ sup_t) {
   const int lane = threadIdx.x & 31;
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= 2LL * nshapes * SUP_VERTS) return;
@@ -342,6 +355,10 @@ __global__ void k_support_vertices(int nshapes, const double3* __restrict__ node
     }
     // the largest |p| of the solid: at a corner of its cells
     if (v == 0 && lane == 0) sup_r[sh] = __double2float_ru(mag[0] * (1.0 + 1e-9));
+    // The largest |p| of the solid itself. For p along u = sum l_i v_i (l_i >= 0, v_i the vertices of
+    // u's triangle) |p| = u . p <= sum l_i h(v_i) <= max(h(v) / |v|) sum l_i |v_i|, and the last sum is at
+    // most 1 / cos(0.1179) = 1.0070, a cell of the cube map being 1 / 12 wide at distance 1 or more.
+    if (lane == 0 && mx > 0.) atomicMax(&sup_t[sh], __float_as_int(__double2float_ru((mx + slack) / lw * 1.0071)));
   }
   // relative 1e-9 covers the rounding of the dot products and of the vertex coordinates
   if (lane == 0) vtx[w] = mx > -1e299 ? __double2float_ru(mx + slack + 1e-9 * fabs(mx) + 1e-30) : -1e30f;
@@ -362,11 +379,11 @@ __global__ void k_support_pack(int nshapes, const float* __restrict__ vtx, float
 
 void launch_support_tables(int nshapes, const double3* node_pos, const int* node_off, const int* node_cnt,
                            const double4* pts, const long long* pts_off, float* vtx, float4* sup_n, float4* sup_s,
-                           float* sup_r, cudaStream_t s) {
+                           float* sup_r, float* sup_t, cudaStream_t s) {
   const long long warps = 2LL * nshapes * SUP_VERTS;
   if (warps <= 0) return;
   k_support_vertices<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(nshapes, node_pos, node_off, node_cnt, pts,
-                                                                         pts_off, vtx, sup_r);
+                                                                         pts_off, vtx, sup_r, reinterpret_cast<int*>(sup_t));
   const long long cells = 2LL * nshapes * SUP_CELLS;
   k_support_pack<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(nshapes, vtx, sup_n, sup_s);
 }
