@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128) k_nearest(const double* __restrict__ tri,
                                                  const float4* __restrict__ sphere, int nc, GridArgs g, int n,
                                                  double* __restrict__ dist, double* __restrict__ norm) {
   const int lane = threadIdx.x & 31;
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // thread numbers pass 32 bits at 2^27 nodes
   if (i >= n) return;
   const double3 p = g.node(i % g.nx, i / g.nx % g.ny, i / (g.nx * g.ny));
   const float px = (float)p.x, py = (float)p.y, pz = (float)p.z;
