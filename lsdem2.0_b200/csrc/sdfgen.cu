@@ -523,30 +523,42 @@ extern "C" int lsdem_mesh_grid(const double* verts, int n_verts, const int* tris
   if (cudaSetDevice(device) != cudaSuccess) return LSDEM_ERR_CUDA;
   const long long n = (long long)size3[0] * size3[1] * size3[2];
   // node and triangle indices are 32-bit on the way below the brute force
-  const bool small = n < (1ll << 30) && n_tris < (1 << 28);
+  bool small = n < (1ll << 30) && n_tris < (1 << 28);
   const int nc = (n_tris + kCluster - 1) / kCluster;
   unsigned slots = 64;
   while (small && slots < 6u * (unsigned)n_tris) slots *= 2;
   // one allocation for the call
-  size_t bytes = 0;
-  auto part = [&](size_t b) {
-    const size_t at = bytes;
-    bytes += (b + 255) & ~(size_t)255;
-    return at;
+  size_t bytes, o_vert, o_tris, o_tri, o_sph, o_trif, o_out, o_dist, o_norm, o_par, o_list, o_in, o_zero, o_keys, o_sums, o_flag;
+  auto layout = [&] {
+    bytes = 0;
+    auto part = [&](size_t b) {
+      const size_t at = bytes;
+      bytes += (b + 255) & ~(size_t)255;
+      return at;
+    };
+    o_vert = part(24 * (size_t)n_verts), o_tris = part(12 * (size_t)n_tris);
+    o_tri = part(8 * (size_t)kTriD * n_tris), o_sph = part(16 * (size_t)nc), o_trif = part(48 * (size_t)n_tris);
+    o_out = part(8 * (size_t)n);
+    const size_t m = small ? (size_t)n : 0;
+    o_dist = part(8 * m), o_norm = part(8 * m), o_par = part(4 * m), o_list = part(4 * m), o_in = part(m);
+    o_zero = bytes, o_keys = part(small ? 8 * (size_t)slots : 0), o_sums = part(small ? 4 * (size_t)slots : 0);
+    o_flag = part(8);  // {open, components}
   };
-  const size_t o_vert = part(24 * (size_t)n_verts), o_tris = part(12 * (size_t)n_tris);
-  const size_t o_tri = part(8 * (size_t)kTriD * n_tris), o_sph = part(16 * (size_t)nc), o_trif = part(48 * (size_t)n_tris);
-  const size_t o_out = part(8 * (size_t)n);
-  const size_t o_dist = part(small ? 8 * (size_t)n : 0), o_norm = part(small ? 8 * (size_t)n : 0);
-  const size_t o_par = part(small ? 4 * (size_t)n : 0), o_list = part(small ? 4 * (size_t)n : 0);
-  const size_t o_in = part(small ? (size_t)n : 0);
-  const size_t o_zero = bytes, o_keys = part(small ? 8 * (size_t)slots : 0), o_sums = part(small ? 4 * (size_t)slots : 0);
-  const size_t o_flag = part(8);  // {open, components}
+  layout();
   char* d = nullptr;
   int rc = LSDEM_OK;
   cudaStream_t st = nullptr;
   if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) rc = LSDEM_ERR_CUDA;
-  if (rc == LSDEM_OK && cudaMalloc(&d, bytes) != cudaSuccess) rc = LSDEM_ERR_NOMEM;
+  if (rc == LSDEM_OK && cudaMalloc(&d, bytes) != cudaSuccess) {
+    d = nullptr;
+    if (small) {  // 33 bytes a node do not fit: the brute force takes 8
+      small = false;
+      layout();
+      if (cudaMalloc(&d, bytes) != cudaSuccess) d = nullptr;
+    }
+    cudaGetLastError();
+    if (!d) rc = LSDEM_ERR_NOMEM;
+  }
   if (rc == LSDEM_OK) {
     auto at = [&](size_t o) { return d + o; };
     double* d_tri = (double*)at(o_tri);
