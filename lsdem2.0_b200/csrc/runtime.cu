@@ -628,7 +628,8 @@ void alloc_contacts(lsdem_solver* s, ContactsDev& c, long long cap) {
 }
 
 // Learned form: the network queues (rows per shape), the pending nodes and the pair
-// records of both narrowphase launches. Per-step scratch: contents are not kept.
+// records of each narrowphase launch (images have one of their own where they are searched in every
+// step; from the image list they are screened with the rest). Per-step scratch: contents are not kept.
 void alloc_net(lsdem_solver* s) {
   const int n = std::max(s->P.n(), 1);
   const int ns = std::max((int)s->shapes.size(), 1);
@@ -636,11 +637,12 @@ void alloc_net(lsdem_solver* s) {
   if (s->cap_netq <= 0) s->cap_netq = std::max<long long>(1 << 14, s->cap_pend / ns * 2);
   s->cap_pend = std::min<long long>(s->cap_pend, 0x7fffffffLL);
   s->cap_netq = std::min<long long>(s->cap_netq, 0x7fffffffLL / ns);
+  const bool apart = s->nsets > 0 && (!s->reuse_on || (s->periodic & 8));
   for (int l = 0; l < 2; ++l) {
     auto& N = s->net[l];
-    const long long pairs = l == 0 ? (long long)n * (s->slots[0][0].cap + s->slots[0][1].cap + s->slots[0][2].cap)
+    const long long pairs = l == 0 ? (long long)n * (s->slots[0][0].cap + s->slots[0][1].cap + (apart ? 0 : s->slots[0][2].cap))
                                    : (long long)n * s->slots[0][2].cap;
-    if (l == 1 && s->nsets == 0) {
+    if (l == 1 && !apart) {
       N.qcap = N.pcap = N.paircap = 0;
       N.row.release(); N.cnt.release(); N.pend_n.release(); N.ctr.release();
       N.pend_v.release(); N.pair.release();
@@ -2706,6 +2708,7 @@ int lsdem_set_neighbour_lists(lsdem_solver* s, int on) {
     s->reuse_on = on != 0;
     ++s->graph_gen;
     s->force_reuse = true;
+    s->net_dirty = true;  // the launches the network queues are for
   }
   return LSDEM_OK;
 }
