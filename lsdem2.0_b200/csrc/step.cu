@@ -260,7 +260,10 @@ LD bool wall_far(const StepArgs& a, int w, double3 l, double reach) {
   return phi > bound;
 }
 
-// Appends this lane's entries A * cap + j, j < cnt, to a flat pair list, with
+// Entry of a flat pair list: A * cap + slot in 32 bits, unsigned (alloc_slots bounds it).
+LD int pair_code(int A, int cap, int slot) { return (int)((unsigned)A * cap + slot); }
+
+// Appends this lane's entries (A, j), j < cnt, to a flat pair list, with
 // one atomic per warp (all lanes of the warp call it).
 LD void append_pairs(int* list, int* ctr, int A, int cap, int cnt) {
   const int lane = threadIdx.x & 31;
@@ -273,7 +276,7 @@ LD void append_pairs(int* list, int* ctr, int A, int cap, int cnt) {
   int base = 0;
   if (lane == 31 && tot > 0) base = atomicAdd(ctr, tot);
   base = __shfl_sync(FULL, base, 31) + incl - cnt;
-  for (int j = 0; j < cnt; ++j) list[base + j] = (int)((unsigned)A * cap + j);
+  for (int j = 0; j < cnt; ++j) list[base + j] = pair_code(A, cap, j);
 }
 
 // Centres and bounding radii in a sorted order (idx), FP32, for the candidate
@@ -1564,15 +1567,15 @@ __global__ void __launch_bounds__(NP_WARPS * 32, KINDS == 1 ? 8 : 5) k_screen_f(
       if ((KINDS & 1) && e < n0) {
         const unsigned idx = __ldg(a.pl.list[0] + e);
         const int A = idx / a.pp.cap;
-        make_pair_f<KIND_PP, SDFK>(a, A, idx - A * a.pp.cap, __ldg(a.pp.id + idx), F);
+        make_pair_f<KIND_PP, SDFK>(a, A, idx - (unsigned)A * a.pp.cap, __ldg(a.pp.id + idx), F);
       } else if ((KINDS & 2) && e < n0 + n1) {
         const unsigned idx = a.pl.list[1][e - n0];
         const int A = idx / a.pw.cap;
-        make_pair_f<KIND_WALL, SDFK>(a, A, idx - A * a.pw.cap, a.pw.id[idx], F);
+        make_pair_f<KIND_WALL, SDFK>(a, A, idx - (unsigned)A * a.pw.cap, a.pw.id[idx], F);
       } else if (KINDS & 4) {
         const unsigned idx = __ldg(a.pl.list[2] + e - n0 - n1);
         const int A = idx / a.pgh.cap;
-        make_pair_f<KIND_GHOST, SDFK>(a, A, idx - A * a.pgh.cap, __ldg(a.pgh.id + idx), F);
+        make_pair_f<KIND_GHOST, SDFK>(a, A, idx - (unsigned)A * a.pgh.cap, __ldg(a.pgh.id + idx), F);
       }
     }
     __syncwarp();
@@ -2163,7 +2166,7 @@ __global__ void k_ghost_candidates(StepArgs a, const int* __restrict__ g2_idx, c
               int base = 0;
               if (lane == 0 && m) base = atomicAdd(&a.pl.ctr[2], __popc(m));
               base = __shfl_sync(FULL, base, 0);
-              if (ok) a.pl.list[2][base + __popc(m & lanemask_lt())] = A * a.pgh.cap + slot;
+              if (ok) a.pl.list[2][base + __popc(m & lanemask_lt())] = pair_code(A, a.pgh.cap, slot);
             }
           }
         }
@@ -2237,7 +2240,7 @@ __global__ void __launch_bounds__(128) k_image_candidates(StepArgs a) {
       int at = 0;
       if (lane == 0 && mk) at = atomicAdd(&a.pl.ctr[2], __popc(mk));
       at = __shfl_sync(FULL, at, 0);
-      if (ok) a.pl.list[2][at + __popc(mk & lanemask_lt())] = (int)((unsigned)A * a.pgh.cap + slot);
+      if (ok) a.pl.list[2][at + __popc(mk & lanemask_lt())] = pair_code(A, a.pgh.cap, slot);
     }
   }
   need = __reduce_max_sync(FULL, need);
