@@ -163,12 +163,10 @@ struct BucketScratch {
 };
 
 size_t scan_temp_elems(long long n);
-// gate (optional): the launches return at once when *gate is zero
-void scan_i32(const int* in, int* out, long long n, int* tmp, bool inclusive, cudaStream_t s,
-              const int* gate = nullptr);
+void scan_i32(const int* in, int* out, long long n, int* tmp, bool inclusive, cudaStream_t s);
 void scan_i64(const long long* in, long long* out, long long n, long long* tmp, bool inclusive, cudaStream_t s);
 void bucket_sort(const int* key, int n, int ncells, BucketScratch& w, int* sorted_idx, int* sorted_key, int* start,
-                 int* end, cudaStream_t s, const int* gate = nullptr);
+                 int* end, cudaStream_t s);
 
 // Nodes the FP32 screen could not reject, by pair, for the FP64
 // contact pass. One node cursor per step; one pair list per narrowphase launch

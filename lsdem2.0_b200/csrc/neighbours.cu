@@ -109,7 +109,6 @@ LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* i
   const int n0 = __ldcg(w.offs + 1), nL = n - __ldcg(w.offs + a.pg.ncells + 1);  // in no cell
   const GridP& g = a.pg;
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
-  const bool sep = a.S.sup_n != nullptr;
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
   for (int v = tid >> 5; v < m; v += T >> 5) {
     const int W = __ldcg(list + v);
@@ -124,7 +123,7 @@ LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* i
       rb.p = pB;
       const bool first = W < B;
       const CandRec &r0 = first ? rw : rb, &r1 = first ? rb : rw;
-      if (sep && pair_separated<2>(sup, r0.p, n1_f(r0.p), r0.q, r0.sc, r0.sh, r1.p, r1.q, r1.sc, r1.sh, gap)) return;
+      if (pair_separated<2>(sup, r0.p, n1_f(r0.p), r0.q, r0.sc, r0.sh, r1.p, r1.q, r1.sc, r1.sh, gap)) return;
       const int A = first ? W : B, at = atomicAdd(&a.nbr_cnt[A], 1);
       if (at >= 0 && at < a.nbr_cap) a.nbr[(size_t)at * n + A] = first ? B : W;
       if (at >= a.nbr_cap) {
@@ -217,7 +216,6 @@ LD void grid_image_list(cg::grid_group& grid, const StepArgs& a, const BucketScr
   grid.sync();
   const int nimg = __ldcg(a.G.count);
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
-  const bool sep = a.S.sup_n != nullptr;
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
   for (int v = tid >> 5; v < nimg; v += T >> 5) {  // one warp per image
     const int t = __ldcg(a.G.list + v), moved = t & 1, s = (t >> 1) / n, i = (t >> 1) % n;
@@ -242,7 +240,7 @@ LD void grid_image_list(cg::grid_group& grid, const StepArgs& a, const BucketScr
         if (A >= 0 && !(dist2_f(pa, rb.p) > R * R)) {
           int kA;
           const CandRec ra = cand_rec(a, A, kA);
-          keep = !(sep && pair_separated<2>(sup, pa, n1_f(pa), ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh, gap));
+          keep = !pair_separated<2>(sup, pa, n1_f(pa), ra.q, ra.sc, ra.sh, rb.p, rb.q, rb.sc, rb.sh, gap);
         }
         const unsigned b = __ballot_sync(FULL, keep);
         int at = 0;
@@ -295,7 +293,6 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   // then tested one lane per pair, since a lane testing as it walks would leave most of the
   // warp idle (2M settling particles: 2.5 ms a rebuild that way, 1.7 ms now).
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
-  const bool sep = a.S.sup_n != nullptr;
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
   const int lane = threadIdx.x & 31;
   int* buf = s_buf[threadIdx.x >> 5];
@@ -367,8 +364,8 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
           const int4 mA = a.pk_meta[to], mB = a.pk_meta[kB];
           const float4 po = a.cell_pk[to];
           B = mB.y;
-          keep = !(sep && pair_separated<2>(sup, po, n1_f(po), a.pk_q[to], __int_as_float(mA.w), mA.z, a.cell_pk[kB],
-                                            a.pk_q[kB], __int_as_float(mB.w), mB.z, gap));
+          keep = !pair_separated<2>(sup, po, n1_f(po), a.pk_q[to], __int_as_float(mA.w), mA.z, a.cell_pk[kB],
+                                    a.pk_q[kB], __int_as_float(mB.w), mB.z, gap);
         }
         const unsigned mk = __ballot_sync(FULL, keep);
         const int at = cnt[ow] + __popc(mk & ((1u << lane) - 1u) & (~0u << max(first - i0, 0)));

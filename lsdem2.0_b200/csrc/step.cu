@@ -651,7 +651,6 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * blockDim.x + threadIdx.x, t0 = t - lane;
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
-  const bool sep = a.S.sup_n != nullptr;
   const int cap = a.pp.cap;
   __shared__ int s_slot[4][32][SLOT_SH + 1];
   __shared__ WallBox s_wall[WALLS_SH];
@@ -680,19 +679,15 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
         slot(lane, A, n++) = k;
         return;
       }
-      if (sep) {
-        int w = fixed;
+      int w = fixed;
 #pragma unroll 1
-        for (int j = fixed; j <= n; ++j) {
-          const int kj = j < n ? slot(lane, A, j) : k;
-          if (pair_separated_call(sup, a.cell_pk, a.pk_meta, a.pk_q, t, kj)) continue;
-          if (w < cap) slot(lane, A, w++) = kj;
-          else ++extra;
-        }
-        n = fixed = w;
-      } else {
-        ++extra;
+      for (int j = fixed; j <= n; ++j) {
+        const int kj = j < n ? slot(lane, A, j) : k;
+        if (pair_separated_call(sup, a.cell_pk, a.pk_meta, a.pk_q, t, kj)) continue;
+        if (w < cap) slot(lane, A, w++) = kj;
+        else ++extra;
       }
+      n = fixed = w;
     };
     const int3 c = clamp_cell(cell_of(xA, a.pg), a.pg.size);
     // the (up to) 3 cells of a row along x are contiguous in the sorted order
@@ -729,7 +724,7 @@ __global__ void __launch_bounds__(128) k_candidates_walk(StepArgs a) {
       int& o = slot(ow, oA, j);
       const int k = o;
       int B = a.pk_meta[k].y;
-      if (sep && j >= ofix && pair_separated_at(sup, a.cell_pk, a.pk_meta, a.pk_q, t0 + ow, k)) B = -1;
+      if (j >= ofix && pair_separated_at(sup, a.cell_pk, a.pk_meta, a.pk_q, t0 + ow, k)) B = -1;
       o = B;
     }
   }
@@ -2121,10 +2116,10 @@ __global__ void k_ghost_candidates(StepArgs a, const int* __restrict__ g2_idx, c
     const int z0 = axis_lo(xg.z, g.mn.z, g.inv.z, g.size.z, reach, cz), z1 = axis_hi(xg.z, g.mn.z, g.inv.z, g.size.z, reach, cz);
     const float3 xgf = make_float3((float)xg.x, (float)xg.y, (float)xg.z);
     const float Rgf = (float)Rg, n1g = fabsf(xgf.x) + fabsf(xgf.y) + fabsf(xgf.z);
-    // separation test of the pair (owner A, image) along the line of centres, as for
+    // separation test of the pair (owner A, image), as for
     // particle pairs: a translated image has the particle's orientation, shape and scale
     // (turned sector images are not tested)
-    const bool sep = a.S.sup_n != nullptr && !a.G.sector;
+    const bool sep = !a.G.sector;
     const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
     const Quat qi = a.P.quat[i];
     const float4 qbf = make_float4((float)qi.q0, (float)qi.q1, (float)qi.q2, (float)qi.q3);
