@@ -395,76 +395,66 @@ LD bool solid_angle_f(float3 p, float4 a, float4 b, float4 c, float& angle) {
   return true;
 }
 
-// Solid-angle sum of each component's root: inside[root]. A block takes kRoots roots at a time
-// (four read the triangles together, but leave the chip two blocks an SM for the thousand-odd
-// components of a body: 278 us against 131 with one). In FP32
+// Solid-angle sum of each component's root: inside[root], one block per root at a time (four at
+// a time read the triangles together, but leave the chip two blocks an SM for the thousand-odd
+// components of a body: 278 us against 131). In FP32
 // the mesh and the node are rounded to 1e-7 of the mesh's size, each vertex alike in all its
 // triangles, so the mesh stays closed, and nodes farther than 1e-5 of that size from it stay on
-// their side.
-constexpr int kRoots = 1;
+// their side. Nodes nearer than that sum in FP64, and those on the surface as far as rounding goes
+// in the triangles' order, which is the reference's: a block's threads take the angles and one of
+// them adds (43,200 triangles of a box, 11,600 of 91,000 nodes on its faces: 300 ms for the call with
+// one thread taking the angles, too, 5.4 ms with the block).
 __global__ void __launch_bounds__(128) k_component_sign(const double* __restrict__ tri, const float4* __restrict__ trif,
                                                         int nt, GridArgs g, double scale,
                                                         const double* __restrict__ dist, const int* __restrict__ list,
                                                         const int* __restrict__ count, unsigned char* inside) {
-  __shared__ double s_sum[4][kRoots];
-  __shared__ int s_again[kRoots];
-  const int n = *count, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto node = [&](int i) { return g.node(i % g.nx, i / g.nx % g.ny, i / (g.nx * g.ny)); };
+  __shared__ double s_sum[128];
+  const int n = *count, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto angle = [&](double3 q, int t) {
     const double* r = tri + (size_t)kTriD * t;
     return solid_angle(q, d3(r[0], r[1], r[2]), d3(r[3], r[4], r[5]), d3(r[6], r[7], r[8]));
   };
+  auto block_sum = [&](double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+    __syncthreads();  // the last sum has been read
+    if (lane == 0) s_sum[warp] = v;
+    __syncthreads();
+    return s_sum[0] + s_sum[1] + s_sum[2] + s_sum[3];
+  };
   const double pi4 = 4.0 * 3.14159265358979323846;
-  for (int k = blockIdx.x * kRoots; k < n; k += gridDim.x * kRoots) {
-    const int m = min(kRoots, n - k);
-    double sum[kRoots];
-    float3 q[kRoots];
-#pragma unroll
-    for (int v = 0; v < kRoots; ++v) {
-      const double3 p = node(list[min(k + v, n - 1)]);
-      q[v] = make_float3((float)(p.x * scale), (float)(p.y * scale), (float)(p.z * scale));
-      sum[v] = 0.0;
-    }
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-      const float4 a = __ldg(trif + 3 * (size_t)t), b = __ldg(trif + 3 * (size_t)t + 1), c = __ldg(trif + 3 * (size_t)t + 2);
-#pragma unroll
-      for (int v = 0; v < kRoots; ++v) {
+  for (int k = blockIdx.x; k < n; k += gridDim.x) {
+    const int i = list[k];
+    const double3 p = g.node(i % g.nx, i / g.nx % g.ny, i / (g.nx * g.ny));
+    const double d = dist[i];
+    double w = 0.0;
+    bool sure = d == 0.0;  // the value there does not depend on the side
+    if (d * scale > 1e-5) {
+      const float3 q = make_float3((float)(p.x * scale), (float)(p.y * scale), (float)(p.z * scale));
+      double sum = 0.0;
+      for (int t = tid; t < nt; t += 128) {
+        const float4 a = __ldg(trif + 3 * (size_t)t), b = __ldg(trif + 3 * (size_t)t + 1), c = __ldg(trif + 3 * (size_t)t + 2);
         float f;
-        sum[v] += solid_angle_f(q[v], a, b, c, f) ? (double)f : angle(node(list[min(k + v, n - 1)]), t);
+        sum += solid_angle_f(q, a, b, c, f) ? (double)f : angle(p, t);
       }
+      w = block_sum(sum) / pi4;
+      sure = fabs(w - rint(w)) < 0.05;
     }
-#pragma unroll
-    for (int v = 0; v < kRoots; ++v) {
-      for (int o = 16; o > 0; o >>= 1) sum[v] += __shfl_xor_sync(~0u, sum[v], o);
-      if (lane == 0) s_sum[warp][v] = sum[v];
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < m) {
-      const int v = threadIdx.x, i = list[k + v];
-      const double w = (s_sum[0][v] + s_sum[1][v] + s_sum[2][v] + s_sum[3][v]) / pi4;
-      inside[i] = fabs(w) > 0.5;
-      s_again[v] = !(fabs(w - rint(w)) < 0.05) || !(dist[i] * scale > 1e-5);
-    }
-    __syncthreads();
-    for (int v = 0; v < m; ++v) {  // in FP64 where that was not sure
-      if (!s_again[v]) continue;
-      const int i = list[k + v];
-      const double3 p = node(i);
-      double s = 0.0;
-      if (dist[i] < 1e-6 * g.h) {  // on the surface as far as rounding goes: the reference's own sum
-        if (threadIdx.x == 0)
-          for (int t = 0; t < nt; ++t) s += angle(p, t);
-      } else {
-        for (int t = threadIdx.x; t < nt; t += blockDim.x) s += angle(p, t);
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(~0u, s, o);
-        if (lane == 0) s_sum[warp][0] = s;
+    if (!sure && d < 1e-6 * g.h) {
+      double sum = 0.0;
+      for (int t0 = 0; t0 < nt; t0 += 128) {
+        __syncthreads();  // the last angles have been added
+        if (t0 + tid < nt) s_sum[tid] = angle(p, t0 + tid);
         __syncthreads();
-        s = s_sum[0][0] + s_sum[1][0] + s_sum[2][0] + s_sum[3][0];
-        __syncthreads();
+        if (tid == 0)
+          for (int t = 0; t < min(128, nt - t0); ++t) sum += s_sum[t];
       }
-      if (threadIdx.x == 0) inside[i] = fabs(s / pi4) > 0.5;
+      w = sum / pi4;  // the first thread's
+    } else if (!sure) {
+      double sum = 0.0;
+      for (int t = tid; t < nt; t += 128) sum += angle(p, t);
+      w = block_sum(sum) / pi4;
     }
-    __syncthreads();
+    if (tid == 0) inside[i] = fabs(w) > 0.5;
   }
 }
 
