@@ -101,36 +101,56 @@ LD bool in_reach(const StepArgs& a, float4 pa, float n1a, float4 pb) {
 // are added to the lists now, so that the next step, which finds them moved by the domain, needs no
 // rebuild of its own. The partners of such a body are bodies in a cell, and the crossers that
 // will be; it is itself a partner, of any body of smaller index, once it is in a cell, so that the
-// bodies in no cell are looked through, too. One warp per such body; list[0, m) holds them.
+// bodies in no cell are looked through, too. list[0, m) holds them.
 // (Only where the domain is wide enough that a body cannot be near both positions: a.cross.)
+//
+// A warp walks the cells of one crosser; the crossers and the bodies in no cell are tested against
+// each crosser in chunks of 32, spread over the warps (100k bodies with 30k of them above the domain,
+// one or two crossers a step: 660 us a step with all of it by the crosser's warp, 333 this way). The
+// work is the product of two counts: above CROSS_PAIRS the next step rebuilds instead (bodies that
+// are handed over a domain's length off all cross at once).
+static constexpr long long CROSS_PAIRS = 1ll << 24;
 LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* idx, const int* list, int m) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x, lane = threadIdx.x & 31;
   const int n = a.P.n;
   const int n0 = __ldcg(w.offs + 1), nL = n - __ldcg(w.offs + a.pg.ncells + 1);  // in no cell
+  if ((long long)m * (m + n0 + nL) > CROSS_PAIRS) {
+    if (tid == 0) *a.reuse_next = 2;
+    return;
+  }
   const GridP& g = a.pg;
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
-  for (int v = tid >> 5; v < m; v += T >> 5) {
-    const int W = __ldcg(list + v);
-    const double3 xw = wrap_pos(a.P.pos[W], g, a.wrap_axes);
+  // crosser v at its next position
+  int W = 0;
+  double3 xw = d3(0., 0., 0.);
+  CandRec rw;
+  float n1w = 0.f;
+  auto take = [&](int v) {
+    W = __ldcg(list + v);
+    xw = wrap_pos(a.P.pos[W], g, a.wrap_axes);
     int key;
-    CandRec rw = cand_rec(a, W, key);
+    rw = cand_rec(a, W, key);
     rw.p = make_float4((float)xw.x, (float)xw.y, (float)xw.z, rw.p.w);
-    const float n1w = n1_f(rw.p);
-    auto add = [&](int B, float4 pB) {
-      if (!__ldcg(a.kin + max(W, B)) || !in_reach(a, rw.p, n1w, pB)) return;
-      CandRec rb = cand_rec(a, B, key);
-      rb.p = pB;
-      const bool first = W < B;
-      const CandRec &r0 = first ? rw : rb, &r1 = first ? rb : rw;
-      if (pair_separated<2>(sup, r0.p, n1_f(r0.p), r0.q, r0.sc, r0.sh, r1.p, r1.q, r1.sc, r1.sh, gap)) return;
-      const int A = first ? W : B, at = atomicAdd(&a.nbr_cnt[A], 1);
-      if (at >= 0 && at < a.nbr_cap) a.nbr[(size_t)at * n + A] = first ? B : W;
-      if (at >= a.nbr_cap) {
-        atomicMax(&a.status->need_nbr, at + 1);
-        atomicOr(&a.status->flags, OVF_NBR);
-      }
-    };
+    n1w = n1_f(rw.p);
+  };
+  auto add = [&](int B, float4 pB) {
+    if (!__ldcg(a.kin + max(W, B)) || !in_reach(a, rw.p, n1w, pB)) return;
+    int key;
+    CandRec rb = cand_rec(a, B, key);
+    rb.p = pB;
+    const bool first = W < B;
+    const CandRec &r0 = first ? rw : rb, &r1 = first ? rb : rw;
+    if (pair_separated<2>(sup, r0.p, n1_f(r0.p), r0.q, r0.sc, r0.sh, r1.p, r1.q, r1.sc, r1.sh, gap)) return;
+    const int A = first ? W : B, at = atomicAdd(&a.nbr_cnt[A], 1);
+    if (at >= 0 && at < a.nbr_cap) a.nbr[(size_t)at * n + A] = first ? B : W;
+    if (at >= a.nbr_cap) {
+      atomicMax(&a.status->need_nbr, at + 1);
+      atomicOr(&a.status->flags, OVF_NBR);
+    }
+  };
+  for (int v = tid >> 5; v < m; v += T >> 5) {
+    take(v);
     const double R = a.P.radius[W] + a.rmax + (double)a.skin;
     const double ext = 1.001 * R + 1e-4 * (fabs(xw.x) + fabs(xw.y) + fabs(xw.z) + 4.0 * R);
     const int3 lo = ball_cell(xw - d3(ext, ext, ext), g), hi = ball_cell(xw + d3(ext, ext, ext), g);
@@ -140,13 +160,17 @@ LD void grid_cross_lists(const StepArgs& a, const BucketScratch& w, const int* i
         const int st = __ldcg(w.offs + h0 + 1), en = __ldcg(w.offs + h0 + (hi.x - lo.x) + 2);
         for (int k = st + lane; k < en; k += 32) add(a.pk_meta[k].y, a.cell_pk[k]);
       }
-    for (int u = v + 1 + lane; u < m; u += 32) {  // the other bodies of the list, once
+  }
+  const int chunks = (m + n0 + nL + 31) / 32;
+  for (int q = tid >> 5; q < m * chunks; q += T >> 5) {
+    const int v = q / chunks, u = (q - v * chunks) * 32 + lane;
+    take(v);
+    if (u < m) {  // the other crossers, once
       const int B = __ldcg(list + u);
       const double3 x = wrap_pos(a.P.pos[B], g, a.wrap_axes);
-      add(B, make_float4((float)x.x, (float)x.y, (float)x.z, __ldg(a.rec_s + B).x));
-    }
-    for (int u = lane; u < n0 + nL; u += 32) {  // the bodies in no cell that did not cross
-      const int k = u < n0 ? u : n - nL + u - n0, B = __ldcg(idx + k);
+      if (u > v) add(B, make_float4((float)x.x, (float)x.y, (float)x.z, __ldg(a.rec_s + B).x));
+    } else if (u < m + n0 + nL) {  // the bodies in no cell that did not cross
+      const int k = u - m < n0 ? u - m : n - nL + u - m - n0, B = __ldcg(idx + k);
       const double3 x = a.P.pos[B], p = wrap_pos(x, g, a.wrap_axes);
       if (p.x == x.x && p.y == x.y && p.z == x.z) add(B, a.cell_pk[k]);
     }

@@ -4,7 +4,11 @@ A body outside the domain owns pairs (its cell is clamped) and is no one's partn
 inside exists when the outside one has the smaller index. The two of a scene touch across a face; one of them, or both, cross it
 in the third of twelve steps and nothing else sets off a rebuild, so that the steps after the crossing live on what
 that rebuild listed. Every step equals the run without lists.
+
+Where many bodies cross at once, their pairs are left to the next step's rebuild.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -72,3 +76,40 @@ def test_pair_with_a_body_outside(lsdem, case, others, prec):
     assert a[4] <= 3  # the first step's, the crossing's and at most one that the contact's motion sets off
     assert (b[0][-1][0] > 0 and b[0][-1][2] > 0) or case == "inside owns"
     _compare(a, b)
+
+
+@pytest.mark.parametrize("n", [3_000, 4_500, 60_000])  # 3,000 are looked up (below 2^24 pairs), the others not
+def test_all_bodies_cross_at_once(lsdem, n):
+    """Bodies handed over a domain's length off, some of them touching, across faces among them."""
+    from lsdem_b200 import scenes
+    rng = np.random.default_rng(n)
+    m = int(np.ceil(n ** (1.0 / 3.0)))
+    i = np.arange(n)
+    a = 9.8e-3
+    pos = np.stack([i % m, (i // m) % m, i // (m * m)], 1) * a + rng.uniform(0.0, 1e-3, size=(n, 3))
+    side = m * a
+    shp = scenes.make_ellipsoid(AXES, 16, 100)
+    mp = lsdem.mass_properties(shp["sdf"], shp["size"], shp["origin"], shp["spacing"], 2500.0)
+    out, took = [], []
+    for lists in (True, False):
+        sv = lsdem.Solver()
+        sid = sv.add_shape(shp["nodes"], shp["sdf"], shp["size"], shp["origin"], shp["spacing"])
+        sv.add_particles(np.full(n, sid), pos + [side, 0, -side], scenes.random_quaternions(np.random.default_rng(1), n),
+                         1.0 / mp["mass"], np.tile(mp["inv_inertia"], (n, 1)), 1e5, 8e4, 0.5, 0.6, vel=np.zeros((n, 3)))
+        sv.set_capacity(pp=64, wall=1, ghost=64, contacts=1 << 21)
+        sv.set_periodic(7)
+        sv.set_neighbour_lists(lists)
+        sv.initialize(np.zeros(3), np.full(3, side), np.zeros(3))
+        sv.set_record_contacts(True)
+        per = []
+        t0 = time.perf_counter()
+        for _ in range(4):
+            sv.step(1e-7, 1)
+            st = sv.step_stats()
+            per.append((0, 0, st["contacts"]))
+        took.append(time.perf_counter() - t0)
+        out.append((per, sv.contacts(lsdem.CONTACT_PARTICLE), sv.contacts(lsdem.CONTACT_GHOST), sv.state()))
+        sv.close()
+    _compare(*out)
+    assert out[0][0][-1][2] > 0
+    assert took[0] < 5 * took[1] + 0.1, took
