@@ -50,18 +50,17 @@ __device__ __forceinline__ void cx(int& ka, int& a, int& kb, int& b) {
   }
 }
 
-// Bodies of the first and last bucket (outside every cell) where these are longer than 64, by
-// one block, in ascending index order.
-__device__ inline void special_buckets(const int* __restrict__ key, int n, int ncells, const int* offs,
-                                       int* __restrict__ sorted_idx, int* sw) {
+// Bodies i0 to i1 of the first and last bucket (outside every cell) where these are longer than 64,
+// by one block, in ascending index order from base0 and baseL on.
+__device__ inline void special_buckets(const int* __restrict__ key, int i0, int i1, int ncells, const int* offs, int base0,
+                                       int baseL, int* __restrict__ sorted_idx, int* sw) {
   const int L = ncells + 1;
-  const int n0 = offs[1] - offs[0], nL = offs[L + 1] - offs[L];
-  if (n0 <= 64 && nL <= 64) return;
-  int base0 = offs[0], baseL = offs[L];
-  for (int t0 = 0; t0 < n; t0 += blockDim.x) {
+  const bool long0 = offs[1] - offs[0] > 64, longL = offs[L + 1] - offs[L] > 64;
+  if (!long0 && !longL) return;
+  for (int t0 = i0; t0 < i1; t0 += blockDim.x) {
     const int i = t0 + threadIdx.x;
-    const int b = i < n ? bucket_of(key[i], ncells) : -1;
-    const int f0 = b == 0 && n0 > 64, fL = b == L && nL > 64;
+    const int b = i < i1 ? bucket_of(key[i], ncells) : -1;
+    const int f0 = b == 0 && long0, fL = b == L && longL;
     int tot0, totL;
     const int r0 = block_exclusive_scan<int>(f0, sw, &tot0);
     const int rL = block_exclusive_scan<int>(fL, sw, &totL);

@@ -132,7 +132,7 @@ __global__ void k_bucket_scatter(const int* __restrict__ key, int n, int ncells,
 __global__ void k_special_buckets(const int* __restrict__ key, int n, int ncells, const int* __restrict__ offs,
                                   int* __restrict__ sorted_idx) {
   __shared__ int sw[32];
-  special_buckets(key, n, ncells, offs, sorted_idx, sw);
+  special_buckets(key, 0, n, ncells, offs, offs[0], offs[ncells + 1], sorted_idx, sw);
 }
 
 // Cell ranges [start, end) of every cell (-1 when empty; findStartAndEnd,

@@ -113,3 +113,43 @@ def test_all_bodies_cross_at_once(lsdem, n):
     _compare(*out)
     assert out[0][0][-1][2] > 0
     assert took[0] < 5 * took[1] + 0.1, took
+
+
+@pytest.mark.parametrize("n, outside", [(700, 63), (700, 64), (700, 65), (700, 699), (300, 257), (5_000, 1_200)])
+def test_order_of_bodies_in_no_cell(lsdem, n, outside):
+    """Bodies outside in any order among the others: listed in index order by chunks of a block each (above 64 of them)."""
+    from lsdem_b200 import scenes
+    rng = np.random.default_rng(n + outside)
+    m = int(np.ceil(n ** (1.0 / 3.0)))
+    p = rng.permutation(m ** 3)
+    i = np.arange(n)
+    a = 9e-3
+    pos = (np.stack([i % m, (i // m) % m, i // (m * m)], 1) + 0.5) * a + rng.uniform(-2e-4, 2e-4, size=(n, 3))
+    z = np.sort(pos[:, 2])
+    cut = 0.5 * (z[n - outside - 1] + z[n - outside])
+    pos = pos[np.argsort(p[:n])]
+    shp = scenes.make_ellipsoid(AXES, 16, 200)
+    mp = lsdem.mass_properties(shp["sdf"], shp["size"], shp["origin"], shp["spacing"], 2500.0)
+    out = []
+    for lists in (True, False):
+        sv = lsdem.Solver()
+        sid = sv.add_shape(shp["nodes"], shp["sdf"], shp["size"], shp["origin"], shp["spacing"])
+        sv.add_particles(np.full(n, sid), pos, scenes.random_quaternions(np.random.default_rng(2), n), 1.0 / mp["mass"],
+                         np.tile(mp["inv_inertia"], (n, 1)), 1e5, 8e4, 0.5, 0.6,
+                         vel=np.random.default_rng(3).normal(0.0, 2.0, size=(n, 3)))
+        sv.set_capacity(pp=64, wall=1, ghost=64, contacts=1 << 20)
+        sv.set_periodic(3)
+        sv.set_neighbour_lists(lists)
+        sv.initialize(np.array([0.0, 0.0, -0.01]), np.array([m * a, m * a, cut]), np.zeros(3))
+        sv.set_record_contacts(True)
+        per = []
+        for _ in range(8):
+            sv.step(2e-6, 1)
+            per.append((0, 0, sv.step_stats()["contacts"]))
+        h = sv.hash()
+        key = h["key"]
+        assert np.array_equal(h["sorted_idx"], np.argsort(key, kind="stable"))
+        out.append((per, sv.contacts(lsdem.CONTACT_PARTICLE), sv.contacts(lsdem.CONTACT_GHOST), sv.state()))
+        sv.close()
+    assert abs((key < 0).sum() - outside) <= 12  # some move through the upper face
+    _compare(*out)
