@@ -967,7 +967,7 @@ LD const SlotView& slots_of(const StepArgs& a, bool old) {
 // admitted node (LSParticleContactDetectionKernel.cu:63-115, contactKernel.cu:75-117 /
 // :155-190 / :225-270); writes the contact at pos.
 LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, const PairK& K, int ni, int ostart,
-                     int ocnt, int pos, bool can_write, double3& FA, double3& TA, double3& FB, double3& TB) {
+                     int ocnt, int rank, int pos, bool can_write, double3& FA, double3& TA, double3& FB, double3& TB) {
   const double3 w = node_world(a, S, ni);
   double ov, fx, fy, fz, cr[8];
   sdf_eval(w, P, ov, fx, fy, fz, cr);
@@ -975,14 +975,17 @@ LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, cons
   n = rotate(P.q, n);
   n = normalize_dev(n);
   const double3 pc = w + 0.5 * ov * n;
-  // carried-over spring: binary search of node ni in the old segment (sorted by node)
+  // carried-over spring: search of node ni in the old segment (sorted by node), outwards from its
+  // rank in the new one, where it mostly still is, then by halves
   double3 spring = d3(0., 0., 0.);
-  int lo = 0, hi = ocnt - 1;
+  int lo = 0, hi = ocnt - 1, mid = min(rank, hi), away = 1;
+  bool below = false, above = false;
   while (lo <= hi) {
-    const int mid = (lo + hi) >> 1;
     const int v = a.C_old.node[ostart + mid];
     if (v == ni) { spring = a.C_old.spring[ostart + mid]; break; }
-    if (v < ni) lo = mid + 1; else hi = mid - 1;
+    if (v < ni) { lo = mid + 1; below = true; } else { hi = mid - 1; above = true; }
+    if (below && above) mid = (lo + hi) >> 1;
+    else { mid = below ? min(hi, mid + away) : max(lo, mid - away); away *= 4; }
   }
   const double3 vc = S.v + cross(S.w, pc - S.x) - (P.v + cross(P.w, pc - P.x));
   double3 F;
@@ -1607,21 +1610,27 @@ LD Partner load_partner_of(const StepArgs& a, int kind, int pid) {
 // A warp takes up to 32 pairs and runs their nodes, then their contacts, one lane each, whichever
 // pair they are of. A pair of a bed has 1.5 queued nodes and 0.7 contacts, so that a warp per
 // pair left 30 of its lanes idle through a chain of dependent loads, eight warps an SM (100k
-// bodies with 336k contacts: 2325 us that way, 150 us now). With few pairs a warp takes
-// one, and the lanes are its nodes as before.
+// bodies with 336k contacts: 2325 us that way, 150 us now). A warp takes fewer where there are
+// not 32 for each, or where pairs have many nodes: at least 64 nodes, on the average. In 32s, bodies
+// with faces pressed together, hundreds of contacts a pair, left most warps waiting for a few (100k
+// bodies, 4.3M contacts of 115k pairs: 2160 us that way, 1190 us; 8,000 cubes, 5.2M contacts: a step
+// of 770 us, 925 with the constants formed for each contact and the old segment searched by halves).
+// A pair's constants are formed once, by the lane that has the pair.
 // Between the two runs a pair's hits stand at the front of its part of the node queue, in node
 // order; one atomic per warp reserves the segments of its pairs.
 __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int li) {
   __shared__ int4 s_pair[NP_WARPS][32];   // {A, partner, first node, hits}
   __shared__ int4 s_seg[NP_WARPS][32];    // {segment (-1: does not fit), old segment, its length, kind}
+  __shared__ PairK s_cst[NP_WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int4* pair = s_pair[warp];
   int4* seg = s_seg[warp];
+  PairK* cst = s_cst[warp];
   const int np = min(a.mb.ctr[1 + li], a.mb.pcap);
   if (blockIdx.x == 0 && threadIdx.x == 0)  // this step's demand, for the capacity planning
     atomicMax(&a.status->need_queue, max(a.mb.ctr[0], min(np, 0x3fffffff) * 2));
   const int W = gridDim.x * NP_WARPS;
-  const int per = min(32, (np + W - 1) / W);
+  const int per = max(1, min(min(32, (np + W - 1) / W), (int)min(32ll, 64ll * np / max(1, a.mb.ctr[0]))));
   for (int p0 = (blockIdx.x * NP_WARPS + warp) * per; p0 < np; p0 += W * per) {
     __syncwarp();  // the previous pairs' records are still read
     int4 e = make_int4(-1, 0, 0, 0);  // A < 0: reserved by a pair whose nodes did not fit the queue
@@ -1700,6 +1709,10 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
       cur.seg_cnt[sidx] = fits ? h : 0;
       if (!fits) atomicOr(&a.status->flags, OVF_CONTACT);
       seg[lane] = make_int4(fits ? base : -1, ostart, ocnt, kind);
+      if (h > 0) {
+        const Partner P = load_partner_of(a, kind, pid);
+        cst[lane] = kind == KIND_WALL ? pair_constants<KIND_WALL>(a, e.x, P) : pair_constants<KIND_PP>(a, e.x, P);
+      }
     }
     __syncwarp();
     for (int i0 = 0; i0 < total; i0 += 32) {
@@ -1718,8 +1731,8 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
         S.sc = a.P.scale[A];
         S.n0 = a.S.node_off[a.P.shape[A]];
         const Partner P = load_partner_of(a, k, pr.y);
-        const PairK K = k == KIND_WALL ? pair_constants<KIND_WALL>(a, A, P) : pair_constants<KIND_PP>(a, A, P);
-        contact_node(a, S, P, K, a.mb.node[pr.z + i - first], sg.y, sg.z, sg.x + i - first, sg.x >= 0, FA, TA, FB, TB);
+        const PairK K = cst[ow];
+        contact_node(a, S, P, K, a.mb.node[pr.z + i - first], sg.y, sg.z, i - first, sg.x + i - first, sg.x >= 0, FA, TA, FB, TB);
         // an image of the owner itself takes no reaction
         if (!(k == KIND_GHOST && P.real == A)) real = P.real;
       }
