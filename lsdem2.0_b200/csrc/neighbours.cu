@@ -340,14 +340,20 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   // walks until its shared buffer of bodies within reach + skin is full; the warp's buffers are
   // then tested one lane per pair, since a lane testing as it walks would leave most of the
   // warp idle (2M settling particles: 2.5 ms a rebuild that way, 1.7 ms now).
+  // Where the bodies do not fill the grid's threads, 2 to 8 lanes share a body, each with its part of
+  // the rows (3,000 polydisperse bodies at 5 m/s, rebuilt in 46 of 80 steps: 133 us a step with one
+  // lane a body, 100 this way).
   const SupTabs sup{a.S.sup_n, a.S.sup_s, a.S.sup_r};
   const float gap = 0.8f * a.skin * (1.0f + 1e-5f);
   const int lane = threadIdx.x & 31;
   int* buf = s_buf[threadIdx.x >> 5];
   int* cnt = s_cnt[threadIdx.x >> 5];
+  int sh = 0;  // 1 << sh lanes per body
+  while (sh < 3 && (long long)n << (sh + 1) <= T) ++sh;
+  const int body = lane >> sh, part = lane & ((1 << sh) - 1);
   int need = 0;
-  for (int t0 = tid - lane; t0 < n; t0 += T) {
-    const int t = t0 + lane;
+  for (int t0 = (tid >> 5) * (32 >> sh); t0 < n; t0 += (T >> 5) * (32 >> sh)) {
+    const int t = t0 + body;
     float4 pa = make_float4(0.f, 0.f, 0.f, 0.f);
     float n1a = 0.f;
     int A = 0, r = 0, rows = 0, ny = 1, k = 0, en = 0;
@@ -371,6 +377,8 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
                      max(hi.z, min(c.z + 1, a.pg.size.z - 1)));
       ny = hi.y - lo.y + 1;
       rows = ny * (hi.z - lo.z + 1);
+      r = (rows * part) >> sh;
+      rows = (rows * (part + 1)) >> sh;
     }
     cnt[lane] = 0;
     while (__any_sync(FULL, r < rows || k < en)) {
@@ -405,10 +413,11 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
         const int i = i0 + lane;
         const int ow = lane_of(incl, i);
         const int first = __shfl_sync(FULL, incl - m, ow), oA = __shfl_sync(FULL, A, ow);
+        const int ob = ow >> sh, fb = __shfl_sync(FULL, incl - m, ob << sh);  // the body, its first entry
         bool keep = false;
         int B = 0;
         if (i < total) {
-          const int kB = buf[32 * (i - first) + ow], to = t0 + ow;
+          const int kB = buf[32 * (i - first) + ow], to = t0 + ob;
           const int4 mA = a.pk_meta[to], mB = a.pk_meta[kB];
           const float4 po = a.cell_pk[to];
           B = mB.y;
@@ -416,16 +425,16 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
                                     a.pk_q[kB], __int_as_float(mB.w), mB.z, gap);
         }
         const unsigned mk = __ballot_sync(FULL, keep);
-        const int at = cnt[ow] + __popc(mk & ((1u << lane) - 1u) & (~0u << max(first - i0, 0)));
+        const int at = cnt[ob] + __popc(mk & ((1u << lane) - 1u) & (~0u << max(fb - i0, 0)));
         if (keep && at < a.nbr_cap) a.nbr[(size_t)at * n + oA] = B;
-        const int nx = __shfl_down_sync(FULL, ow, 1);
+        const int nx = __shfl_down_sync(FULL, ob, 1);
         __syncwarp();
-        if (i < total && (lane == 31 || nx != ow || i + 1 == total)) cnt[ow] = at + keep;
+        if (i < total && (lane == 31 || nx != ob || i + 1 == total)) cnt[ob] = at + keep;
         __syncwarp();
       }
     }
-    if (t < n) {
-      const int nl = cnt[lane];
+    if (t < n && part == 0) {
+      const int nl = cnt[body];
       // an overflowed list: the batch re-runs with longer lists
       a.nbr_cnt[A] = nl <= a.nbr_cap ? nl : -1;
       if (nl > a.nbr_cap) atomicOr(&a.status->flags, OVF_NBR);
@@ -461,8 +470,12 @@ void launch_rebuild(const StepArgs& a, const BucketScratch& w, const ImageSort& 
     blocks = std::min(std::max(1, sms * per), REBUILD_SUMS / 2);
   }
   if (a.P.n <= 0) return;
-  // one thread per body or two buckets; fewer blocks make the barriers of a small system cheaper
-  const int want = std::max((a.P.n + RB_THREADS - 1) / RB_THREADS, (a.pg.ncells / 2 + RB_THREADS) / RB_THREADS);
+  // One thread per two buckets; four per body, or one block, whose barriers are the cheapest; with
+  // images, one per nine images of the sets (201 bodies in a narrow box that rebuild in two of
+  // three steps: 190 us a step with one block, 99 with 22)
+  int want = (a.pg.ncells / 2 + RB_THREADS) / RB_THREADS;
+  if (a.P.n > RB_THREADS) want = (int)std::max<long long>(want, (4ll * a.P.n + RB_THREADS - 1) / RB_THREADS);
+  if (a.gl.list) want = (int)std::max<long long>(want, ((long long)a.G.nsets * a.P.n + 63) / 64);
   StepArgs aa = a;
   BucketScratch ww = w;
   ImageSort im = img;
