@@ -1615,7 +1615,9 @@ LD Partner load_partner_of(const StepArgs& a, int kind, int pid) {
 // with faces pressed together, hundreds of contacts a pair, left most warps waiting for a few (100k
 // bodies, 4.3M contacts of 115k pairs: 2160 us that way, 1190 us; 8,000 cubes, 5.2M contacts: a step
 // of 770 us, 925 with the constants formed for each contact and the old segment searched by halves).
-// A pair's constants are formed once, by the lane that has the pair.
+// A pair's constants are formed once, by the lane that has the pair, where the contacts take more than
+// one round; in one round, with each contact, beside its loads (2,000 bodies on a floor: 38.9 us a
+// step with the constants first, 37.7 this way).
 // Between the two runs a pair's hits stand at the front of its part of the node queue, in node
 // order; one atomic per warp reserves the segments of its pairs.
 __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int li) {
@@ -1630,7 +1632,8 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
   if (blockIdx.x == 0 && threadIdx.x == 0)  // this step's demand, for the capacity planning
     atomicMax(&a.status->need_queue, max(a.mb.ctr[0], min(np, 0x3fffffff) * 2));
   const int W = gridDim.x * NP_WARPS;
-  const int per = max(1, min(min(32, (np + W - 1) / W), (int)min(32ll, 64ll * np / max(1, a.mb.ctr[0]))));
+  int per = 1;
+  if (np > W) per = max(1, min(min(32, (np + W - 1) / W), (int)fminf(32.f, 64.f * (float)np / (float)max(1, a.mb.ctr[0]))));
   for (int p0 = (blockIdx.x * NP_WARPS + warp) * per; p0 < np; p0 += W * per) {
     __syncwarp();  // the previous pairs' records are still read
     int4 e = make_int4(-1, 0, 0, 0);  // A < 0: reserved by a pair whose nodes did not fit the queue
@@ -1690,6 +1693,7 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
       if (lane >= o) incl += v;
     }
     total = __shfl_sync(FULL, incl, 31);
+    const bool many = total > 32;  // contacts fill more than one round of the lanes
     int base = 0;
     if (lane == 0 && total > 0) base = atomicAdd(a.C.count, total);
     base = __shfl_sync(FULL, base, 0) + incl - h;
@@ -1709,7 +1713,7 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
       cur.seg_cnt[sidx] = fits ? h : 0;
       if (!fits) atomicOr(&a.status->flags, OVF_CONTACT);
       seg[lane] = make_int4(fits ? base : -1, ostart, ocnt, kind);
-      if (h > 0) {
+      if (h > 0 && many) {
         const Partner P = load_partner_of(a, kind, pid);
         cst[lane] = kind == KIND_WALL ? pair_constants<KIND_WALL>(a, e.x, P) : pair_constants<KIND_PP>(a, e.x, P);
       }
@@ -1731,7 +1735,8 @@ __global__ void __launch_bounds__(NP_WARPS * 32, 3) k_contacts_f(StepArgs a, int
         S.sc = a.P.scale[A];
         S.n0 = a.S.node_off[a.P.shape[A]];
         const Partner P = load_partner_of(a, k, pr.y);
-        const PairK K = cst[ow];
+        const PairK K = many ? cst[ow]
+                             : (k == KIND_WALL ? pair_constants<KIND_WALL>(a, A, P) : pair_constants<KIND_PP>(a, A, P));
         contact_node(a, S, P, K, a.mb.node[pr.z + i - first], sg.y, sg.z, i - first, sg.x + i - first, sg.x >= 0, FA, TA, FB, TB);
         // an image of the owner itself takes no reaction
         if (!(k == KIND_GHOST && P.real == A)) real = P.real;
