@@ -27,7 +27,9 @@ static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int RB_THREADS = 256;
 static constexpr int RB_BUF = 12;  // bodies within reach + skin a lane gathers before the warp tests them
 
-// The stable cell sort of bucket_sort (sort_scan.cu), phase by phase.
+// The stable cell sort of bucket_sort (sort_scan.cu), phase by phase; the members of a cell in any
+// order where ORDERED is false (the images' search, whose list has none).
+template <bool ORDERED>
 LD void grid_cell_sort(cg::grid_group& grid, const int* key, int n, int ncells, const BucketScratch& w, int* sorted_idx,
                        int* sums, int* sw) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
@@ -89,6 +91,7 @@ LD void grid_cell_sort(cg::grid_group& grid, const int* key, int n, int ncells, 
     special_buckets(key, i0, i1, ncells, w.offs, base0, n - nL + baseL, sorted_idx, sw);
   }
   grid.sync();
+  if (!ORDERED) return;
   for (int b = tid; b < nb; b += T) {
     const int s = w.offs[b], L = w.offs[b + 1] - s;
     if (L <= 1 || (b == 0 && L > 64)) continue;
@@ -224,7 +227,7 @@ LD void grid_image_list(cg::grid_group& grid, const StepArgs& a, const BucketScr
     for (int i = tid; i < n; i += T)
       im.key[i] = lin3(clamp_cell(cell_of(wrap_pos(a.P.pos[i], g, a.wrap_axes), g), g.size), g.size);
     grid.sync();
-    grid_cell_sort(grid, im.key, n, g.ncells, im.w, im.idx, sums, sw);
+    grid_cell_sort<false>(grid, im.key, n, g.ncells, im.w, im.idx, sums, sw);
     for (int k = tid; k < n; k += T) {
       const int B = __ldcg(im.idx + k);
       const double3 p = wrap_pos(a.P.pos[B], g, a.wrap_axes);
@@ -332,7 +335,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2) k_rebuild(StepArgs a, BucketScr
   int* cross_n = sums + REBUILD_SUMS;
   int* cross_list = w.tmp;  // the sort's, free after it
   if (tid == 0) *cross_n = 0;
-  grid_cell_sort(grid, a.P.key, n, a.pg.ncells, w, sorted_idx, sums, sw);
+  grid_cell_sort<true>(grid, a.P.key, n, a.pg.ncells, w, sorted_idx, sums, sw);
   if (tid == 0) atomicAdd(&a.status->builds, 1);
   for (int k = tid; k < n; k += T) pack_cell(a, k, __ldcg(sorted_idx + k));
   grid.sync();
