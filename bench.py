@@ -98,25 +98,20 @@ NET_FLOP = 8704
 
 
 # Algorithmic bytes of k_screen_f (the screen of every form; contacts are evaluated by the
-# separate FP64 contact pass): per owner particle (pose, scale, shape, slot count: 72 B) and
-# per candidate pair (partner id, pose, radius, grid origin and spacing, shape,
-# segment words: 120 B). B_CONTACT: per contact of a step (node id, FP64 spring read and
-# write, history lookup).
+# separate FP64 contact pass) per candidate pair: the owner's pose, scale and shape (72 B), the
+# partner's id, pose, radius, grid origin and spacing, shape and the segment words (120 B).
+# B_CONTACT: per contact of a step (node id, FP64 spring read and write, history lookup).
 B_CONTACT = 56
-B_PARTICLE_SCREEN = 72
-B_PAIR_SCREEN = 120
+B_PAIR_SCREEN = 72 + 120
 # whole-step algorithmic bytes per particle (state, keys, sort, candidates)
 B_STEP_PARTICLE = 448
-# What bounds the screen: an ncu full-set capture of k_screen_f<1, 2, 0> (particle pairs,
+# What bounds the screen: an ncu full-set capture of k_screen_f<1, 2, 0, 0> (particle pairs,
 # FP32/BF16 form) on the settling configuration at 200,000 particles (two launches alike).
 SCREEN_CAPTURE = {
     "case": "settling configuration at 200,000 particles, FP32/BF16 form, particle-pair screen, steps 2-3",
-    "dram_bytes_per_launch": 38.35e6,
-    # 72 B x 200,000 owners + 120 B x ~51,500 particle pairs (of 55,400 pairs of all kinds)
-    "algorithmic_bytes_per_launch": 72 * 200_000 + 120 * 51_500,
-    "issue_active": 0.616, "warps_active": 0.447, "warps_active_limit": 0.50,
-    "leading_stall": "long_scoreboard (5.5 warps per issue): dependent L2 loads",
-    "dram_throughput": 0.039,
+    "dram_bytes_per_launch": 19.02e6, "pairs": 9_463,
+    "issue_active": 0.508, "warps_active": 0.404, "warps_active_limit": 0.50,
+    "leading_stall": "long_scoreboard (6.6 warps per issue): dependent L2 loads",
 }
 
 
@@ -769,12 +764,11 @@ def main():
         # a step runs the particle/wall launch and the image launch: per-launch bytes = per-step / 2
         launches_per_step = 2 if g_calls else 1
         kernel = "k_screen_f"
-        bytes_launch = (B_PARTICLE_SCREEN * n * launches_per_step + B_PAIR_SCREEN * pairs) / launches_per_step
-        # DRAM bytes per launch: the capture's measured traffic scaled by algorithmic bytes
-        # (its excess over them is the 16-bit template store read once per step after the
-        # L2 flush, so the scaling overstates it for larger cases: an upper estimate)
-        traffic = (SCREEN_CAPTURE["dram_bytes_per_launch"] / SCREEN_CAPTURE["algorithmic_bytes_per_launch"] *
-                   bytes_launch) if prec != 0 else None
+        bytes_launch = B_PAIR_SCREEN * pairs / launches_per_step
+        # DRAM bytes per launch: the capture's (nearly all of it the 16-bit template store, read
+        # once per step after the L2 flush) and the further pairs' algorithmic bytes
+        traffic = max(SCREEN_CAPTURE["dram_bytes_per_launch"] + bytes_launch - B_PAIR_SCREEN * SCREEN_CAPTURE["pairs"],
+                      bytes_launch) if prec != 0 else None
         achieved = bytes_launch / (avg_ms * 1e-3) / 1e9
         b_step = B_STEP_PARTICLE * n + B_CONTACT * stats["contacts"] + 16 * pairs
         ms_step = head["ms"] / args.steps
@@ -803,12 +797,12 @@ def main():
             "contacts_per_s": stats["contacts"] * per_s,
             "node_tests_per_s": scr.get("node_tests", 0.0) * per_s if scr else None,
             # The screen is bound by load latency and instruction issue, not by DRAM: its
-            # algorithmic bytes over its launch time are a few percent of HBM bandwidth
+            # algorithmic bytes over its launch time are about a percent of HBM bandwidth
             # (reported as such), the issue and warp figures come from ncu.
             "roofline": {"bound": "latency/issue", "kernel": kernel, "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                          "algorithmic_bytes_per_launch": bytes_launch, "avg_launch_ms": avg_ms,
-                         "traffic_kind": "scaled from a 200,000-particle ncu capture" if prec != 0 else None,
+                         "traffic_kind": "a 200,000-particle ncu capture and the further pairs' bytes" if prec != 0 else None,
                          "hbm_is_limiter": False,
                          "limiter": ({"bound": "L2 load latency / issue", "issue_active": SCREEN_CAPTURE["issue_active"],
                                       "warps_active": SCREEN_CAPTURE["warps_active"],

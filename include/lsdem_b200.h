@@ -80,7 +80,8 @@ int lsdem_mesh_grid_box(const double* verts, int n_verts, double spacing, int pa
  * (LevelSetObjectGenerator.h:122-224, 454-500, 758-802, 888-914).
  * positive_inside = TriangleMeshParticle::setLevelSetPositiveInside. verts: n_verts
  * x 3, tris: n_tris x 3 vertex indices, sdf_out: size3[0] x size3[1] x size3[2]
- * values in the order ix + nx (iy + ny iz), host memory; blocking. LSDEM_ERR_ARG
+ * values in the order ix + nx (iy + ny iz), host memory; blocking. Device memory:
+ * 33 bytes a node, or 8, and more time, where that does not fit. LSDEM_ERR_ARG
  * for a mesh the reference's isValid rejects (no vertices or triangles, an index
  * out of range or repeated within a triangle). */
 int lsdem_mesh_grid(const double* verts, int n_verts, const int* tris, int n_tris, const double* origin3,
@@ -360,7 +361,9 @@ int lsdem_set_graphs(lsdem_solver* s, int on);
  * entered or left the domain, or one crossed a periodic face. Contacts and results are
  * the same as with on = 0, which sorts and walks the 27 cells every step as the
  * reference does (LSSolver.h:1000-1011, mySpatialGrid.cu,
- * LSParticleContactDetectionKernel.cu). */
+ * LSParticleContactDetectionKernel.cu). The numbers of candidate pairs of
+ * lsdem_step_stats may differ between the two: a pair that a rebuild showed to be apart is
+ * no candidate of the steps that use its lists. */
 int lsdem_set_neighbour_lists(lsdem_solver* s, int on);
 
 /* Snapshot of the dynamic state (no counterpart in the reference, which writes its

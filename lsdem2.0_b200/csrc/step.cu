@@ -1023,8 +1023,8 @@ LD void contact_node(const StepArgs& a, const SelfCtx& S, const Partner& P, cons
 //
 // Per pair, the owner's node offsets n (template units) map to the partner's
 // frame by l = M n + dB, M = R_B^T R_A scale_A, dB = R_B^T (xA - xB), and to its
-// grid by g = l invh + cg, cg = -origin invh. M and dB are formed in FP32 from the
-// step's FP32 rotation matrices (each entry rounded once from FP64) and from
+// grid by g = l invh + cg, cg = -origin invh. M and dB are formed in FP32 from
+// the pair's FP32 rotation matrices (each entry rounded once from FP64) and from
 // xA - xB rounded from FP64.
 //
 // Error bounds (unit roundoff u = 2^-24; |.|_1 norms bound the Euclidean ones):
@@ -1253,7 +1253,7 @@ LD int window_state(const StepArgs& a, double3 x, float3 ra, float e0, int key) 
 }
 
 // FP32 screen of one node (offset nd, template units): false only when the
-// FP64 test (node_hits) certainly rejects it.
+// FP64 test (k_contacts_f) certainly rejects it.
 template <int KIND, int SDFK, class FX>
 LD bool node_may_hit_f(const StepArgs& a, const FX& F, float4 nd, bool& looked) {
   const float3 l = mulf(F.M, nd.x, nd.y, nd.z) + F.dB;
@@ -1273,7 +1273,7 @@ LD bool node_may_hit_f(const StepArgs& a, const FX& F, float4 nd, bool& looked) 
 }
 
 // Cluster cull (sphere of radius rad about the cluster centre cn, template
-// units): false only when no node of the cluster can pass node_hits.
+// units): false only when no node of the cluster can pass the FP64 test.
 //  - particle partners: the sphere misses the partner's bounding sphere;
 //  - the sphere misses the partner's grid box (nodes outside it fail the SDF test);
 //  - phi / h at q, the centre projected into the box shrunk by m >= eg, exceeds
