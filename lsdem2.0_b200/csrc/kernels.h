@@ -44,12 +44,10 @@ struct ShapeView {
   const double* sdf;          // FP64 SDF store
   const int* node_off;        // per shape, into node_pos
   const int* node_cnt;        // per shape
-  const int* cl_off;          // per shape, into cl_sphere
+  const int* cl_off;          // per shape, into cl_sphere_f
   const int* cl_cnt;          // per shape
   const double3* node_pos;    // node store, cluster order, unscaled
-  const int* node_orig;       // original node index within the shape
-  const double4* cl_sphere;   // cluster bounding sphere (xyz centre, w radius), unscaled
-  const float4* cl_sphere_f;  // the same rounded to FP32 (the precision forms' screen)
+  const float4* cl_sphere_f;  // cluster bounding sphere (xyz centre, w radius), unscaled, rounded to FP32
   const float4* sub_sphere;   // 4 per cluster (same shape offsets x 4): spheres of 8 nodes,
                               //   unscaled; radius < 0 for a sub-cluster past the last node
   const double* node_box;     // 8 per shape (unscaled): node bounding box lo xyz, hi xyz,
@@ -107,7 +105,6 @@ struct BodyView {
   const double* scale;       // uniform template scale
   const double3* origin;     // grid node (0,0,0) in body frame (scaled)
   const double* invh;        // inverse grid spacing (scaled)
-  const long long* node_base;  // global id of the first surface node (particles)
   int* key;                  // cell key of this step, -1 outside the domain
 };
 
@@ -225,8 +222,6 @@ struct StepArgs {
   float4* cell_pk;        // particle grid, sorted order: FP32 centre and bounding radius
   const int* cell_off;    // particle grid: sorted position of the first body of cell k at [k + 1]
                           //   (bucket offsets of the cell sort, ncells + 3 entries)
-  const int* cell_start;
-  const int* cell_end;
   SlotView pp, pw, pgh;          // this step
   SlotView pp_old, pw_old, pgh_old;  // previous step
   ContactView C, C_old;
@@ -256,8 +251,8 @@ struct StepArgs {
   int* reuse;
   int* reuse_next;
   float move;             // 0.4 skin
-  const float* turn;      // particle order: largest distance from the centre of a point that counts
   float skin;             // neighbour-list margin beyond the candidate reach (length)
+  const float* turn;      // particle order: largest distance from the centre of a point that counts
   double3* xb;            // particle order: position at the last list build
   float4* qb;             // particle order: orientation at the last list build
   unsigned char* kin;     // particle order: in a cell, as the last list build expects it

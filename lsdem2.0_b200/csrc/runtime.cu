@@ -274,7 +274,6 @@ void build_clusters(ShapeHost& s) {
 struct BodyHost {
   std::vector<double> pos, vel, angvel, quat, force, torque, invm, invI, radius, kn, ks, mu, res, scale, origin, invh;
   std::vector<int> shape;
-  std::vector<long long> node_base;
   int n() const { return (int)shape.size(); }
 };
 
@@ -284,7 +283,6 @@ struct BodyDev {
   DArr<double> invm, radius, kn, ks, mu, res, scale, invh;
   DArr<Sym6> invI;
   DArr<int> shape, key;
-  DArr<long long> node_base;
 };
 
 struct SlotsDev {
@@ -345,9 +343,8 @@ struct lsdem_solver {
   DArr<int3> s_gsize;
   DArr<long long> s_sdf_off;
   DArr<double> s_sdf;
-  DArr<int> s_node_off, s_node_cnt, s_cl_off, s_cl_cnt, s_node_orig;
+  DArr<int> s_node_off, s_node_cnt, s_cl_off, s_cl_cnt;
   DArr<double3> s_node_pos;
-  DArr<double4> s_cl;
   DArr<float4> s_clf;   // cluster spheres in FP32 (each component rounded to nearest)
   DArr<float4> s_sub;   // sub-cluster spheres, 4 per cluster (FP32, radius rounded up)
   DArr<double> s_nbox;  // per shape: node bounding box (lo xyz, hi xyz), largest node distance, 0
@@ -711,7 +708,6 @@ void upload_bodies(lsdem_solver* s, BodyHost& H, BodyDev& D) {
   CK(D.invh.upload(H.invh.data(), n, st));
   CK(D.shape.upload(H.shape.data(), n, st));
   CK(D.key.alloc(std::max<size_t>(n, 1)));
-  if (!H.node_base.empty()) CK(D.node_base.upload(H.node_base.data(), n, st));
 }
 
 // Brings the host copies of the bodies' state up to date with the device after steps:
@@ -808,7 +804,7 @@ void initialize(lsdem_solver* s) {
   std::vector<int3> gs;
   std::vector<long long> sdf_off;
   std::vector<double> sdf;
-  std::vector<int> node_off, node_cnt, cl_off, cl_cnt, node_orig;
+  std::vector<int> node_off, node_cnt, cl_off, cl_cnt;
   std::vector<double3> node_pos;
   std::vector<double4> cl;
   for (const ShapeHost& sh : s->shapes) {
@@ -821,7 +817,6 @@ void initialize(lsdem_solver* s) {
     for (int k = 0; k < M; ++k) {
       const double* p = &sh.nodes[3 * sh.perm[k]];
       node_pos.push_back(make_double3(p[0], p[1], p[2]));
-      node_orig.push_back(sh.perm[k]);
     }
     cl_off.push_back((int)cl.size());
     cl_cnt.push_back((int)(sh.cl.size() / 4));
@@ -838,8 +833,6 @@ void initialize(lsdem_solver* s) {
   CK(s->s_cl_off.upload(cl_off.data(), cl_off.size(), st));
   CK(s->s_cl_cnt.upload(cl_cnt.data(), cl_cnt.size(), st));
   CK(s->s_node_pos.upload(node_pos.data(), node_pos.size(), st));
-  CK(s->s_node_orig.upload(node_orig.data(), node_orig.size(), st));
-  CK(s->s_cl.upload(cl.data(), cl.size(), st));
   {
     std::vector<float4> clf(cl.size());
     for (size_t c = 0; c < cl.size(); ++c)
@@ -1004,13 +997,6 @@ void initialize(lsdem_solver* s) {
       nf[i] = make_float4((float)node_pos[i].x, (float)node_pos[i].y, (float)node_pos[i].z, 0.f);
     CK(s->s_node_f.upload(nf.data(), nf.size(), st));
   }
-  // node ids (LSBoundaryNode order: particle by particle, caller node order)
-  s->P.node_base.resize(s->P.n());
-  long long nb = 0;
-  for (int i = 0; i < s->P.n(); ++i) {
-    s->P.node_base[i] = nb;
-    nb += (long long)(s->shapes[s->P.shape[i]].nodes.size() / 3);
-  }
   upload_bodies(s, s->P, s->dP);
   upload_bodies(s, s->W, s->dW);
   // grids: cell = 2 x max bounding radius (LSParticle.h:241-256)
@@ -1152,15 +1138,14 @@ StepArgs make_args(lsdem_solver* s, double dt) {
     v.pos = D.pos.p; v.vel = D.vel.p; v.angvel = D.angvel.p; v.force = D.force.p; v.torque = D.torque.p;
     v.quat = D.quat.p; v.invmass = D.invm.p; v.invI = D.invI.p; v.radius = D.radius.p; v.kn = D.kn.p;
     v.ks = D.ks.p; v.mu = D.mu.p; v.res = D.res.p; v.shape = D.shape.p; v.scale = D.scale.p;
-    v.origin = D.origin.p; v.invh = D.invh.p; v.node_base = D.node_base.p; v.key = D.key.p;
+    v.origin = D.origin.p; v.invh = D.invh.p; v.key = D.key.p;
     return v;
   };
   a.P = bv(s->dP, s->P.n());
   a.W = bv(s->dW, s->W.n());
   a.S.gsize = s->s_gsize.p; a.S.sdf_off = s->s_sdf_off.p; a.S.sdf = s->s_sdf.p;
   a.S.node_off = s->s_node_off.p; a.S.node_cnt = s->s_node_cnt.p; a.S.cl_off = s->s_cl_off.p;
-  a.S.cl_cnt = s->s_cl_cnt.p; a.S.node_pos = s->s_node_pos.p; a.S.node_orig = s->s_node_orig.p;
-  a.S.cl_sphere = s->s_cl.p;
+  a.S.cl_cnt = s->s_cl_cnt.p; a.S.node_pos = s->s_node_pos.p;
   a.S.cl_sphere_f = s->s_clf.p;
   a.S.node_box = s->s_nbox.p;
   a.S.sub_sphere = s->s_sub.p;
@@ -1173,7 +1158,7 @@ StepArgs make_args(lsdem_solver* s, double dt) {
   a.S.sup_r = s->sup_r.p;
   a.pg = s->pg;
   a.wg = s->wg;
-  a.cell_idx = s->cell_idx.p; a.cell_start = s->cell_start.p; a.cell_end = s->cell_end.p;
+  a.cell_idx = s->cell_idx.p;
   a.cell_pk = s->cell_pk.p;
   a.cell_off = s->bk_offs.p;
   auto sv = [](SlotsDev& d) {
