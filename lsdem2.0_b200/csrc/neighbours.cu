@@ -474,7 +474,7 @@ void launch_rebuild(const StepArgs& a, const BucketScratch& w, const ImageSort& 
   }
   if (a.P.n <= 0) return;
   // One thread per two buckets; four per body, or one block, whose barriers are the cheapest; with
-  // images, one per nine images of the sets (201 bodies in a narrow box that rebuild in two of
+  // images, a block per 64 pairs of a set and a body (201 bodies in a narrow box that rebuild in two of
   // three steps: 190 us a step with one block, 99 with 22)
   int want = (a.pg.ncells / 2 + RB_THREADS) / RB_THREADS;
   if (a.P.n > RB_THREADS) want = (int)std::max<long long>(want, (4ll * a.P.n + RB_THREADS - 1) / RB_THREADS);
